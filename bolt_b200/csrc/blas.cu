@@ -2,7 +2,7 @@
 // mirrors of Bolt's public blas_enhance functions (`b200_*`).
 //
 // Host logic only: argument checks, the tmp / packed-weight protocol of Bolt's callers, pointer
-// staging, kernel selection.  The arithmetic lives in gemm_i8_tcgen05.cu, gemm_i8_simt.cu, gemv_i8.cu.
+// staging, kernel selection.  The arithmetic lives in gemm_i8_tcgen05.cu, gemm_i8_gather.cu, gemv_i8.cu.
 #include <cstring>
 #include <utility>
 
@@ -163,8 +163,8 @@ EE run_gemm(U32 N, U32 M, U32 K, bool a_t, const void *A, const void *B, const v
     } else if (ep.scatter_n > 0) {
         return NOT_SUPPORTED;  // the scatter epilogue exists on the tensor-core path only
     } else {
-        ret = launch_gemm_simt(M, N, K, dA, a_t, dB, Kp, dC, ep, st);
-        tls().last_gemm_tc = 0;
+        ret = launch_gemm_gather(M, N, K, dA, a_t, dB, Kp, dC, ep, st);
+        tls().last_gemm_tc = 1;
     }
     B200_EE(ret);
     return sg.finish();

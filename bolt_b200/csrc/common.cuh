@@ -56,7 +56,7 @@ struct WeightTwin {
 
 // kernel families whose dynamic shared-memory limit has to be raised above 48 KiB; the attribute
 // belongs to the device that is current when it is set, so it is remembered per device context
-enum KernelFamily { KF_GEMM = 0, KF_CONV, KF_CONV_HALF, KF_GEMV, KF_GEMV_ROW, KF_BNN, KF_PROBE, KF_COUNT };
+enum KernelFamily { KF_GEMM = 0, KF_CONV, KF_CONV_HALF, KF_GEMV, KF_GEMV_ROW, KF_BNN, KF_GATHER, KF_PROBE, KF_COUNT };
 
 struct DeviceCtx {
     int device = 0;
@@ -180,7 +180,7 @@ EE launch_gemm_tcgen05(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, con
     uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st);
 bool gemm_tcgen05_eligible(uint32_t M, uint32_t N, uint32_t K, const void *A, const void *B,
     uint32_t Kp, bool a_transposed);
-EE launch_gemm_simt(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed,
+EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed,
     const int8_t *B, uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st);
 EE launch_pack_rhs(const int8_t *src, bool src_is_nk, uint32_t N, uint32_t K, int8_t *dst,
     uint32_t Kp, uint32_t Np, int32_t *offsetC, cudaStream_t st);

@@ -1,9 +1,4 @@
-// gemm_i8_simt.cu -- weight packing (+ colsum offset) and the any-shape CUDA-core GEMM.
-//
-// The tensor-core kernel needs 16-byte aligned rows (K % 16 == 0, A row-major).  Everything
-// else -- ragged K, transposed A, the 1..33 shapes of Bolt's own cover test
-// (compute/blas_enhance/tests/test_mmm.cpp:165-171) -- runs here on dp4a-free integer math.
-// Same arithmetic, same epilogue.
+// pack_rhs.cu -- weight packing for the GEMM and GEMV kernels (K-major copy + column sums).
 #include "common.cuh"
 
 namespace b200 {
@@ -75,69 +70,6 @@ __global__ void scale_offset_kernel(int32_t *offsetC, uint32_t N)
     }
 }
 
-// ---- any-shape GEMM: one thread per output element, 16 x 16 tiles through shared memory ----------
-constexpr int TS = 16;
-__global__ void gemm_simt_kernel(uint32_t M, uint32_t N, uint32_t K, const uint8_t *__restrict__ A, int a_t,
-    const int8_t *__restrict__ B, uint32_t Kp, void *C, GemmEpilogue ep)
-{
-    __shared__ uint8_t sa[TS][TS + 1];
-    __shared__ int8_t sb[TS][TS + 1];
-    const uint32_t m = blockIdx.y * TS + threadIdx.y;
-    const uint32_t n = blockIdx.x * TS + threadIdx.x;
-    int acc = 0;
-    for (uint32_t k0 = 0; k0 < K; k0 += TS) {
-        {
-            // A tile: sa[row m][k]
-            const uint32_t k = k0 + threadIdx.x;
-            uint8_t v = 0;
-            if (m < M && k < K) {
-                v = a_t ? A[(size_t)k * M + m] : A[(size_t)m * K + k];
-            }
-            sa[threadIdx.y][threadIdx.x] = v;
-            // B tile: sb[col n][k], B is [Np][Kp]
-            const uint32_t nn = blockIdx.x * TS + threadIdx.y;
-            int8_t w = 0;
-            if (nn < N && k < K) {
-                w = B[(size_t)nn * Kp + k];
-            }
-            sb[threadIdx.y][threadIdx.x] = w;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < TS; ++k) {
-            acc += (int)sa[threadIdx.y][k] * (int)sb[threadIdx.x][k];
-        }
-        __syncthreads();
-    }
-    if (m >= M || n >= N) {
-        return;
-    }
-    if (ep.offsetC != nullptr) {
-        acc += ep.offsetC[n];
-    }
-    const size_t o = (size_t)m * N + n;
-    if (ep.out_kind != 2 && ep.accumulate) {
-        acc += reinterpret_cast<const int32_t *>(C)[o];
-    }
-    if (ep.out_kind == 0) {
-        reinterpret_cast<int32_t *>(C)[o] = acc;
-        return;
-    }
-    float fac = ep.factor;
-    if (ep.col_factor != nullptr) {
-        fac = ep.col_factor[n];
-    } else if (ep.per_channel) {
-        const float sa_ = ep.row_scale ? ep.row_scale[m] : (ep.sA_dev ? *ep.sA_dev : ep.sA);
-        const float sb_ = ep.col_scale ? ep.col_scale[n] : ep.sB;
-        fac = __fdiv_rn(ep.num, __fmul_rn(sa_, sb_));
-    }
-    if (ep.out_kind == 1) {
-        reinterpret_cast<float *>(C)[o] = acc_to_f32(acc, fac);
-    } else {
-        reinterpret_cast<uint8_t *>(C)[o] = (uint8_t)acc_to_u8(acc, fac);
-    }
-}
-
 }  // namespace
 
 EE launch_pack_rhs(const int8_t *src, bool src_is_nk, uint32_t N, uint32_t K, int8_t *dst, uint32_t Kp,
@@ -163,22 +95,6 @@ EE launch_pack_rhs(const int8_t *src, bool src_is_nk, uint32_t N, uint32_t K, in
             count_launch();
         }
     }
-    B200_CUDA(cudaGetLastError());
-    return SUCCESS;
-}
-
-EE launch_gemm_simt(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed, const int8_t *B,
-    uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st)
-{
-    if (M == 0 || N == 0) {
-        return SUCCESS;
-    }
-    dim3 grid((N + TS - 1) / TS, (M + TS - 1) / TS);
-    if (grid.y > 65535) {
-        return NOT_SUPPORTED;
-    }
-    gemm_simt_kernel<<<grid, dim3(TS, TS), 0, st>>>(M, N, K, A, a_transposed ? 1 : 0, B, Kp, C, ep);
-    count_launch();
     B200_CUDA(cudaGetLastError());
     return SUCCESS;
 }
