@@ -56,7 +56,7 @@ struct WeightTwin {
 
 // kernel families whose dynamic shared-memory limit has to be raised above 48 KiB; the attribute
 // belongs to the device that is current when it is set, so it is remembered per device context
-enum KernelFamily { KF_GEMM = 0, KF_CONV, KF_CONV_HALF, KF_GEMV, KF_GEMV_ROW, KF_BNN, KF_GATHER, KF_PROBE, KF_COUNT };
+enum KernelFamily { KF_GEMM = 0, KF_CONV, KF_CONV_HALF, KF_GEMV, KF_GEMV_ROW, KF_BNN, KF_GATHER, KF_MATMUL, KF_MATMUL_ROW, KF_PROBE, KF_COUNT };
 
 struct DeviceCtx {
     int device = 0;
@@ -182,6 +182,30 @@ bool gemm_tcgen05_eligible(uint32_t M, uint32_t N, uint32_t K, const void *A, co
     uint32_t Kp, bool a_transposed);
 EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed,
     const int8_t *B, uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st);
+
+// The products of one matmul call, C[i] = A[ia(i)] * B[ib(i)]
+struct MatmulOperand {
+    const void *p;
+    uint64_t elems;        // of all its products
+    int f32;               // binary32, quantized by the call (else u8 A / s8 B; M = 1: s8 A / u8 B)
+    int transposed;        // A: stored [K][M]; B: stored [N][K]
+    float scale;           // f32: lower bound of the dynamic scale, else the scale
+    uint32_t dims[4];      // batch extents
+    int direct;            // as many products as C has
+    unsigned *slots;       // f32: scratch for the partial maxima
+    uint64_t max_slots;
+};
+struct MatmulBatch {
+    uint32_t M, N, K;
+    uint64_t batches;
+    uint32_t c_dims[4];
+    MatmulOperand a, b;
+    void *C;
+    int out_kind;          // 1 fp32, 2 u8 with the scale c_scale
+    int accumulate;
+    float c_scale;
+};
+EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st);
 EE launch_pack_rhs(const int8_t *src, bool src_is_nk, uint32_t N, uint32_t K, int8_t *dst,
     uint32_t Kp, uint32_t Np, int32_t *offsetC, cudaStream_t st);
 EE launch_gemv_row(uint32_t N, uint32_t K, const uint8_t *Mx, bool transposed, const int8_t *v, void *y, int out_kind,

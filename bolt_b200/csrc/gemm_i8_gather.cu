@@ -14,6 +14,10 @@
 // CUDA-core kernel that stood here, 61 us with this one (about 40 us of both are the quantization and the host).
 #include <cuda.h>
 
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -31,21 +35,24 @@ constexpr int CTAS_PER_SM = 3;
 struct Ctl {
     uint64_t done[2];       // the MMAs reading a stage have completed
     uint32_t tmem_base;
+    float scale[2];         // of the two operands (batched products)
 };
 constexpr size_t SMEM_BYTES = 1024 + 2 * (size_t)(STAGE_A + MAX_BN * BLOCK_K) + sizeof(Ctl);
 static_assert(8 * 32 * EPI_PITCH * 4 <= 2 * (STAGE_A + 32 * BLOCK_K), "the epilogue staging reuses the operand stages");
 
 // where an operand lies: element (row, k)
 enum Layout {
-    ROWS_K = 0,   // p[row * ld + k]
-    K_ROWS = 1    // p[k * ld + row]
+    ROWS_K = 0,       // bytes p[row * ld + k]
+    K_ROWS = 1,       // bytes p[k * ld + row]
+    F32_ROWS_K = 2,   // the same two in binary32, quantized while they are loaded
+    F32_K_ROWS = 3
 };
 struct Operand {
     const uint8_t *p;
-    uint64_t ld;
+    uint64_t ld;       // in elements
     uint32_t rows;     // rows that exist
-    uint32_t k;        // bytes of K that may be read; zeros beyond
-    int vec;           // ROWS_K: 16, 8 or 1 (alignment of every row); K_ROWS: 4 or 1
+    uint32_t k;        // elements of K that may be read; zeros beyond
+    int vec;           // ROWS_K: 16, 8 or 1 (alignment of every row); K_ROWS: 4 or 1; F32_*: 1 if float4 loads are aligned
 };
 
 struct GatherParams {
@@ -55,6 +62,17 @@ struct GatherParams {
     GemmEpilogue ep;
     int vec_c;         // 4-element vectors of C are aligned
     int *status;
+};
+
+// The products of Bolt's matmul operator: one per batch index, operands quantized on the way in.
+struct BatchParams {
+    uint64_t batches;
+    uint32_t c_dims[4], a_dims[4], b_dims[4];   // batch extents, innermost first; an operand's may be smaller (broadcast)
+    int a_direct, b_direct;                     // as many products of the operand as of C: same index
+    uint64_t a_bytes, b_bytes, c_bytes;         // one product's operands and result
+    const unsigned *a_max, *b_max;              // partial maxima of |a|, |b| (float bits); null: the scale is a_scale, b_scale
+    uint32_t a_slots, b_slots;
+    float a_scale, b_scale, c_scale;
 };
 
 // 16 bytes from any address, of which the first n (>= 1) exist: aligned words that hold at least one of
@@ -82,9 +100,89 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t *p, uint32_t n)
     return make_uint4(r[0], r[1], r[2], r[3]);
 }
 
+// quantizeF32ToU8 (avx512/quantize.cpp:135-178) with the zero point taken off again, and quantizeF32ToI8 (:195-233)
+template <bool ZERO_POINT>
+__device__ __forceinline__ uint32_t quantize1(float x, float s)
+{
+    if (ZERO_POINT) {
+        return (uint32_t)(min(255, max(1, cvt_rne_x86(__fadd_rn(__fmul_rn(x, s), 128.0f)))) ^ 0x80);
+    }
+    return (uint32_t)(min(127, max(-127, cvt_rne_x86(__fmul_rn(x, s)))) & 0xFF);
+}
+template <bool ZERO_POINT>
+__device__ __forceinline__ uint32_t quantize4(float4 v, float s)
+{
+    const uint32_t lo = __byte_perm(quantize1<ZERO_POINT>(v.x, s), quantize1<ZERO_POINT>(v.y, s), 0x0040);
+    const uint32_t hi = __byte_perm(quantize1<ZERO_POINT>(v.z, s), quantize1<ZERO_POINT>(v.w, s), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
+}
+// the first n (0..4) of four floats
+__device__ __forceinline__ float4 load4f(const float *p, uint32_t n, int vec)
+{
+    if (vec && n == 4) {
+        return __ldg(reinterpret_cast<const float4 *>(p));
+    }
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    v.x = n > 0 ? __ldg(p) : 0.f;
+    v.y = n > 1 ? __ldg(p + 1) : 0.f;
+    v.z = n > 2 ? __ldg(p + 2) : 0.f;
+    v.w = n > 3 ? __ldg(p + 3) : 0.f;
+    return v;
+}
+__device__ __forceinline__ uint32_t first_bytes(uint32_t w, uint32_t n)
+{
+    return n >= 4 ? w : (n == 0 ? 0u : w & ((1u << (8 * n)) - 1u));
+}
+
+// The same tile from binary32.  Bytes beyond K are zeros (not quantized zeros).
+template <int LAYOUT, bool ZERO_POINT>
+__device__ __forceinline__ void load_tile_f32(const Operand &o, uint32_t r0, uint32_t rows_tile, uint32_t kb, uint8_t *dst, float s)
+{
+    const float *base = reinterpret_cast<const float *>(o.p);
+    const uint32_t k0 = kb * BLOCK_K;
+    const uint32_t left = o.k - k0;
+    const uint32_t sh = left <= 32 ? 3u : (left <= 64 ? 4u : 5u);   // words of 4 k per row: 8, 16 or 32
+    if (LAYOUT == F32_ROWS_K) {
+        // lanes along K: a thread makes one 4-byte word of a float4
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < (rows_tile << sh); i += THREADS) {
+            const uint32_t row = i >> sh, q = i & ((1u << sh) - 1u), k = k0 + q * 4;
+            uint32_t w = 0;
+            if (r0 + row < o.rows && k < o.k) {
+                const uint32_t n = min(4u, o.k - k);
+                w = first_bytes(quantize4<ZERO_POINT>(load4f(base + (uint64_t)(r0 + row) * o.ld + k, n, o.vec), s), n);
+            }
+            *reinterpret_cast<uint32_t *>(dst + row * 128 + (((q >> 2) ^ (row & 7)) << 4) + (q & 3) * 4) = w;
+        }
+    } else {
+        // 4 rows x 4 k per thread, transposed in registers; a warp covers 16 rows (64 bytes of each k) x 32 k
+#pragma unroll 2
+        for (uint32_t i = threadIdx.x; i < (rows_tile << sh) / 4; i += THREADS) {
+            const uint32_t rest = i >> 5;
+            const uint32_t q = (i & 7) + ((rest & ((1u << (sh - 3)) - 1u)) << 3), row = (((i >> 3) & 3) + ((rest >> (sh - 3)) << 2)) * 4;
+            const uint32_t k = k0 + q * 4, have = r0 + row < o.rows ? min(4u, o.rows - (r0 + row)) : 0u;
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                w[j] = 0;
+                if (k + j < o.k && have != 0) {
+                    w[j] = quantize4<ZERO_POINT>(load4f(base + (uint64_t)(k + j) * o.ld + r0 + row, have, o.vec), s);
+                }
+            }
+            const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+            const uint32_t d = __byte_perm(w[0], w[1], 0x7362), e = __byte_perm(w[2], w[3], 0x7362);
+            const uint32_t t[4] = {__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(d, e, 0x5410), __byte_perm(d, e, 0x7632)};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                *reinterpret_cast<uint32_t *>(dst + (row + j) * 128 + (((q >> 2) ^ ((row + j) & 7)) << 4) + (q & 3) * 4) = t[j];
+            }
+        }
+    }
+}
+
 // K block `kb` of rows [r0, r0 + rows_tile) into the 128-byte swizzled tile at `dst`: the 16-byte chunk c of row r
-// lies at r * 128 + ((c ^ (r & 7)) << 4).  Rows and bytes that do not exist become zeros.
-template <int LAYOUT>
+// lies at r * 128 + ((c ^ (r & 7)) << 4).  Rows and bytes that do not exist become zeros; then every byte is XORed.
+template <int LAYOUT, uint32_t XOR>
 __device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_t rows_tile, uint32_t kb, uint8_t *dst)
 {
     const uint32_t k0 = kb * BLOCK_K;
@@ -107,7 +205,7 @@ __device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_
                     v = load16_any(p, n);
                 }
             }
-            *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) = v;
+            *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(v.x ^ XOR, v.y ^ XOR, v.z ^ XOR, v.w ^ XOR);
         }
     } else {
         // a thread takes 4 rows x 16 k (sixteen 4-byte loads, lanes along the rows) and transposes in registers
@@ -144,7 +242,7 @@ __device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 *reinterpret_cast<uint4 *>(dst + (row + j) * 128 + ((c ^ ((row + j) & 7)) << 4)) =
-                    make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
+                    make_uint4(t[j][0] ^ XOR, t[j][1] ^ XOR, t[j][2] ^ XOR, t[j][3] ^ XOR);
             }
         }
     }
@@ -220,8 +318,47 @@ __device__ __forceinline__ void finish(const GatherParams &p, void *C, uint32_t 
     }
 }
 
-template <int LA>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_gather_kernel(const __grid_constant__ GatherParams p)
+// scale = max(given, 127 / max|x|), the dynamic scale of quantize (avx512/quantize.cpp:129-133), from the partial
+// maxima that absmax_pair_kernel left; called by a whole warp
+__device__ __forceinline__ float dynamic_scale(const unsigned *slots, uint32_t n, float given, uint32_t lane)
+{
+    unsigned m = 0;
+    for (uint32_t i = lane; i < n; i += 32) {
+        m = max(m, slots[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    const float mx = __uint_as_float(m);
+    const float s = (mx == 0.f) ? 1.0f : __fdiv_rn(127.0f, mx);
+    return (given > s) ? given : s;
+}
+// which of the operand's products goes with C's product `ic`
+__device__ __forceinline__ uint64_t batch_index(uint64_t ic, const uint32_t (&c)[4], const uint32_t (&x)[4], int direct)
+{
+    if (direct) {
+        return ic;
+    }
+    uint32_t idx[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        idx[i] = (uint32_t)(ic % c[i]);
+        ic /= c[i];
+    }
+    uint64_t g = 0;
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+        g = g * x[i] + (idx[i] < x[i] ? idx[i] : 0u);
+    }
+    return g;
+}
+
+// BATCH: A arrives as (or is made) signed by taking the zero point off, so that sum (a - 128) b needs no column sums:
+// it equals sum a b - 128 sum b in 32-bit arithmetic.
+template <int LA, int LB, bool BATCH>
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
+gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant__ BatchParams bp)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -244,22 +381,57 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_gather_kernel(const
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const uint32_t idesc = make_idesc_i8(p.block_n);
+    const uint32_t idesc = make_idesc_i8(p.block_n) | (BATCH ? 1u << 7 : 0u);   // bit 7: A is s8
     const uint32_t num_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
-    const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
+    const uint64_t per_batch = (uint64_t)p.tiles_m * p.tiles_n;
+    const uint64_t tiles = BATCH ? per_batch * bp.batches : per_batch;
+    Operand oa = p.a, ob = p.b;
+    void *C = p.C;
+    float scale_a = 0.f, scale_b = 0.f, factor = 0.f;
+    if (BATCH) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // the partial maxima (and everything before them) are there
+        if (warp < 2) {
+            const bool a = warp == 0;
+            const float given = a ? bp.a_scale : bp.b_scale;
+            const unsigned *slots = a ? bp.a_max : bp.b_max;
+            const float s = slots ? dynamic_scale(slots, a ? bp.a_slots : bp.b_slots, given, lane) : given;
+            if (lane == 0) {
+                ctl->scale[warp] = s;
+            }
+        }
+        __syncthreads();
+        scale_a = ctl->scale[0];
+        scale_b = ctl->scale[1];
+        factor = __fdiv_rn(p.ep.out_kind == 2 ? bp.c_scale : 1.0f, __fmul_rn(scale_a, scale_b));
+    }
     uint32_t issued = 0;   // K blocks handed to the tensor core so far: stage = issued & 1, parity from issued >> 1
     bool dead = false;
 
     for (uint64_t tile = blockIdx.x; tile < tiles && !dead; tile += gridDim.x) {
-        const uint32_t m0 = (uint32_t)(tile % p.tiles_m) * BLOCK_M, n0 = (uint32_t)(tile / p.tiles_m) * p.block_n;
+        const uint64_t batch = BATCH ? tile / per_batch : 0u;
+        const uint64_t in_batch = tile - batch * per_batch;
+        const uint32_t m0 = (uint32_t)(in_batch % p.tiles_m) * BLOCK_M, n0 = (uint32_t)(in_batch / p.tiles_m) * p.block_n;
+        if (BATCH) {
+            oa.p = p.a.p + batch_index(batch, bp.c_dims, bp.a_dims, bp.a_direct) * bp.a_bytes;
+            ob.p = p.b.p + batch_index(batch, bp.c_dims, bp.b_dims, bp.b_direct) * bp.b_bytes;
+            C = reinterpret_cast<uint8_t *>(p.C) + batch * bp.c_bytes;
+        }
         for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
             const uint32_t s = issued & 1;
             uint8_t *sa = smem + s * stage_bytes, *sb = sa + STAGE_A;
             // the MMAs that read this stage two K blocks ago are done
             bool ok = issued < 2 || mbar_wait(&ctl->done[s], ((issued >> 1) + 1) & 1);
             if (ok) {
-                load_tile<LA>(p.a, m0, BLOCK_M, kb, sa);
-                load_tile<ROWS_K>(p.b, n0, p.block_n, kb, sb);
+                if constexpr (LA >= F32_ROWS_K) {
+                    load_tile_f32<LA, true>(oa, m0, BLOCK_M, kb, sa, scale_a);
+                } else {
+                    load_tile<LA, BATCH ? 0x80808080u : 0u>(oa, m0, BLOCK_M, kb, sa);
+                }
+                if constexpr (LB >= F32_ROWS_K) {
+                    load_tile_f32<LB, false>(ob, n0, p.block_n, kb, sb, scale_b);
+                } else {
+                    load_tile<LB, 0u>(ob, n0, p.block_n, kb, sb);
+                }
                 fence_proxy_async_smem();
             }
             if (__syncthreads_or(!ok)) {
@@ -321,14 +493,14 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_gather_kernel(const
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         off[j] = p.ep.offsetC ? __ldg(p.ep.offsetC + n + j) : 0;
-                        cf[j] = p.ep.out_kind ? column_factor(p.ep, n + j) : 0.f;
+                        cf[j] = BATCH ? factor : (p.ep.out_kind ? column_factor(p.ep, n + j) : 0.f);
                     }
 #pragma unroll 4
                     for (uint32_t i = lane >> 3; i < 32; i += 4) {
                         if (mq + i < p.M) {
                             const int4 v = *reinterpret_cast<const int4 *>(stg + i * EPI_PITCH + (lane & 7) * 4);
                             int acc[4] = {v.x + off[0], v.y + off[1], v.z + off[2], v.w + off[3]};
-                            finish<4>(p, p.C, mq + i, n, acc, cf);
+                            finish<4>(p, C, mq + i, n, acc, cf);
                         }
                     }
                 }
@@ -336,12 +508,12 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_gather_kernel(const
                 const uint32_t n = nc + lane;
                 if (n < p.N) {
                     const int off = p.ep.offsetC ? __ldg(p.ep.offsetC + n) : 0;
-                    const float cf[1] = {p.ep.out_kind ? column_factor(p.ep, n) : 0.f};
+                    const float cf[1] = {BATCH ? factor : (p.ep.out_kind ? column_factor(p.ep, n) : 0.f)};
 #pragma unroll 4
                     for (uint32_t i = 0; i < 32; ++i) {
                         if (mq + i < p.M) {
                             int acc[1] = {stg[i * EPI_PITCH + lane] + off};
-                            finish<1>(p, p.C, mq + i, n, acc, cf);
+                            finish<1>(p, C, mq + i, n, acc, cf);
                         }
                     }
                 }
@@ -363,12 +535,188 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) gemm_gather_kernel(const
     }
 }
 
+// Partial maxima of |a| and |b| (float bits): the first ga blocks take a, the others b; block i of an operand writes
+// slot i.  No initial value and no atomic: whoever needs the scale reduces the few hundred slots itself.
+constexpr int MAX_THREADS = 512;
+__device__ __forceinline__ unsigned abs4(float4 v)
+{
+    return max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
+        max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu));
+}
+__global__ void __launch_bounds__(MAX_THREADS)
+absmax_pair_kernel(const float *a, uint64_t na, unsigned *a_slots, uint32_t ga, const float *b, uint64_t nb, unsigned *b_slots, uint32_t gb)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const bool first = blockIdx.x < ga;
+    const float *x = first ? a : b;
+    const uint64_t n = first ? na : nb;
+    const uint32_t blk = first ? blockIdx.x : blockIdx.x - ga;
+    const uint64_t stride = (uint64_t)(first ? ga : gb) * MAX_THREADS;
+    const uint64_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0;
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    unsigned m = 0;
+    uint64_t i = (uint64_t)blk * MAX_THREADS + threadIdx.x;
+    const uint64_t tid = i;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+        const float4 v0 = __ldg(x4 + i), v1 = __ldg(x4 + i + stride), v2 = __ldg(x4 + i + 2 * stride), v3 = __ldg(x4 + i + 3 * stride);
+        m = max(m, max(max(abs4(v0), abs4(v1)), max(abs4(v2), abs4(v3))));
+    }
+    for (; i < n4; i += stride) {
+        m = max(m, abs4(__ldg(x4 + i)));
+    }
+    for (uint64_t j = n4 * 4 + tid; j < n; j += stride) {
+        m = max(m, __float_as_uint(__ldg(x + j)) & 0x7FFFFFFFu);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    __shared__ unsigned warp_max[MAX_THREADS / 32];
+    if ((threadIdx.x & 31) == 0) {
+        warp_max[threadIdx.x >> 5] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < MAX_THREADS / 32; ++w) {
+            m = max(m, warp_max[w]);
+        }
+        (first ? a_slots : b_slots)[blk] = m;
+    }
+}
+
+__device__ __forceinline__ int dp4a_s8s8(uint32_t a, uint32_t b, int acc)
+{
+    int d;
+    asm("dp4a.s32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(acc));
+    return d;
+}
+// u8 results of the row GEMV: all but the last N % 4 rows through vpmovusdb, those add 128, compare signed with 255
+// and keep the low byte (mvm_avx512_vnni_row.cpp:384-406, 884-900)
+__device__ __forceinline__ void store_mvm(void *y, uint32_t n, uint32_t N, int acc, int out_kind, float factor)
+{
+    if (out_kind == 1) {
+        reinterpret_cast<float *>(y)[n] = acc_to_f32(acc, factor);
+    } else if (n >= N - (N % 4)) {
+        const int t = (int)((uint32_t)cvt_rne_x86(__fmul_rn(__int2float_rn(acc), factor)) + 128u);
+        reinterpret_cast<uint8_t *>(y)[n] = (t < 255) ? (uint8_t)t : (uint8_t)255;
+    } else {
+        reinterpret_cast<uint8_t *>(y)[n] = (uint8_t)acc_to_u8(acc, factor);
+    }
+}
+
+// A decoding step's attention is bound by reading the matrix; one query against 384 keys of 64 takes one block of
+// 32 keys x 64 per 8 KiB.
+// One row of C per product: y[n] = sum_k (m_u8[n, k] - 128) v_s8[k], the vector being A and the matrix B, both
+// quantized on the way in.  Blocks of 256 threads take MVM_ROWS rows n of one product at a time.
+// LB ROWS_K: 2^k lanes share a row, four k each, dp4a; LB K_ROWS: lanes along n, the warps split K.
+constexpr uint32_t MVM_ROWS = 32;
+template <int LB>
+__global__ void __launch_bounds__(THREADS)
+mvm_batch_kernel(const __grid_constant__ GatherParams p, const __grid_constant__ BatchParams bp, int a_f32)
+{
+    extern __shared__ __align__(16) uint8_t sv[];   // the vector as s8, zero padded to a multiple of 128
+    __shared__ float scales[2];
+    __shared__ int part[THREADS / 32][32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp < 2) {
+        const float given = warp == 0 ? bp.a_scale : bp.b_scale;
+        const unsigned *slots = warp == 0 ? bp.a_max : bp.b_max;
+        const float s = slots ? dynamic_scale(slots, warp == 0 ? bp.a_slots : bp.b_slots, given, lane) : given;
+        if (lane == 0) {
+            scales[warp] = s;
+        }
+    }
+    __syncthreads();
+    const float sa = scales[0], sb = scales[1];
+    const float factor = __fdiv_rn(p.ep.out_kind == 2 ? bp.c_scale : 1.0f, __fmul_rn(sa, sb));
+    const uint32_t blocks_n = (p.N + MVM_ROWS - 1) / MVM_ROWS;
+    const uint32_t k_pad = (p.K + 127) & ~127u;
+    for (uint64_t t = blockIdx.x; t < blocks_n * bp.batches; t += gridDim.x) {
+        const uint64_t batch = t / blocks_n;
+        const uint32_t n0 = (uint32_t)(t - batch * blocks_n) * MVM_ROWS;
+        const uint8_t *pa = p.a.p + batch_index(batch, bp.c_dims, bp.a_dims, bp.a_direct) * bp.a_bytes;
+        const uint8_t *pb = p.b.p + batch_index(batch, bp.c_dims, bp.b_dims, bp.b_direct) * bp.b_bytes;
+        uint8_t *y = reinterpret_cast<uint8_t *>(p.C) + batch * bp.c_bytes;
+        __syncthreads();   // the previous product's vector and partial sums have been read
+        for (uint32_t k = threadIdx.x; k < k_pad; k += THREADS) {
+            uint32_t v = 0;
+            if (k < p.K) {
+                v = a_f32 ? quantize1<false>(__ldg(reinterpret_cast<const float *>(pa) + k), sa) : (uint32_t)__ldg(pa + k);
+            }
+            sv[k] = (uint8_t)v;
+        }
+        __syncthreads();
+        if (LB == ROWS_K || LB == F32_ROWS_K) {
+            const uint32_t words = (p.K + 3) / 4;
+            uint32_t sh = 0;                       // 2^sh lanes per row
+            while (sh < 5 && (1u << sh) < words) {
+                ++sh;
+            }
+            const uint32_t per_warp = 32u >> sh, sub = lane & ((1u << sh) - 1u);
+            for (uint32_t r = warp * per_warp; r < MVM_ROWS; r += (THREADS / 32) * per_warp) {
+                const uint32_t n = n0 + r + (lane >> sh);
+                int acc = 0;
+                if (n < p.N && r + (lane >> sh) < MVM_ROWS) {
+                    for (uint32_t q = sub; q < words; q += 1u << sh) {
+                        const uint32_t have = min(4u, p.K - q * 4);
+                        uint32_t w;
+                        if (LB == F32_ROWS_K) {
+                            w = quantize4<true>(load4f(reinterpret_cast<const float *>(pb) + (uint64_t)n * p.K + q * 4, have, p.b.vec), sb);
+                        } else {
+                            const uint8_t *e = pb + (uint64_t)n * p.K + q * 4;
+                            if (p.b.vec >= 8 && have == 4) {
+                                w = __ldg(reinterpret_cast<const uint32_t *>(e));
+                            } else {
+                                w = 0;
+                                for (uint32_t j = 0; j < have; ++j) {
+                                    w |= (uint32_t)__ldg(e + j) << (8 * j);
+                                }
+                            }
+                            w ^= 0x80808080u;
+                        }
+                        // (beyond K the vector is zero)
+                        acc = dp4a_s8s8(w, *reinterpret_cast<const uint32_t *>(sv + q * 4), acc);
+                    }
+                }
+                for (uint32_t o = (1u << sh) >> 1; o > 0; o >>= 1) {
+                    acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                }
+                if (sub == 0 && n < p.N && r + (lane >> sh) < MVM_ROWS) {
+                    store_mvm(y, n, p.N, acc, p.ep.out_kind, factor);
+                }
+            }
+        } else {
+            const uint32_t n = n0 + lane;
+            int acc = 0;
+            if (n < p.N) {
+#pragma unroll 8
+                for (uint32_t k = warp; k < p.K; k += THREADS / 32) {
+                    const uint64_t e = (uint64_t)k * p.N + n;
+                    const uint32_t q = LB == F32_K_ROWS ? quantize1<true>(__ldg(reinterpret_cast<const float *>(pb) + e), sb) : ((uint32_t)__ldg(pb + e) ^ 0x80u);
+                    acc += (int)(int8_t)q * (int)(int8_t)sv[k];
+                }
+            }
+            part[warp][lane] = acc;
+            __syncthreads();
+            if (warp == 0 && n < p.N) {
+#pragma unroll
+                for (int w = 1; w < THREADS / 32; ++w) {
+                    acc += part[w][lane];
+                }
+                store_mvm(y, n, p.N, acc, p.ep.out_kind, factor);
+            }
+        }
+    }
+}
+
 // Tile width: as few column blocks of at most 128 as cover N, narrower while there are fewer tiles than SMs.
-uint32_t pick_bn(uint32_t tiles_m, uint32_t N, int sms)
+uint32_t pick_bn(uint64_t tiles_m, uint32_t N, int sms)
 {
     const uint32_t blocks = (N + MAX_BN - 1) / MAX_BN;
     uint32_t bn = (uint32_t)B200_ALIGN((N + blocks - 1) / blocks, 32);
-    while (bn > 32 && (uint64_t)tiles_m * ((N + bn - 1) / bn) < (uint64_t)sms) {
+    while (bn > 32 && tiles_m * ((N + bn - 1) / bn) < (uint64_t)sms) {
         bn -= 32;
     }
     return bn;
@@ -397,7 +745,7 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
         return UNKNOWN;
     }
     {
-        const void *ks[2] = {(const void *)gemm_gather_kernel<ROWS_K>, (const void *)gemm_gather_kernel<K_ROWS>};
+        const void *ks[2] = {(const void *)gemm_gather_kernel<ROWS_K, ROWS_K, false>, (const void *)gemm_gather_kernel<K_ROWS, ROWS_K, false>};
         B200_EE(raise_smem_limit(c, KF_GATHER, ks, 2, SMEM_BYTES));
     }
     GatherParams p;
@@ -426,12 +774,197 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
     const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n, slots = (uint64_t)c->sm_count * CTAS_PER_SM;
     const uint32_t grid = (uint32_t)(tiles < slots ? tiles : slots);
     if (a_transposed) {
-        gemm_gather_kernel<K_ROWS><<<grid, THREADS, SMEM_BYTES, st>>>(p);
+        gemm_gather_kernel<K_ROWS, ROWS_K, false><<<grid, THREADS, SMEM_BYTES, st>>>(p, BatchParams());
     } else {
-        gemm_gather_kernel<ROWS_K><<<grid, THREADS, SMEM_BYTES, st>>>(p);
+        gemm_gather_kernel<ROWS_K, ROWS_K, false><<<grid, THREADS, SMEM_BYTES, st>>>(p, BatchParams());
     }
     count_launch();
     B200_CUDA(cudaGetLastError());
+    return SUCCESS;
+}
+
+namespace {
+
+template <int LA, int LB>
+cudaError_t launch_batch(uint32_t grid, const GatherParams &p, const BatchParams &bp, const cudaLaunchConfig_t &base)
+{
+    cudaLaunchConfig_t cfg = base;
+    cfg.gridDim = dim3(grid);
+    return cudaLaunchKernelEx(&cfg, gemm_gather_kernel<LA, LB, true>, p, bp);
+}
+template <int LA>
+cudaError_t launch_batch_b(int lb, uint32_t grid, const GatherParams &p, const BatchParams &bp, const cudaLaunchConfig_t &base)
+{
+    switch (lb) {
+        case ROWS_K:
+            return launch_batch<LA, ROWS_K>(grid, p, bp, base);
+        case K_ROWS:
+            return launch_batch<LA, K_ROWS>(grid, p, bp, base);
+        case F32_ROWS_K:
+            return launch_batch<LA, F32_ROWS_K>(grid, p, bp, base);
+        default:
+            return launch_batch<LA, F32_K_ROWS>(grid, p, bp, base);
+    }
+}
+template <int LA>
+void batch_kernels(const void **ks)
+{
+    ks[0] = (const void *)gemm_gather_kernel<LA, ROWS_K, true>;
+    ks[1] = (const void *)gemm_gather_kernel<LA, K_ROWS, true>;
+    ks[2] = (const void *)gemm_gather_kernel<LA, F32_ROWS_K, true>;
+    ks[3] = (const void *)gemm_gather_kernel<LA, F32_K_ROWS, true>;
+}
+bool programmatic_launch()
+{
+    static const bool on = [] {
+        const char *e = getenv("BOLT_B200_NO_PDL");
+        return !(e != nullptr && e[0] != '\0' && e[0] != '0');
+    }();
+    return on;
+}
+Operand operand(const MatmulOperand &o, uint32_t rows, uint32_t K, bool rows_contiguous)
+{
+    Operand r;
+    r.p = reinterpret_cast<const uint8_t *>(o.p);
+    r.ld = rows_contiguous ? rows : K;
+    r.rows = rows;
+    r.k = K;
+    const uint64_t a = reinterpret_cast<uintptr_t>(o.p);
+    if (o.f32) {
+        r.vec = (a % 16 == 0) && (r.ld % 4 == 0);
+    } else if (rows_contiguous) {
+        r.vec = ((a | r.ld) % 4 == 0) ? 4 : 1;
+    } else {
+        r.vec = row_alignment(o.p, r.ld);
+    }
+    return r;
+}
+
+}  // namespace
+
+// All products of a matmul call: at most one pass over the binary32 operands for their scales, then one kernel that
+// quantizes, multiplies and converts.  BERT-base attention of 32 x 128 tokens, scores and context (384 products of
+// 128 x 64 x 128 and of 128 x 128 x 64): 57 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
+// floor is 15 us (each operand and result once); the operands are read a second time for their scales.
+EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
+{
+    DeviceCtx *c = ctx();
+    if (c == nullptr) {
+        return UNKNOWN;
+    }
+    const size_t mvm_smem = B200_ALIGN((size_t)mb.K, 128);
+    if (mb.M == 1 && mvm_smem > 200 * 1024) {
+        return NOT_SUPPORTED;
+    }
+    {
+        const void *ks[16];
+        batch_kernels<ROWS_K>(ks);
+        batch_kernels<K_ROWS>(ks + 4);
+        batch_kernels<F32_ROWS_K>(ks + 8);
+        batch_kernels<F32_K_ROWS>(ks + 12);
+        B200_EE(raise_smem_limit(c, KF_MATMUL, ks, 16, SMEM_BYTES));
+        const void *kv[4] = {(const void *)mvm_batch_kernel<ROWS_K>, (const void *)mvm_batch_kernel<K_ROWS>,
+            (const void *)mvm_batch_kernel<F32_ROWS_K>, (const void *)mvm_batch_kernel<F32_K_ROWS>};
+        B200_EE(raise_smem_limit(c, KF_MATMUL_ROW, kv, 4, 200 * 1024));
+    }
+    GatherParams p;
+    std::memset(&p, 0, sizeof(p));
+    BatchParams bp;
+    std::memset(&bp, 0, sizeof(bp));
+    p.M = mb.M;
+    p.N = mb.N;
+    p.K = mb.K;
+    p.a = operand(mb.a, mb.M, mb.K, mb.a.transposed);
+    p.b = operand(mb.b, mb.N, mb.K, !mb.b.transposed);
+    p.C = mb.C;
+    p.ep.out_kind = mb.out_kind;
+    p.ep.accumulate = mb.accumulate;
+    p.status = c->d_status;
+    bp.batches = mb.batches;
+    for (int i = 0; i < 4; ++i) {
+        bp.c_dims[i] = mb.c_dims[i];
+        bp.a_dims[i] = mb.a.dims[i];
+        bp.b_dims[i] = mb.b.dims[i];
+    }
+    bp.a_direct = mb.a.direct;
+    bp.b_direct = mb.b.direct;
+    bp.a_bytes = (uint64_t)mb.M * mb.K * (mb.a.f32 ? 4 : 1);
+    bp.b_bytes = (uint64_t)mb.N * mb.K * (mb.b.f32 ? 4 : 1);
+    const uint32_t esz = mb.out_kind == 2 ? 1 : 4;
+    bp.c_bytes = (uint64_t)mb.M * mb.N * esz;
+    bp.a_scale = mb.a.scale;
+    bp.b_scale = mb.b.scale;
+    bp.c_scale = mb.c_scale;
+    // every product starts at a multiple of its size, so the vectors' alignment has to hold for that too
+    auto all_batches = [&](Operand &o, const MatmulOperand &m, uint64_t bytes) {
+        if (m.f32) {
+            o.vec = o.vec && (bytes % 16 == 0 || mb.batches == 1);
+        } else if (m.transposed != (&m == &mb.b)) {
+            o.vec = (bytes % 4 == 0 || mb.batches == 1) ? o.vec : 1;
+        } else if (mb.batches != 1 && bytes % 16 != 0) {
+            o.vec = (bytes % 8 == 0 && o.vec >= 8) ? 8 : 1;
+        }
+    };
+    all_batches(p.a, mb.a, bp.a_bytes);
+    all_batches(p.b, mb.b, bp.b_bytes);
+    p.vec_c = (mb.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(mb.C) | (mb.batches == 1 ? 0 : bp.c_bytes)) % (4 * esz) == 0);
+
+    // partial maxima: 64 KiB of operand per block at least, two blocks per SM at most, and no more slots than given
+    auto blocks_for = [&](const MatmulOperand &o) -> uint32_t {
+        if (!o.f32) {
+            return 0;
+        }
+        uint64_t g = (o.elems + 4 * MAX_THREADS - 1) / (4 * MAX_THREADS);
+        g = std::min<uint64_t>(g, 2 * (uint64_t)c->sm_count);
+        return (uint32_t)std::min<uint64_t>(g, o.max_slots);
+    };
+    const uint32_t ga = blocks_for(mb.a), gb = blocks_for(mb.b);
+    bp.a_max = ga ? mb.a.slots : nullptr;
+    bp.b_max = gb ? mb.b.slots : nullptr;
+    bp.a_slots = ga;
+    bp.b_slots = gb;
+    if (ga + gb) {
+        absmax_pair_kernel<<<ga + gb, MAX_THREADS, 0, st>>>(reinterpret_cast<const float *>(mb.a.p), mb.a.elems, mb.a.slots, ga,
+            reinterpret_cast<const float *>(mb.b.p), mb.b.elems, mb.b.slots, gb);
+        count_launch();
+        B200_CUDA(cudaGetLastError());
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = (ga + gb) && programmatic_launch() ? 1 : 0;   // its set-up runs beside the reduction
+    const int la = (mb.a.f32 ? 2 : 0) + (mb.a.transposed ? 1 : 0);
+    const int lb = (mb.b.f32 ? 2 : 0) + (mb.b.transposed ? 0 : 1);
+    cudaError_t e;
+    if (mb.M == 1) {
+        const uint64_t work = (uint64_t)((mb.N + MVM_ROWS - 1) / MVM_ROWS) * mb.batches;
+        cfg.gridDim = dim3((uint32_t)std::min<uint64_t>(work, 8 * (uint64_t)c->sm_count));
+        cfg.dynamicSmemBytes = mvm_smem;
+        const int af = mb.a.f32 ? 1 : 0;
+        e = lb == ROWS_K ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<ROWS_K>, p, bp, af)
+            : lb == K_ROWS ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<K_ROWS>, p, bp, af)
+            : lb == F32_ROWS_K ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<F32_ROWS_K>, p, bp, af)
+                               : cudaLaunchKernelEx(&cfg, mvm_batch_kernel<F32_K_ROWS>, p, bp, af);
+    } else {
+        p.tiles_m = (mb.M + BLOCK_M - 1) / BLOCK_M;
+        p.block_n = pick_bn((uint64_t)p.tiles_m * mb.batches, mb.N, c->sm_count);
+        p.tiles_n = (mb.N + p.block_n - 1) / p.block_n;
+        p.tmem_cols = p.block_n > 64 ? 128u : p.block_n;
+        cfg.dynamicSmemBytes = SMEM_BYTES;
+        const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n * mb.batches;
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)c->sm_count * CTAS_PER_SM);
+        e = la == ROWS_K ? launch_batch_b<ROWS_K>(lb, grid, p, bp, cfg)
+            : la == K_ROWS ? launch_batch_b<K_ROWS>(lb, grid, p, bp, cfg)
+            : la == F32_ROWS_K ? launch_batch_b<F32_ROWS_K>(lb, grid, p, bp, cfg)
+                               : launch_batch_b<F32_K_ROWS>(lb, grid, p, bp, cfg);
+        tls().last_gemm_tc = 1;
+    }
+    count_launch();
+    B200_CUDA(e);
     return SUCCESS;
 }
 

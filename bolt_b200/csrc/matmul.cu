@@ -1,13 +1,16 @@
 // matmul.cu -- the int8 branch of Bolt's `matmul` operator (compute/tensor/src/matmul.cpp:303-557) for
 // CUDA_B200: both operands may arrive as fp32 and are quantized per call (dynamic scale 127 / absmax, or the
-// scale the tensor carries), B is an activation and is therefore packed on the fly for every batch, the
-// product runs on the tensor-core GEMM (or on a GEMV kernel when the result is a row or a column), and the
-// result is written as fp32 (accumulator / (scaleA * scaleB)) or requantized to u8.
+// scale the tensor carries), and the result is written as fp32 (accumulator / (scaleA * scaleB)) or requantized
+// to u8.  All products of a call run in one launch that quantizes its operands while it loads them
+// (launch_matmul_batch); a single large product, and a result of one column, take the quantize / pack / multiply
+// kernels one after the other.
 //
 // The x86 convention applies (matmul.cpp:373-398): u8 activations with zero point 128 times s8, except
 // when the result is a vector, where A becomes s8 and B u8.  Leading (batch) dimensions broadcast as in
-// matmul.cpp:489-517.  All work is enqueued on the thread's stream; scales come back to the host, which is
-// what the operator's interface (Tensor::get_scale) requires.
+// matmul.cpp:489-517.  All work is enqueued on the thread's stream; the scale of a dynamically requantized u8 result
+// comes back to the host, which is what the operator's interface (Tensor::get_scale) requires.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -177,6 +180,38 @@ U32 global_index(uint64_t ic, const TensorDesc &c, const TensorDesc &x)
     return g;
 }
 
+// One launch for all products, or one product after the other through quantize, pack and the TMA GEMM?  The batched
+// kernel never packs and keeps the host out of it, but it converts an fp32 operand again for every tile row / column
+// of the other one and fills the tensor pipe a quarter as well.  Measured (fp32 in and out, us per call, one launch
+// against one by one): 1 x 512^3 37 / 75, 1 x 1024^3 73 / 83, 1 x 2048^3 209 / 112; 4 x 512^3 42 / 123,
+// 4 x 1024^3 112 / 145, 4 x 2048^3 903 / 272; 384 x (128 x 64 x 128 and 128 x 128 x 64) 57 / 8000 for the pair.
+bool one_launch(const Plan &p)
+{
+    const uint64_t M = p.a.dims[1 - p.kDimA], N = p.b.dims[1 - p.kDimB], K = p.a.dims[p.kDimA];
+    if (M == 1) {
+        return true;    // a row per product: the batched GEMV
+    }
+    return N != 1 && M * N <= (1ull << 30) / K;
+}
+
+// the scratch of the batched kernel: an operand's partial maxima lie where its quantized copy would
+MatmulOperand batch_operand(const void *data, const TensorDesc &d, bool f32, int transposed, F32 scale, uint64_t loops, uint64_t loopsC, char *scratch)
+{
+    MatmulOperand o;
+    o.p = data;
+    o.elems = elems(d);
+    o.f32 = f32 ? 1 : 0;
+    o.transposed = transposed;
+    o.scale = scale;
+    for (U32 i = 0; i < 4; ++i) {
+        o.dims[i] = i + 2 < d.nDims ? d.dims[i + 2] : 1;
+    }
+    o.direct = loops == loopsC;
+    o.slots = reinterpret_cast<unsigned *>(scratch);
+    o.max_slots = B200_ALIGN(o.elems, 256) / 4;
+    return o;
+}
+
 }  // namespace
 }  // namespace b200
 
@@ -317,10 +352,15 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
         return NOT_MATCH;
     }
 
-    char *t = reinterpret_cast<char *>(tmp);
+    const bool fused = one_launch(p);
+    // (the tmp bytes count 1 KiB more than what is laid out in it)
+    char *t = fused ? reinterpret_cast<char *>(B200_ALIGN(reinterpret_cast<uintptr_t>(tmp), 16)) : reinterpret_cast<char *>(tmp);
+    char *slotsA = t, *slotsB = t + (p.quantA ? B200_ALIGN(nA, 256) : 0);
     F32 scaleO = 1;
     // operands: quantize into tmp, or take the caller's quantized bytes and scale (matmul.cpp:401-421)
-    if (p.quantA) {
+    if (fused) {
+        t = slotsB + (p.quantB ? B200_ALIGN(nB, 256) : 0);
+    } else if (p.quantA) {
         F32 s = aScale;
         TensorDesc q = p.a;
         q.dt = p.qa;
@@ -331,7 +371,9 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
     } else {
         scaleO *= aScale;
     }
-    if (p.quantB) {
+    if (fused) {
+        // the scales are found and used on the device
+    } else if (p.quantB) {
         F32 s = bScale;
         TensorDesc q = p.b;
         q.dt = p.qb;
@@ -363,24 +405,37 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
         fill_rows_kernel<<<grid, 256, 0, st>>>(reinterpret_cast<uint8_t *>(prod), prod_bytes,
             reinterpret_cast<const uint8_t *>(bias), (uint32_t)bias_bytes);
         count_launch();
-    } else {
+    } else if (!fused) {
         B200_CUDA(cudaMemsetAsync(prod, 0, prod_bytes, st));
     }
 
+    if (fused) {
+        MatmulBatch mb;
+        mb.M = p.a.dims[1 - p.kDimA];
+        mb.N = p.b.dims[1 - p.kDimB];
+        mb.K = p.a.dims[p.kDimA];
+        mb.batches = p.loopsC;
+        for (U32 i = 0; i < 4; ++i) {
+            mb.c_dims[i] = i + 2 < p.c.nDims ? p.c.dims[i + 2] : 1;
+        }
+        mb.a = batch_operand(A, p.a, p.quantA, p.dfA == DF_TRANSPOSE, aScale, p.loopsA, p.loopsC, slotsA);
+        mb.b = batch_operand(B, p.b, p.quantB, p.dfB == DF_TRANSPOSE, bScale, p.loopsB, p.loopsC, slotsB);
+        mb.C = prod;
+        mb.out_kind = p.static_u8 ? 2 : 1;
+        mb.accumulate = bias_bytes && !p.static_u8 ? 1 : 0;
+        mb.c_scale = *cScale;
+        B200_EE(launch_matmul_batch(mb, st));
+    }
     const size_t a2 = (size_t)p.a.dims[0] * p.a.dims[1], b2 = (size_t)p.b.dims[0] * p.b.dims[1];
     const size_t c2 = (size_t)p.c.dims[0] * p.c.dims[1] * bytes_of(p.qc);
-    for (uint64_t ic = 0; ic < p.loopsC; ++ic) {
+    for (uint64_t ic = 0; !fused && ic < p.loopsC; ++ic) {
         const uint64_t ia = p.loopsA == p.loopsC ? ic : global_index(ic, p.c, p.a);
         const uint64_t ib = p.loopsB == p.loopsC ? ic : global_index(ic, p.c, p.b);
         const char *pa = reinterpret_cast<const char *>(A) + ia * a2;
         const char *pb = reinterpret_cast<const char *>(B) + ib * b2;
         char *pc = reinterpret_cast<char *>(prod) + ic * c2;
         EE ret;
-        if (p.a.dims[1 - p.kDimA] == 1) {
-            ret = b200_matrix_vector_multiply(
-                desc2d(p.qb, p.dfB == DF_TRANSPOSE ? DF_NORMAL : DF_TRANSPOSE, p.b.dims[1], p.b.dims[0]), pb,
-                desc1d(p.qa, p.a.dims[p.kDimA]), pa, p.mmm_bytes, t, desc1d(p.qc, p.c.dims[0]), pc, scalePtr, CUDA_B200);
-        } else if (p.b.dims[1 - p.kDimB] == 1) {
+        if (p.b.dims[1 - p.kDimB] == 1) {
             ret = b200_matrix_vector_multiply(desc2d(p.qa, p.dfA, p.a.dims[1], p.a.dims[0]), pa,
                 desc1d(p.qb, p.b.dims[p.kDimB]), pb, p.mmm_bytes, t, desc1d(p.qc, p.c.dims[1]), pc, scalePtr, CUDA_B200);
         } else {
@@ -392,7 +447,7 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
     }
     // matmul.cpp:535-554: a u8 output without a given scale is quantized from the fp32 product
     if (p.stageC) {
-        F32 scales[2] = {*cScale, scaleO};
+        F32 scales[2] = {*cScale, scaleO};   // (of an fp32 source only the first is read)
         TensorDesc src = p.c;
         src.dt = p.qc;
         B200_EE(quantize_cuda_b200(&src, prod, &p.c, C, scales, 0));

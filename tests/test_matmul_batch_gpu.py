@@ -1,0 +1,63 @@
+"""GPU parity of the matmul operator's one-launch form at the edges of its tiles: every operand type and storage
+order, broadcast batches, results of one row; bit for bit against the oracle."""
+import itertools
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(__file__))
+import oracle as O  # noqa: E402
+import bolt_b200 as B  # noqa: E402
+from bolt_b200 import synth  # noqa: E402
+from test_matmul_gpu import matmul_gpu  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+F, U, I = B.DT_F32, B.DT_U8_Q, B.DT_I8
+
+
+def check(args):
+    C, s = matmul_gpu(*args)
+    Cp, sp = O.port_matmul(*args)
+    assert C.tobytes() == Cp.tobytes() and np.float32(s) == np.float32(sp)
+
+
+def operand(seed, shape, dt):
+    return synth.normal(seed, shape) if dt == F else (synth.u8(seed, shape) if dt == U else synth.s8(seed, shape))
+
+
+@pytest.mark.parametrize("m,k,n", [(2, 3, 5), (7, 31, 8), (32, 64, 129), (129, 65, 31), (130, 257, 100), (128, 128, 64)])
+@pytest.mark.parametrize("a_dt", [F, U])
+@pytest.mark.parametrize("b_dt", [F, I])
+def test_products(m, k, n, a_dt, b_dt):
+    for ta, tb in itertools.product((0, 1), (0, 1)):
+        a = operand(1, (3, k, m) if ta else (3, m, k), a_dt)
+        b = operand(2, (3, n, k) if tb else (3, k, n), b_dt)
+        sa, sb = (-1.0 if a_dt == F else 11.0), (-1.0 if b_dt == F else 7.0)
+        check((a, a_dt, sa, ta, b, b_dt, sb, tb, None, F, -1.0))
+        check((a, a_dt, sa, ta, b, b_dt, sb, tb, None, U, 3.0))
+
+
+@pytest.mark.parametrize("k,n", [(3, 5), (64, 384), (384, 64), (130, 33)])
+@pytest.mark.parametrize("a_dt", [F, I])
+@pytest.mark.parametrize("b_dt", [F, U])
+def test_one_row(k, n, a_dt, b_dt):
+    for tb, c_scale in itertools.product((0, 1), (-1.0, 3.0)):
+        a, b = operand(3, (2, 5, 1, k), a_dt), operand(4, (2, 5, n, k) if tb else (2, 5, k, n), b_dt)
+        sa, sb = (-1.0 if a_dt == F else 9.0), (-1.0 if b_dt == F else 13.0)
+        check((a, a_dt, sa, 0, b, b_dt, sb, tb, None, F if c_scale < 0 else U, c_scale))
+
+
+def test_broadcast_bias_and_scale_edges():
+    a, b = synth.normal(5, (4, 3, 20, 24)), synth.normal(6, (1, 3, 24, 40))
+    check((a, F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0))
+    check((a[:, :1], F, -1.0, 0, synth.normal(7, (4, 3, 24, 40)), F, -1.0, 0, None, F, -1.0))
+    check((a, F, -1.0, 0, b, F, -1.0, 0, synth.normal(8, (40,)), F, -1.0))
+    check((a, F, 500.0, 0, b, F, -1.0, 0, None, F, -1.0))              # a given scale above the dynamic one wins
+    check((np.zeros_like(a), F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0))
+
+
+def test_single_large_product_goes_one_by_one():
+    a, b = synth.normal(9, (1, 1040, 1024)), synth.normal(10, (1, 1024, 1040))
+    check((a, F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0))
