@@ -8,24 +8,34 @@
 //   DoReFa  : sum = popcount(x AND w)
 //   output  = fma_fp16( (fp16)(int16)sum, scale[oc], bias[oc] ), fp16 NCHWc8
 //
-// Three kernels: binarise + zero-pad the fp16 NCHWc8 input into [N][Hp][Wp][C/32] words (one
-// streaming pass, 16x smaller than the input), repack the filter bits into [OC][tap][C/32] words
-// (once), and the convolution: a CTA owns 128 output pixels x 64 output channels, keeps its weight
-// slice in shared memory (read as 128-bit broadcasts), each thread one pixel with 64 integer
-// accumulators in registers; XOR/AND + __popc on 32 channels at a time; fp16 fused multiply-add
-// epilogue, 16-byte stores.  The work is bound by the popcount rate (16 per clock per SM), not by
-// HBM: 3x3, C = 256 needs 72 word-operations per output, the bytes are 50x less than that.
+// Three kernels: binarise + zero-pad the fp16 NCHWc8 input into bit words [N][C/32][Hp][Wp] (one streaming pass, 16x
+// smaller than the input), repack the filter bits into [OC][tap][C/32] words (once), and the convolution: an implicit
+// GEMM on the tensor cores (kind::i8), pixels x output channels x (tap, word, bit).  Only the bits travel through
+// memory; a CTA's threads widen them to bytes while they fill the operand stages -- activations to 0 / 1, weights to
+// -1 / +1 (XNOR) or 0 / 1 (DoReFa) -- and with
+//     acc = sum_valid x * (2w - 1),   fh*fw*ic - 2 popcount(x XOR w) = 2 acc + fh*fw*ic - 2 popcount(w)
+// the padding (x = 0) needs no treatment.  The order of the 32 bits of a word inside its 32 bytes of K is free as
+// long as both operands use the same one: word j of 8 takes bits j, j+8, j+16, j+24, one shift and one mask.
+//
+// Measured, 256 -> 256 channels, 3 x 3 on 28 x 28, batch 128, whole call: 519 us with XOR + popcount (16 per clock and
+// SM: 411 us of popcounts alone), 141 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
 #include <cuda_fp16.h>
 
 #include <cstring>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace b200 {
 namespace {
 
-constexpr int PIX_TILE = 128;
-constexpr int OC_TILE = 64;
+using namespace tc;
+
+constexpr int THREADS = 256;
+constexpr int MAX_BN = 128;                       // output channels of a tile
+constexpr int STAGE_A = 2 * BLOCK_M * BLOCK_K;    // two row blocks: 256 pixels
+constexpr int STAGE = STAGE_A + MAX_BN * BLOCK_K; // 48 KiB; two stages, two CTAs per SM
+constexpr uint32_t MAX_WORDS = 800;               // (tap, word) pairs of a filter
 
 struct B4d {
     DataType dt;
@@ -68,16 +78,16 @@ __global__ void bnn_pack_filter_kernel(const uint8_t *__restrict__ src, uint32_t
     }
 }
 
-// fp16 NCHWc8 -> bit words [N][Hp][Wp][Cw], zero words in the padding ring
+// fp16 NCHWc8 -> bit words [N][Cw][Hp][Wp], zero words in the padding ring.  Lanes run along the row, so that both
+// the 16-byte reads of a channel block and the 4-byte writes are contiguous.
 __global__ void bnn_binarize_pad_kernel(const __half *__restrict__ in, uint32_t N, uint32_t IC, uint32_t IH, uint32_t IW,
     uint32_t Hp, uint32_t Wp, uint32_t pt, uint32_t pl, uint32_t Cw, float threshold, uint32_t *__restrict__ out)
 {
-    const size_t total = (size_t)N * Hp * Wp * Cw;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t cw = (uint32_t)(i % Cw);
-        const uint32_t x = (uint32_t)((i / Cw) % Wp);
-        const uint32_t y = (uint32_t)((i / ((size_t)Cw * Wp)) % Hp);
-        const uint32_t n = (uint32_t)(i / ((size_t)Cw * Wp * Hp));
+    const uint32_t total = N * Hp * Wp * Cw;   // the scratch is smaller than 4 GiB, so words count in 32 bits
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const uint32_t row = i / Wp, x = i - row * Wp;
+        const uint32_t pl_ = row / Hp, y = row - pl_ * Hp;
+        const uint32_t n = pl_ / Cw, cw = pl_ - n * Cw;
         uint32_t word = 0;
         const int iy = (int)y - (int)pt, ix = (int)x - (int)pl;
         if (iy >= 0 && iy < (int)IH && ix >= 0 && ix < (int)IW) {
@@ -105,97 +115,276 @@ __global__ void bnn_binarize_pad_kernel(const __half *__restrict__ in, uint32_t 
 
 struct BnnParams {
     uint32_t N, OH, OW, OC, Hp, Wp, Cw, FH, FW, sH, sW;
-    uint32_t kbits;  // fh * fw * ic
-    int xnor;
+    uint32_t kbits;     // fh * fw * ic
+    uint32_t kw_words;  // fh * fw * Cw
+    uint32_t row_blocks, block_n, tiles_m, tiles_n, tmem_cols;   // tile: row_blocks (1 or 2) x 128 pixels, block_n channels
     const uint32_t *xb;
     const uint32_t *wb;
     const __half *scale;
     const __half *bias;
     __half *out;
+    int *status;
 };
 
-template <bool XNOR>
-__global__ void __launch_bounds__(PIX_TILE)
-bnn_conv_kernel(const BnnParams p)
+struct BnnCtl {
+    uint64_t done[2];
+    uint32_t tmem_base;
+    __align__(16) int corr[MAX_BN];      // XNOR: kbits - 2 popcount(w) of every channel of the tile
+    __half2 scale[MAX_BN / 2], bias[MAX_BN / 2];
+};
+constexpr size_t BNN_SMEM = 1024 + 2 * (size_t)STAGE + sizeof(BnnCtl);
+
+// 32 bits -> 32 bytes of 0 / 1 (or of -1 / +1), two 16-byte chunks
+template <bool SIGNS>
+__device__ __forceinline__ uint32_t widen(uint32_t w, int j)
 {
-    extern __shared__ __align__(16) uint32_t sw[];  // [OC_TILE][taps * Cw] padded to a multiple of 4 words
-    const uint32_t taps = p.FH * p.FW;
-    const uint32_t kw_words = taps * p.Cw;
-    const uint32_t kw_pad = (kw_words + 3) & ~3u;
-    const uint32_t oc0 = blockIdx.y * OC_TILE;
-    for (uint32_t i = threadIdx.x; i < OC_TILE * kw_pad; i += blockDim.x) {
-        const uint32_t o = i / kw_pad, k = i - o * kw_pad;
-        sw[i] = (oc0 + o < p.OC && k < kw_words) ? p.wb[(size_t)(oc0 + o) * kw_words + k] : 0u;
+    const uint32_t t = (w >> j) & 0x01010101u;
+    if (!SIGNS) {
+        return t;
     }
+    const uint32_t u = t ^ 0x01010101u;
+    return (u * 255u) | t;
+}
+template <bool SIGNS>
+__device__ __forceinline__ void store_word(uint8_t *tile, uint32_t row, uint32_t word, uint32_t w, bool valid)
+{
+    uint32_t v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = widen<SIGNS>(w, j);
+        if (SIGNS && !valid) {
+            v[j] = 0;   // beyond K (the activations are zero there too, but only one side has to be)
+        }
+    }
+    uint8_t *r = tile + row * 128;
+    *reinterpret_cast<uint4 *>(r + (((2 * word) ^ (row & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<uint4 *>(r + (((2 * word + 1) ^ (row & 7)) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
+}
+
+// Tile = up to 256 pixels x up to 128 channels; K in blocks of 4 words = 128 bytes.  256 threads: each widens the
+// word (threadIdx & 3) of rows threadIdx / 4, + 64, + 128, + 192 of the pixels and of rows + 0, + 64 of the weights;
+// the words of K block k+1 are fetched while block k is widened, and two stages let the MMAs of block k run beside
+// the widening of block k+1.  Two CTAs share an SM, so one's epilogue runs beside the other's MMAs.
+template <bool XNOR>
+__global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_constant__ BnnParams p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    BnnCtl *ctl = reinterpret_cast<BnnCtl *>(smem + 2 * STAGE);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        mbar_init(&ctl->done[0], 1);
+        mbar_init(&ctl->done[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)),
+                     "r"(p.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
     __syncthreads();
-    const size_t npix = (size_t)p.N * p.OH * p.OW;
-    const size_t pidx = (size_t)blockIdx.x * PIX_TILE + threadIdx.x;
-    if (pidx >= npix) {
-        return;
-    }
-    const uint32_t ow = (uint32_t)(pidx % p.OW);
-    const uint32_t oh = (uint32_t)((pidx / p.OW) % p.OH);
-    const uint32_t n = (uint32_t)(pidx / ((size_t)p.OW * p.OH));
-    int acc[OC_TILE];
+    tcgen05_fence_after();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t tmem_base = ctl->tmem_base;
+    const uint32_t idesc = make_idesc_i8(p.block_n);
+    const uint32_t num_kb = (p.kw_words + 3) / 4;
+    const uint32_t tiles = p.tiles_m * p.tiles_n;
+    const uint32_t npix = p.N * p.OH * p.OW;
+    const uint32_t plane = p.Hp * p.Wp;
+    const uint32_t word = threadIdx.x & 3, row0 = threadIdx.x >> 2;
+    const uint32_t a_rows = 2 * p.row_blocks, b_rows = (p.block_n + 63) / 64;   // rows of 64 this thread serves
+    uint32_t issued = 0, staged_n0 = 0xFFFFFFFFu;
+    bool dead = false;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t m0 = (tile % p.tiles_m) * p.row_blocks * BLOCK_M, n0 = (tile / p.tiles_m) * p.block_n;
+        if (n0 != staged_n0) {
+            // constants of the tile's channels (the previous tile's epilogue is over: it ended with a barrier)
+            for (uint32_t o = warp; o < p.block_n; o += THREADS / 32) {
+                int ones = 0;
+                if (XNOR && n0 + o < p.OC) {
+                    for (uint32_t k = lane; k < p.kw_words; k += 32) {
+                        ones += __popc(__ldg(p.wb + (size_t)(n0 + o) * p.kw_words + k));
+                    }
 #pragma unroll
-    for (int o = 0; o < OC_TILE; ++o) {
-        acc[o] = 0;
-    }
-    // walk K four words at a time: one 128-bit broadcast read of the weights per output channel
-    for (uint32_t k4 = 0; k4 < kw_pad; k4 += 4) {
-        uint32_t x[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t k = k4 + j;
-            uint32_t v = 0;
-            if (k < kw_words) {
-                const uint32_t tap = k / p.Cw, cw = k - tap * p.Cw;
-                const uint32_t kh = tap / p.FW, kw = tap - kh * p.FW;
-                v = __ldg(p.xb + (((size_t)n * p.Hp + oh * p.sH + kh) * p.Wp + ow * p.sW + kw) * p.Cw + cw);
+                    for (int s = 16; s > 0; s >>= 1) {
+                        ones += __shfl_xor_sync(0xffffffffu, ones, s);
+                    }
+                }
+                if (lane == 0) {
+                    const bool in = n0 + o < p.OC;
+                    ctl->corr[o] = (int)p.kbits - 2 * ones;
+                    reinterpret_cast<__half *>(ctl->scale)[o] = in ? p.scale[n0 + o] : __half(0.f);
+                    reinterpret_cast<__half *>(ctl->bias)[o] = in ? p.bias[n0 + o] : __half(0.f);
+                }
             }
-            x[j] = v;
+            staged_n0 = n0;
+        }
+        // first word of this thread's pixels (tap 0, word 0) and weights
+        uint32_t xo[4], wo[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t pix = m0 + row0 + 64 * i;
+            xo[i] = 0xFFFFFFFFu;
+            if ((uint32_t)i < a_rows && pix < npix) {
+                const uint32_t ow = pix % p.OW, t = pix / p.OW, oh = t % p.OH, n = t / p.OH;
+                xo[i] = (n * p.Cw * p.Hp + oh * p.sH) * p.Wp + ow * p.sW;
+            }
         }
 #pragma unroll
-        for (int o = 0; o < OC_TILE; ++o) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(sw + o * kw_pad + k4);
-            if (XNOR) {
-                acc[o] += __popc(x[0] ^ w.x) + __popc(x[1] ^ w.y) + __popc(x[2] ^ w.z) + __popc(x[3] ^ w.w);
-            } else {
-                acc[o] += __popc(x[0] & w.x) + __popc(x[1] & w.y) + __popc(x[2] & w.z) + __popc(x[3] & w.w);
-            }
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t o = row0 + 64 * i;
+            wo[i] = ((uint32_t)i < b_rows && o < p.block_n && n0 + o < p.OC) ? (n0 + o) * p.kw_words : 0xFFFFFFFFu;
         }
-    }
-    // epilogue: int16 sum -> fp16 (round to nearest even), one fused multiply-add, 8 channels = 16 bytes
-    const size_t plane = (size_t)p.OH * p.OW;
-    const size_t pix = (size_t)oh * p.OW + ow;
+        // this thread's word of K block kb is k = 4 kb + word = (kh, kw, cw)
+        uint32_t k = word, cw = word % p.Cw, tap = word / p.Cw, kw = tap % p.FW, kh = tap / p.FW;
+        uint32_t xa[4], wa[2];
+        bool valid = false;
+        auto fetch = [&]() {
+            valid = k < p.kw_words;
+            const uint32_t off = cw * plane + kh * p.Wp + kw;
 #pragma unroll
-    for (int ob = 0; ob < OC_TILE; ob += 8) {
-        const uint32_t oc = oc0 + ob;
-        if (oc >= p.OC) {
+            for (int i = 0; i < 4; ++i) {
+                xa[i] = (valid && xo[i] != 0xFFFFFFFFu) ? __ldg(p.xb + xo[i] + off) : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                wa[i] = (valid && wo[i] != 0xFFFFFFFFu) ? __ldg(p.wb + wo[i] + k) : 0u;
+            }
+            k += 4;
+            cw += 4;
+            while (cw >= p.Cw) {
+                cw -= p.Cw;
+                if (++kw == p.FW) {
+                    kw = 0;
+                    ++kh;
+                }
+            }
+        };
+        fetch();
+        for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
+            const uint32_t s = issued & 1;
+            uint8_t *sa = smem + s * STAGE, *sb = sa + STAGE_A;
+            const bool ok = issued < 2 || mbar_wait(&ctl->done[s], ((issued >> 1) + 1) & 1);
+            if (ok) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if ((uint32_t)i < a_rows) {
+                        store_word<false>(sa, row0 + 64 * i, word, xa[i], valid);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (row0 + 64 * i < p.block_n) {
+                        store_word<XNOR>(sb, row0 + 64 * i, word, wa[i], valid);
+                    }
+                }
+                fence_proxy_async_smem();
+                fetch();
+            }
+            if (__syncthreads_or(!ok)) {
+                dead = true;
+                break;
+            }
+            if (threadIdx.x == 0) {
+                tcgen05_fence_after();
+                const uint64_t db = make_desc_sw128(smem_u32(sb));
+                for (uint32_t r = 0; r < p.row_blocks; ++r) {
+                    const uint64_t da = make_desc_sw128(smem_u32(sa + r * BLOCK_M * BLOCK_K));
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        umma_i8(tmem_base + r * MAX_BN, da + 2 * q, db + 2 * q, idesc, (kb | q) != 0 ? 1u : 0u);
+                    }
+                }
+                tcgen05_commit(&ctl->done[s]);
+            }
+            __syncwarp();
+        }
+        if (dead) {
             break;
         }
-        unsigned short h[8];
+        {
+            const uint32_t last = issued - 1;
+            const bool ok = mbar_wait(&ctl->done[last & 1], (last >> 1) & 1);
+            if (__syncthreads_or(!ok)) {
+                dead = true;
+                break;
+            }
+        }
+        tcgen05_fence_after();
+        // epilogue: int16 sum -> fp16 (round to nearest even), one fused multiply-add, 8 channels = 16 bytes; a lane is
+        // a pixel, so 32 lanes write 512 contiguous bytes.  Warp = lane quadrant x (row block, or half of the channels).
+        const uint32_t quad = warp & 3, half = warp >> 2, nch = p.block_n >> 5;
+        const uint32_t r = p.row_blocks == 2 ? half : 0u;
+        const uint32_t c_begin = p.row_blocks == 2 ? 0u : (half ? (nch + 1) / 2 : 0u);
+        const uint32_t c_end = p.row_blocks == 2 ? nch : (half ? nch : (nch + 1) / 2);
+        const uint32_t pix = m0 + r * BLOCK_M + quad * 32 + lane;
+        const uint32_t n = pix / (p.OH * p.OW);
+        const size_t oplane = (size_t)p.OH * p.OW;
+        __half *dst = p.out + (size_t)n * p.OC * oplane + (size_t)(pix - n * (uint32_t)oplane) * 8;
+        for (uint32_t c = c_begin; c < c_end; ++c) {
+            uint32_t acc[32];
+            tmem_ld32(tmem_base + ((quad * 32u) << 16) + r * MAX_BN + c * 32, acc);
+            tmem_ld_wait(acc);
+            if (pix < npix) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            int s = XNOR ? ((int)p.kbits - 2 * acc[ob + j]) : acc[ob + j];
-            const __half hs = __short2half_rn((short)s);
-            __half r = hs;
-            if (oc + j < p.OC) {
-                r = __hfma(hs, p.scale[oc + j], p.bias[oc + j]);
+                for (int ob = 0; ob < 32; ob += 8) {
+                    const uint32_t oc = n0 + c * 32 + ob;
+                    if (oc < p.OC) {
+                        uint32_t h[4];
+#pragma unroll
+                        for (int j = 0; j < 8; j += 2) {
+                            const uint32_t o = c * 32 + ob + j;
+                            int s0 = (int)acc[ob + j], s1 = (int)acc[ob + j + 1];
+                            if (XNOR) {
+                                const int2 co = *reinterpret_cast<const int2 *>(ctl->corr + o);
+                                s0 = 2 * s0 + co.x;
+                                s1 = 2 * s1 + co.y;
+                            }
+                            // int16 -> fp16 by way of binary32, which holds every int16 exactly
+                            const __half2 hs = __floats2half2_rn((float)(short)s0, (float)(short)s1);
+                            const __half2 v = __hfma2(hs, ctl->scale[o >> 1], ctl->bias[o >> 1]);
+                            h[j >> 1] = *reinterpret_cast<const uint32_t *>(&v);
+                        }
+                        *reinterpret_cast<uint4 *>(dst + (size_t)oc * oplane) = make_uint4(h[0], h[1], h[2], h[3]);
+                    }
+                }
             }
-            h[j] = __half_as_ushort(r);
         }
-        const uint32_t width = min(8u, p.OC - oc);
-        __half *dst = p.out + ((size_t)n * p.OC + oc) * plane + pix * width;
-        if (width == 8) {
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16),
-                h[4] | ((uint32_t)h[5] << 16), h[6] | ((uint32_t)h[7] << 16));
-        } else {
-            for (uint32_t j = 0; j < width; ++j) {
-                dst[j] = __ushort_as_half(h[j]);
-            }
-        }
+        tcgen05_fence_before();
+        __syncthreads();
+        tcgen05_fence_after();
     }
+    if (dead && threadIdx.x == 0) {
+        atomicExch(p.status, 41);
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
+    }
+}
+
+// Tile: 256 pixels x 128 channels where that leaves every SM its two CTAs; with fewer tiles than that, one row block
+// of 128 pixels and then narrower channel blocks.
+void pick_tile(uint64_t npix, uint32_t OC, int sms, BnnParams *p)
+{
+    const uint32_t blocks = (OC + MAX_BN - 1) / MAX_BN;
+    uint32_t bn = (uint32_t)B200_ALIGN((OC + blocks - 1) / blocks, 32), rb = 2;
+    auto tiles = [&] { return ((npix + rb * BLOCK_M - 1) / (rb * BLOCK_M)) * ((OC + bn - 1) / bn); };
+    if (tiles() < 2 * (uint64_t)sms) {
+        rb = 1;
+    }
+    while (bn > 32 && tiles() < (uint64_t)sms) {
+        bn -= 32;
+    }
+    p->row_blocks = rb;
+    p->block_n = bn;
+    p->tiles_m = (uint32_t)((npix + rb * BLOCK_M - 1) / (rb * BLOCK_M));
+    p->tiles_n = (OC + bn - 1) / bn;
+    p->tmem_cols = rb == 2 ? 256u : (bn > 64 ? 128u : bn);
 }
 
 struct BnnGeom {
@@ -342,6 +531,10 @@ EE bnn_run(const TensorDesc *inputDesc, const void *input, const TensorDesc *fil
         d_tmp == nullptr) {
         return ALLOC_FAILED;
     }
+    const size_t npix = (size_t)g.out.n * g.out.h * g.out.w;
+    if (((g.taps * g.Cw + 3) & ~3u) > MAX_WORDS) {
+        return NOT_SUPPORTED;
+    }
     uint32_t *d_xb = reinterpret_cast<uint32_t *>(B200_ALIGN(reinterpret_cast<uintptr_t>(d_tmp), 256));
     {
         const size_t words = g.xb_bytes / 4;
@@ -366,27 +559,24 @@ EE bnn_run(const TensorDesc *inputDesc, const void *input, const TensorDesc *fil
     p.sH = g.sH;
     p.sW = g.sW;
     p.kbits = g.f.h * g.f.w * g.f.c;
-    p.xnor = xnor ? 1 : 0;
+    p.kw_words = g.taps * g.Cw;
     p.xb = d_xb;
     p.wb = d_w;
     p.scale = d_scale;
     p.bias = d_bias;
     p.out = d_out;
-    const uint32_t kw_pad = (g.taps * g.Cw + 3) & ~3u;
-    const size_t smem = (size_t)OC_TILE * kw_pad * 4;
-    if (smem > 200 * 1024) {
-        return NOT_SUPPORTED;
-    }
+    p.status = c->d_status;
+    pick_tile(npix, p.OC, c->sm_count, &p);
     {
         const void *ks[2] = {(const void *)bnn_conv_kernel<true>, (const void *)bnn_conv_kernel<false>};
-        B200_EE(raise_smem_limit(c, KF_BNN, ks, 2, 200 * 1024));
+        B200_EE(raise_smem_limit(c, KF_BNN, ks, 2, BNN_SMEM));
     }
-    const size_t npix = (size_t)g.out.n * g.out.h * g.out.w;
-    dim3 grid((uint32_t)((npix + PIX_TILE - 1) / PIX_TILE), (g.out.c + OC_TILE - 1) / OC_TILE);
+    const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n;
+    const uint32_t grid = (uint32_t)(tiles < 2 * (uint64_t)c->sm_count ? tiles : 2 * (uint64_t)c->sm_count);
     if (xnor) {
-        bnn_conv_kernel<true><<<grid, PIX_TILE, smem, st>>>(p);
+        bnn_conv_kernel<true><<<grid, THREADS, BNN_SMEM, st>>>(p);
     } else {
-        bnn_conv_kernel<false><<<grid, PIX_TILE, smem, st>>>(p);
+        bnn_conv_kernel<false><<<grid, THREADS, BNN_SMEM, st>>>(p);
     }
     count_launch();
     B200_CUDA(cudaGetLastError());
