@@ -11,7 +11,7 @@
 // these products are bound by latency and by the load / store instructions, not by the tensor pipe.
 //
 // Measured, 333 x 515 x 1001 u8 x s8 -> fp32 behind its dynamic quantization, whole calls: 111 us with the 16 x 16
-// CUDA-core kernel that stood here, 61 us with this one (about 40 us of both are the quantization and the host).
+// CUDA-core kernel that stood here, 50 us with this one (about 40 us of both are the quantization and the host).
 #include <cuda.h>
 
 #include <algorithm>
@@ -75,19 +75,22 @@ struct BatchParams {
     float a_scale, b_scale, c_scale;
 };
 
-// 16 bytes from any address, of which the first n (>= 1) exist: aligned words that hold at least one of
-// them, shifted into place
-__device__ __forceinline__ uint4 load16_any(const uint8_t *p, uint32_t n)
+// 16 bytes from any address, of which the first n (0..16) exist: the aligned words that hold at least one of
+// them ...
+__device__ __forceinline__ void load_words(const uint8_t *p, uint32_t n, uint32_t (&v)[5])
 {
     const uintptr_t a = reinterpret_cast<uintptr_t>(p);
     const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    const uint32_t lead = (uint32_t)(a & 3);
-    const uint32_t end = lead + n;
-    uint32_t v[5];
+    const uint32_t end = n ? (uint32_t)(a & 3) + n : 0u;
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
         v[j] = (4u * j < end) ? __ldg(w + j) : 0u;
     }
+}
+// ... shifted into place
+__device__ __forceinline__ uint4 shift_words(const uint8_t *p, uint32_t n, const uint32_t (&v)[5])
+{
+    const uint32_t lead = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
     uint32_t r[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -116,13 +119,13 @@ __device__ __forceinline__ uint32_t quantize4(float4 v, float s)
     const uint32_t hi = __byte_perm(quantize1<ZERO_POINT>(v.z, s), quantize1<ZERO_POINT>(v.w, s), 0x0040);
     return __byte_perm(lo, hi, 0x5410);
 }
-// the first n (0..4) of four floats
+// the first n (0..4) of four floats; with aligned vectors the extents are multiples of 4
 __device__ __forceinline__ float4 load4f(const float *p, uint32_t n, int vec)
 {
-    if (vec && n == 4) {
-        return __ldg(reinterpret_cast<const float4 *>(p));
+    if (vec) {   // n is 0 or 4
+        return n ? __ldg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v;
     v.x = n > 0 ? __ldg(p) : 0.f;
     v.y = n > 1 ? __ldg(p + 1) : 0.f;
     v.z = n > 2 ? __ldg(p + 2) : 0.f;
@@ -142,39 +145,69 @@ __device__ __forceinline__ void load_tile_f32(const Operand &o, uint32_t r0, uin
     const uint32_t k0 = kb * BLOCK_K;
     const uint32_t left = o.k - k0;
     const uint32_t sh = left <= 32 ? 3u : (left <= 64 ? 4u : 5u);   // words of 4 k per row: 8, 16 or 32
+    // eight float4 per thread are on their way before the first is used
     if (LAYOUT == F32_ROWS_K) {
         // lanes along K: a thread makes one 4-byte word of a float4
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < (rows_tile << sh); i += THREADS) {
-            const uint32_t row = i >> sh, q = i & ((1u << sh) - 1u), k = k0 + q * 4;
-            uint32_t w = 0;
-            if (r0 + row < o.rows && k < o.k) {
-                const uint32_t n = min(4u, o.k - k);
-                w = first_bytes(quantize4<ZERO_POINT>(load4f(base + (uint64_t)(r0 + row) * o.ld + k, n, o.vec), s), n);
-            }
-            *reinterpret_cast<uint32_t *>(dst + row * 128 + (((q >> 2) ^ (row & 7)) << 4) + (q & 3) * 4) = w;
-        }
-    } else {
-        // 4 rows x 4 k per thread, transposed in registers; a warp covers 16 rows (64 bytes of each k) x 32 k
-#pragma unroll 2
-        for (uint32_t i = threadIdx.x; i < (rows_tile << sh) / 4; i += THREADS) {
-            const uint32_t rest = i >> 5;
-            const uint32_t q = (i & 7) + ((rest & ((1u << (sh - 3)) - 1u)) << 3), row = (((i >> 3) & 3) + ((rest >> (sh - 3)) << 2)) * 4;
-            const uint32_t k = k0 + q * 4, have = r0 + row < o.rows ? min(4u, o.rows - (r0 + row)) : 0u;
-            uint32_t w[4];
+        const uint32_t total = rows_tile << sh;
+        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 8 * THREADS) {
+            float4 v[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                w[j] = 0;
-                if (k + j < o.k && have != 0) {
-                    w[j] = quantize4<ZERO_POINT>(load4f(base + (uint64_t)(k + j) * o.ld + r0 + row, have, o.vec), s);
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t i = i0 + u * THREADS, row = i >> sh, k = k0 + (i & ((1u << sh) - 1u)) * 4;
+                const uint32_t n = (i < total && r0 + row < o.rows && k < o.k) ? min(4u, o.k - k) : 0u;
+                v[u] = load4f(base + (uint64_t)(r0 + row) * o.ld + k, n, o.vec);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t i = i0 + u * THREADS, row = i >> sh, q = i & ((1u << sh) - 1u), k = k0 + q * 4;
+                if (i < total) {
+                    const uint32_t n = k < o.k ? min(4u, o.k - k) : 0u;
+                    *reinterpret_cast<uint32_t *>(dst + row * 128 + (((q >> 2) ^ (row & 7)) << 4) + (q & 3) * 4) =
+                        first_bytes(quantize4<ZERO_POINT>(v[u], s), n);
                 }
             }
-            const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
-            const uint32_t d = __byte_perm(w[0], w[1], 0x7362), e = __byte_perm(w[2], w[3], 0x7362);
-            const uint32_t t[4] = {__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(d, e, 0x5410), __byte_perm(d, e, 0x7632)};
+        }
+    } else {
+        // 4 rows x 4 k, transposed in registers; a warp covers 16 rows (64 bytes of each k) x 32 k
+        const uint32_t total = (rows_tile << sh) / 4;
+        auto place = [&](uint32_t i, uint32_t &q, uint32_t &row) {
+            const uint32_t rest = i >> 5;
+            q = (i & 7) + ((rest & ((1u << (sh - 3)) - 1u)) << 3);
+            row = (((i >> 3) & 3) + ((rest >> (sh - 3)) << 2)) * 4;
+        };
+        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 2 * THREADS) {
+            float4 v[2][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                *reinterpret_cast<uint32_t *>(dst + (row + j) * 128 + (((q >> 2) ^ ((row + j) & 7)) << 4) + (q & 3) * 4) = t[j];
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t i = i0 + u * THREADS;
+                uint32_t q, row;
+                place(i, q, row);
+                const uint32_t k = k0 + q * 4, have = (i < total && r0 + row < o.rows) ? min(4u, o.rows - (r0 + row)) : 0u;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[u][j] = load4f(base + (uint64_t)(k + j) * o.ld + r0 + row, k + j < o.k ? have : 0u, o.vec);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t i = i0 + u * THREADS;
+                uint32_t q, row;
+                place(i, q, row);
+                if (i < total) {
+                    const uint32_t k = k0 + q * 4;
+                    uint32_t w[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        w[j] = k + j < o.k ? quantize4<ZERO_POINT>(v[u][j], s) : 0u;
+                    }
+                    const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+                    const uint32_t d = __byte_perm(w[0], w[1], 0x7362), e = __byte_perm(w[2], w[3], 0x7362);
+                    const uint32_t t[4] = {__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632), __byte_perm(d, e, 0x5410), __byte_perm(d, e, 0x7632)};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        *reinterpret_cast<uint32_t *>(dst + (row + j) * 128 + (((q >> 2) ^ ((row + j) & 7)) << 4) + (q & 3) * 4) = t[j];
+                    }
+                }
             }
         }
     }
@@ -187,25 +220,51 @@ __device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_
 {
     const uint32_t k0 = kb * BLOCK_K;
     if (LAYOUT == ROWS_K) {
-        // a thread moves 16-byte chunks; eight neighbouring lanes cover one row's 128 bytes
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < rows_tile * 8; i += THREADS) {
-            const uint32_t row = i >> 3, c = i & 7, k = k0 + c * 16;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (r0 + row < o.rows && k < o.k) {
-                const uint8_t *p = o.p + (uint64_t)(r0 + row) * o.ld + k;
-                const uint32_t n = min(16u, o.k - k);
-                if (o.vec == 16 && n == 16) {
-                    v = __ldg(reinterpret_cast<const uint4 *>(p));
-                } else if (o.vec >= 8 && (n & 7) == 0) {
-                    const uint2 lo = __ldg(reinterpret_cast<const uint2 *>(p));
-                    const uint2 hi = n == 16 ? __ldg(reinterpret_cast<const uint2 *>(p) + 1) : make_uint2(0, 0);
-                    v = make_uint4(lo.x, lo.y, hi.x, hi.y);
-                } else {
-                    v = load16_any(p, n);
-                }
+        // a thread moves 16-byte chunks, all (at most four) on their way before the first is stored; eight neighbouring
+        // lanes cover one row's 128 bytes
+        constexpr int CH = BLOCK_M * 8 / THREADS;
+        const uint32_t c = threadIdx.x & 7, row0 = threadIdx.x >> 3, k = k0 + c * 16;
+        const uint8_t *p0 = o.p + (uint64_t)(r0 + row0) * o.ld + k;
+        const uint64_t step = (uint64_t)(THREADS / 8) * o.ld;
+        const uint32_t bytes = k < o.k ? min(16u, o.k - k) : 0u;
+        uint32_t n[CH];
+        uint4 v[CH];
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const uint32_t row = row0 + i * (THREADS / 8);
+            n[i] = (row < rows_tile && r0 + row < o.rows) ? bytes : 0u;
+        }
+        if (o.vec == 16) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                v[i] = n[i] ? __ldg(reinterpret_cast<const uint4 *>(p0 + i * step)) : make_uint4(0, 0, 0, 0);
             }
-            *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(v.x ^ XOR, v.y ^ XOR, v.z ^ XOR, v.w ^ XOR);
+        } else if (o.vec == 8) {
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                const uint2 *p = reinterpret_cast<const uint2 *>(p0 + i * step);
+                const uint2 lo = n[i] ? __ldg(p) : make_uint2(0, 0);
+                const uint2 hi = n[i] == 16 ? __ldg(p + 1) : make_uint2(0, 0);
+                v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            }
+        } else {
+            uint32_t w[CH][5];
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                load_words(p0 + i * step, n[i], w[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                v[i] = shift_words(p0 + i * step, n[i], w[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const uint32_t row = row0 + i * (THREADS / 8);
+            if (row < rows_tile) {
+                *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) =
+                    make_uint4(v[i].x ^ XOR, v[i].y ^ XOR, v[i].z ^ XOR, v[i].w ^ XOR);
+            }
         }
     } else {
         // a thread takes 4 rows x 16 k (sixteen 4-byte loads, lanes along the rows) and transposes in registers
@@ -215,17 +274,18 @@ __device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_
             const uint32_t left = r0 + row < o.rows ? o.rows - (r0 + row) : 0u;
             const uint8_t *p = o.p + (uint64_t)k * o.ld + r0 + row;
             uint32_t w[16];
+            if (o.vec == 4) {   // (then the number of rows is a multiple of 4 too)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                w[j] = 0;
-                if (k + j < o.k && left != 0) {
-                    const uint8_t *q = p + (uint64_t)j * o.ld;
-                    if (o.vec == 4 && left >= 4) {
-                        w[j] = __ldg(reinterpret_cast<const uint32_t *>(q));
-                    } else {
-                        for (uint32_t t = 0; t < min(left, 4u); ++t) {
-                            w[j] |= (uint32_t)__ldg(q + t) << (8 * t);
-                        }
+                for (int j = 0; j < 16; ++j) {
+                    w[j] = (k + j < o.k && left != 0) ? __ldg(reinterpret_cast<const uint32_t *>(p + (uint64_t)j * o.ld)) : 0u;
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    w[j] = 0;
+#pragma unroll
+                    for (uint32_t t = 0; t < 4; ++t) {
+                        w[j] |= (k + j < o.k && t < left) ? (uint32_t)__ldg(p + (uint64_t)j * o.ld + t) << (8 * t) : 0u;
                     }
                 }
             }
@@ -264,24 +324,27 @@ __device__ __forceinline__ float column_factor(const GemmEpilogue &ep, uint32_t 
     return __fdiv_rn(ep.num, __fmul_rn(ep.sA_dev ? *ep.sA_dev : ep.sA, sb));
 }
 
+// what C holds in V consecutive columns of row m
+template <int V>
+__device__ __forceinline__ void read_c(const GatherParams &p, const void *C, uint32_t m, uint32_t n, int (&acc)[V])
+{
+    const int32_t *cin = reinterpret_cast<const int32_t *>(C) + (size_t)m * p.N + n;
+    if (V == 4) {
+        const int4 v = *reinterpret_cast<const int4 *>(cin);
+        acc[0] = v.x;
+        acc[1 % V] = v.y;
+        acc[2 % V] = v.z;
+        acc[3 % V] = v.w;
+    } else {
+        acc[0] = cin[0];
+    }
+}
 // V consecutive results of row m, columns n .. n+V-1
 template <int V>
-__device__ __forceinline__ void finish(const GatherParams &p, void *C, uint32_t m, uint32_t n, int (&acc)[V], const float (&cf)[V])
+__device__ __forceinline__ void finish(const GatherParams &p, void *C, uint32_t m, uint32_t n, const int (&acc)[V], const float (&cf)[V])
 {
     const GemmEpilogue &ep = p.ep;
     const size_t o = (size_t)m * p.N + n;
-    if (ep.out_kind != 2 && ep.accumulate) {
-        const int32_t *cin = reinterpret_cast<const int32_t *>(C) + o;
-        if (V == 4) {
-            const int4 v = *reinterpret_cast<const int4 *>(cin);
-            acc[0] += v.x;
-            acc[1 % V] += v.y;
-            acc[2 % V] += v.z;
-            acc[3 % V] += v.w;
-        } else {
-            acc[0] += cin[0];
-        }
-    }
     if (ep.out_kind == 0) {
         int32_t *out = reinterpret_cast<int32_t *>(C) + o;
         if (V == 4) {
@@ -466,6 +529,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
         const uint32_t quad = warp & 3, half = warp >> 2, nch = p.block_n >> 5;
         const uint32_t c_begin = half ? (nch + 1) / 2 : 0u, c_end = half ? nch : (nch + 1) / 2;
         int32_t *stg = reinterpret_cast<int32_t *>(smem) + warp * 32 * EPI_PITCH;
+        const bool add_c = p.ep.out_kind != 2 && p.ep.accumulate;   // its reads go out together, before the first store
         for (uint32_t c = c_begin; c < c_end; ++c) {
             uint32_t r[32];
             if (num_kb != 0) {
@@ -495,12 +559,27 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                         off[j] = p.ep.offsetC ? __ldg(p.ep.offsetC + n + j) : 0;
                         cf[j] = BATCH ? factor : (p.ep.out_kind ? column_factor(p.ep, n + j) : 0.f);
                     }
-#pragma unroll 4
-                    for (uint32_t i = lane >> 3; i < 32; i += 4) {
-                        if (mq + i < p.M) {
-                            const int4 v = *reinterpret_cast<const int4 *>(stg + i * EPI_PITCH + (lane & 7) * 4);
-                            int acc[4] = {v.x + off[0], v.y + off[1], v.z + off[2], v.w + off[3]};
-                            finish<4>(p, C, mq + i, n, acc, cf);
+                    for (uint32_t i0 = lane >> 3; i0 < 32; i0 += 16) {
+                        int acc[4][4] = {};
+                        if (add_c) {
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                if (mq + i0 + 4 * u < p.M) {
+                                    read_c<4>(p, C, mq + i0 + 4 * u, n, acc[u]);
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint32_t i = i0 + 4 * u;
+                            if (mq + i < p.M) {
+                                const int4 v = *reinterpret_cast<const int4 *>(stg + i * EPI_PITCH + (lane & 7) * 4);
+                                acc[u][0] += v.x + off[0];
+                                acc[u][1] += v.y + off[1];
+                                acc[u][2] += v.z + off[2];
+                                acc[u][3] += v.w + off[3];
+                                finish<4>(p, C, mq + i, n, acc[u], cf);
+                            }
                         }
                     }
                 }
@@ -509,11 +588,22 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                 if (n < p.N) {
                     const int off = p.ep.offsetC ? __ldg(p.ep.offsetC + n) : 0;
                     const float cf[1] = {BATCH ? factor : (p.ep.out_kind ? column_factor(p.ep, n) : 0.f)};
-#pragma unroll 4
-                    for (uint32_t i = 0; i < 32; ++i) {
-                        if (mq + i < p.M) {
-                            int acc[1] = {stg[i * EPI_PITCH + lane] + off};
-                            finish<1>(p, C, mq + i, n, acc, cf);
+                    for (uint32_t i0 = 0; i0 < 32; i0 += 16) {
+                        int acc[16][1] = {};
+                        if (add_c) {
+#pragma unroll
+                            for (int u = 0; u < 16; ++u) {
+                                if (mq + i0 + u < p.M) {
+                                    read_c<1>(p, C, mq + i0 + u, n, acc[u]);
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) {
+                            if (mq + i0 + u < p.M) {
+                                acc[u][0] += stg[(i0 + u) * EPI_PITCH + lane] + off;
+                                finish<1>(p, C, mq + i0 + u, n, acc[u], cf);
+                            }
                         }
                     }
                 }
