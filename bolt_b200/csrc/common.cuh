@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <condition_variable>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -58,6 +59,18 @@ struct WeightTwin {
 // belongs to the device that is current when it is set, so it is remembered per device context
 enum KernelFamily { KF_GEMM = 0, KF_CONV, KF_CONV_HALF, KF_GEMV, KF_GEMV_ROW, KF_BNN, KF_GATHER, KF_MATMUL, KF_MATMUL_ROW, KF_PROBE, KF_COUNT };
 
+// A maximum that a kernel finds and the host waits for.  Device words {running maximum, finished blocks}, both zero
+// between uses (the last block rewinds them); it then stores sequence number and maximum, as one 8-byte word, into
+// mapped host memory, where the host polls: no memset, no copy, no stream synchronisation, and later work of the
+// stream need not be waited for.
+struct MaxMail {
+    unsigned *words;
+    unsigned long long *d_mail;
+    volatile unsigned long long *h_mail;
+    uint32_t seq;
+};
+constexpr int MAX_MAILS = 64;   // as many calls at a time; more wait for one
+
 struct DeviceCtx {
     int device = 0;
     bool smem_raised[KF_COUNT] = {};
@@ -70,7 +83,9 @@ struct DeviceCtx {
     unsigned *d_scratch_u = nullptr;
     std::mutex mu;       // guards the staging workspace (one staged call at a time)
     std::mutex twin_mu;  // guards twins
-    std::mutex scratch_mu;  // guards d_scratch between a reduction and its read-back
+    std::mutex mail_mu;     // guards mail_free
+    std::condition_variable mail_cv;
+    std::vector<MaxMail *> mail_free;
     std::map<const void *, WeightTwin> twins;  // host packed weight -> device copy
     // growable staging workspace for host-pointer calls
     char *ws = nullptr;
@@ -92,6 +107,49 @@ inline void count_launch(int n = 1)
 {
     g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed);
 }
+
+// One MaxMail for the duration of a call (found on a stream that is not being captured: the host has to wait).
+class MaxLease {
+public:
+    explicit MaxLease(DeviceCtx *c);
+    ~MaxLease();
+    const MaxMail &mail() const
+    {
+        return *m_;
+    }
+    // the maximum that the kernel launched on `st` with this mail reports
+    EE wait(cudaStream_t st, int *maximum);
+
+private:
+    DeviceCtx *c_;
+    MaxMail *m_;
+    bool lost_ = false;   // the kernel did not report: its words may be half counted and are not used again
+};
+bool capturing(cudaStream_t st);
+
+#ifdef __CUDACC__
+// by one thread of a block, after a block barrier behind the block's last atomicMax on words[0]
+__device__ __forceinline__ void report_maximum(const MaxMail &m, unsigned blocks)
+{
+    __threadfence();
+    if (atomicInc(m.words + 1, blocks - 1) == blocks - 1) {   // wraps to 0
+        __threadfence();
+        const unsigned mx = atomicExch(m.words, 0u);
+        *reinterpret_cast<volatile unsigned long long *>(m.d_mail) = ((unsigned long long)m.seq << 32) | mx;
+        __threadfence_system();
+    }
+}
+// |x| as a non-negative integer that orders like it: the bits of a binary32, or vpabsd of an int32 (|INT_MIN| stays
+// negative and never wins)
+__device__ __forceinline__ int magnitude(float x)
+{
+    return (int)(__float_as_uint(x) & 0x7FFFFFFFu);
+}
+__device__ __forceinline__ int magnitude(int x)
+{
+    return (int)(x < 0 ? 0u - (unsigned)x : (unsigned)x);
+}
+#endif
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize for every kernel of a family, once per device
 // (the calling thread's device must be current, which ctx() guarantees)

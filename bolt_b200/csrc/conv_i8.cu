@@ -30,6 +30,7 @@
 // (128-byte swizzle).  Warp roles, the tensor-memory double buffering and the bounded waits are those of
 // gemm_i8_tcgen05.cu.
 #include <cstring>
+#include <optional>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -103,6 +104,7 @@ struct ConvParams {
     float sI, sF, num;      // scaleO = sI * sF; factor = num / scaleO (num 1: fp32 out; output scale: fused u8)
     int relu;
     int *status;
+    MaxMail mail;           // KIND 0: where the largest |output| is reported
     // border classes: class = row_class * n_cc + col_class; class 0 has every tap inside
     uint32_t n_rc, n_cc;
     uint8_t rc_lo[MAX_AXIS_CLASSES], rc_hi[MAX_AXIS_CLASSES];   // valid kh range [lo, hi] of a row class
@@ -111,12 +113,12 @@ struct ConvParams {
 };
 
 // KIND 1: fp32 output (dequantize, + eltwise, ReLU).  KIND 0: int32 output after ReLU, the staging
-// buffer of the dynamic u8 path (convolution_direct.cpp:2689-2693).  KIND 2: u8 output with a known
+// buffer of the dynamic u8 path (convolution_direct.cpp:2689-2693), and its largest magnitude in `top`.  KIND 2: u8 output with a known
 // output scale, the arithmetic of quantizeI32ToU8 with both scales given (avx512/quantize.cpp:372-414:
 // vcvtdq2ps, vmulps, vaddps 128, vcvtps2dq, vpmovusdb) fused behind the ReLU.
 template <int KIND>
 __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t *offs, const float *colf, size_t base,
-    uint32_t width, const uint32_t *r /*16 accumulators*/)
+    uint32_t width, const uint32_t *r /*16 accumulators*/, int &top)
 {
     if (KIND == 2) {
         uint8_t *out = reinterpret_cast<uint8_t *>(p.out) + base;
@@ -196,6 +198,7 @@ __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t
                     v.z = max(v.z, 0);
                     v.w = max(v.w, 0);
                 }
+                top = max(top, max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w))));
                 *reinterpret_cast<int4 *>(out + j) = v;
             }
         }
@@ -380,6 +383,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         // After a bounded wait ran out somewhere the warp keeps walking the tiles without touching them:
         // the named barriers below have to be reached by every epilogue warp the same number of times.
         bool dead = false;
+        int top = 0;
         for (uint32_t tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
             const uint32_t acc = it & 1;
             const uint32_t acc_phase = (it >> 1) & 1;
@@ -471,7 +475,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         if (ocb < p.OC) {
                             const uint32_t width = min(16u, p.OC - ocb);
                             const size_t base = ((size_t)n * p.OC + ocb) * plane + pix * width;
-                            store_block16<KIND>(p, offs_px + col, ctl->colf + col, base, width, rr + hb * 16);
+                            store_block16<KIND>(p, offs_px + col, ctl->colf + col, base, width, rr + hb * 16, top);
                         }
                     }
                 }
@@ -522,9 +526,18 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                 release();
             }
         }
+        if (KIND == 0) {
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (lane == 0 && top > 0) {
+                atomicMax(p.mail.words, (unsigned)top);
+            }
+        }
     }
 
     __syncthreads();
+    if (KIND == 0 && threadIdx.x == 0) {
+        report_maximum(p.mail, gridDim.x);
+    }
     if (ctl->abort_flag != 0) {
         for (int i = 0; i < 64; ++i) {
             __nanosleep(2000);
@@ -774,6 +787,7 @@ struct ConvLaunch {
     float sI, sF, num;
     void *out;
     int out_kind, relu;
+    MaxMail mail;
 };
 
 // Launch with programmatic stream serialization (the kernel's set-up overlaps the tail of the previous kernel);
@@ -954,6 +968,7 @@ EE launch_conv_tcgen05(const ConvGeom &g, const ConvLaunch &a, cudaStream_t st)
     p.num = a.num;
     p.relu = a.relu;
     p.status = c->d_status;
+    p.mail = a.mail;
 
     // x as (c16, W, H, N, ICb): a box {.., TN, G} lands as [chunk][image][row][pixel][16 B]
     CUtensorMap map_x, map_w;
@@ -1134,7 +1149,7 @@ EE conv_i8_tmp_bytes(const TensorDesc *inputDesc, const TensorDesc *filterDesc, 
     return SUCCESS;
 }
 
-EE quantize_i32_u8_device(const int32_t *d_src, uint64_t n, uint8_t *d_q, F32 *scale2);
+EE quantize_i32_u8_device(const int32_t *d_src, uint64_t n, int mx, uint8_t *d_q, F32 *scale2);
 EE quantize_f32_u8_device(const float *d_src, uint64_t n, uint8_t *d_q, F32 *scale, int mode);
 
 // ext: NULL for Bolt's semantics; otherwise the extension of bolt_b200_convolution_ex
@@ -1246,6 +1261,17 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
     char *staging = d_tmp + ((g.needs_copy || g.pt || g.pb || g.pl || g.pr) ? B200_ALIGN(g.xp_bytes, 256) : 0);
     a.out = (out_u8 && !fused_u8) ? reinterpret_cast<void *>(staging) : d_out;
 
+    // the dynamic u8 output: the convolution reports the largest accumulator, then one pass converts the staging
+    const bool find_max = out_u8 && !fused_u8 && !f32_staged;
+    std::optional<MaxLease> lease;
+    if (find_max) {
+        if (capturing(st)) {
+            return UNKNOWN;   // the scale has to reach the host
+        }
+        lease.emplace(c);
+        a.mail = lease->mail();
+    }
+
     // input: in place with the padding folded into the coordinates, or through a padded copy
     EE ret = NOT_SUPPORTED;
     if (!g.needs_copy) {
@@ -1282,9 +1308,10 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
         B200_EE(quantize_f32_u8_device(reinterpret_cast<const float *>(a.out), out_elems, reinterpret_cast<uint8_t *>(d_out), &s, 0));
         sc[1] = s;
     } else if (out_u8) {
+        int mx = 0;
+        B200_EE(lease->wait(st, &mx));
         F32 scales[2] = {-1, scaleO};
-        B200_EE(quantize_i32_u8_device(reinterpret_cast<const int32_t *>(a.out), out_elems,
-            reinterpret_cast<uint8_t *>(d_out), scales));
+        B200_EE(quantize_i32_u8_device(reinterpret_cast<const int32_t *>(a.out), out_elems, mx, reinterpret_cast<uint8_t *>(d_out), scales));
         sc[1] = scales[0];
     } else {
         sc[1] = scaleO;
