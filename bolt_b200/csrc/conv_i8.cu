@@ -40,11 +40,11 @@ namespace {
 
 using namespace tc;
 
-constexpr int MAX_BLOCK_N = 256;
 constexpr int EPI_WARPS = 8;
 constexpr int EPI_THREADS = EPI_WARPS * 32;
 constexpr int NUM_THREADS = 64 + EPI_THREADS;
-constexpr int SMEM_A_STAGE = BLOCK_M * BLOCK_K;      // 8 K-chunks x 128 pixels x 16 B
+constexpr int SMEM_A_STAGE = BLOCK_M * BLOCK_K;      // of a full tile: 8 K-chunks x 128 pixels x 16 B
+constexpr int MAX_STAGES = 16;
 constexpr int MAX_CLASSES = 16;                      // border classes of a layer (3 x 3 pad 1: 9)
 constexpr int MAX_AXIS_CLASSES = 8;
 
@@ -56,17 +56,17 @@ constexpr int MAX_AXIS_CLASSES = 8;
 template <int NB>
 struct Cfg {
     static constexpr int MAX_N = NB;
-    static constexpr int STAGES = NB == 256 ? 4 : 3;
+    static constexpr int STAGES = NB == 256 ? 4 : 3;     // of full size; smaller tiles get more
     static constexpr uint32_t TMEM_COLS = 2 * NB;        // two accumulators
-    static constexpr int SMEM_B_STAGE = NB * BLOCK_K;
+    static constexpr uint32_t RING_BYTES = STAGES * (SMEM_A_STAGE + NB * BLOCK_K);
     static constexpr int CLASS_PITCH = NB + 4;           // int32 per class row; +4 staggers the banks of different classes
     static constexpr int CTAS_PER_SM = NB == 256 ? 1 : 2;
 };
 
 template <int NB>
 struct __align__(16) SmemCtl {
-    uint64_t full[Cfg<NB>::STAGES];
-    uint64_t empty[Cfg<NB>::STAGES];
+    uint64_t full[MAX_STAGES];
+    uint64_t empty[MAX_STAGES];
     uint64_t tmem_full[2];
     uint64_t tmem_empty[2];
     uint32_t tmem_base;
@@ -80,7 +80,7 @@ struct __align__(16) SmemCtl {
 template <int NB>
 constexpr size_t smem_bytes()
 {
-    return 1024 + (size_t)Cfg<NB>::STAGES * (SMEM_A_STAGE + Cfg<NB>::SMEM_B_STAGE) + sizeof(SmemCtl<NB>);
+    return 1024 + (size_t)Cfg<NB>::RING_BYTES + sizeof(SmemCtl<NB>);
 }
 
 struct ConvParams {
@@ -95,6 +95,7 @@ struct ConvParams {
     uint32_t total_chunks;  // taps * ICb
     uint32_t num_kb;        // ceil(total_chunks / 8)
     uint32_t block_n, tiles_n, tiles_m;
+    uint32_t stages, a_stage, b_stage;   // pipeline depth and bytes of a stage (multiples of 1024)
     void *out;
     const float *eltwise;
     const int32_t *offsetC; // [OC]: -128 * sum of the filter
@@ -214,8 +215,8 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *smem_a = smem;
-    uint8_t *smem_b = smem + CF::STAGES * SMEM_A_STAGE;
-    SmemCtl<NB> *ctl = reinterpret_cast<SmemCtl<NB> *>(smem + CF::STAGES * (SMEM_A_STAGE + CF::SMEM_B_STAGE));
+    uint8_t *smem_b = smem + p.stages * p.a_stage;
+    SmemCtl<NB> *ctl = reinterpret_cast<SmemCtl<NB> *>(smem + CF::RING_BYTES);
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
@@ -231,7 +232,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     if (threadIdx.x == 0) {
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_w);
-        for (int s = 0; s < CF::STAGES; ++s) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
             mbar_init(&ctl->full[s], 1);
             mbar_init(&ctl->empty[s], 1);
         }
@@ -288,7 +289,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         const uint32_t tap = q / p.ICb;
                         const uint32_t cb = q - tap * p.ICb;
                         const uint32_t kh = tap / p.FW, kw = tap - kh * p.FW;
-                        uint8_t *dst = smem_a + stage * SMEM_A_STAGE + j * chunk_stride;
+                        uint8_t *dst = smem_a + stage * p.a_stage + j * chunk_stride;
                         // taps outside the image start at negative or too large coordinates and read zeros
                         const int x = (int)(ow0 * p.sW + kw * p.dW) - p.pl;
                         const int y = (int)(oh0 * p.sH + kh * p.dH) - p.pt;
@@ -299,8 +300,8 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                             tma_load_5d(&map_x, &ctl->full[stage], dst, 0, x, y, (int)n, (int)cb);
                         }
                     }
-                    tma_load_2d(&map_w, &ctl->full[stage], smem_b + stage * CF::SMEM_B_STAGE, (int)(kb * BLOCK_K), (int)n0);
-                    if (++stage == CF::STAGES) {
+                    tma_load_2d(&map_w, &ctl->full[stage], smem_b + stage * p.b_stage, (int)(kb * BLOCK_K), (int)n0);
+                    if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
                     }
@@ -335,8 +336,8 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                     }
                     tcgen05_fence_after();
                     const uint32_t nq = min(8u, p.total_chunks - kb * 8);
-                    const uint32_t a_addr = smem_u32(smem_a + stage * SMEM_A_STAGE);
-                    const uint64_t db = make_desc_sw128(smem_u32(smem_b + stage * CF::SMEM_B_STAGE));
+                    const uint32_t a_addr = smem_u32(smem_a + stage * p.a_stage);
+                    const uint64_t db = make_desc_sw128(smem_u32(smem_b + stage * p.b_stage));
                     for (uint32_t k = 0; 2 * k < nq; ++k) {
                         // A: two 16-byte K chunks per MMA, chunk_stride apart; 8-pixel groups 128 B apart.  Rows
                         // beyond the tile's pixels read the next chunk's bytes: their accumulators are never
@@ -345,7 +346,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         umma_i8(tmem_d, da, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
                     }
                     tcgen05_commit(&ctl->empty[stage]);
-                    if (++stage == CF::STAGES) {
+                    if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
                     }
@@ -957,6 +958,15 @@ EE launch_conv_tcgen05(const ConvGeom &g, const ConvLaunch &a, cudaStream_t st)
     const bool half_cfg = force_half >= 0 ? force_half != 0 : conv_prefers_half(p.tiles_m, OC, p.num_kb, c->sm_count);
     p.block_n = half_cfg ? pick_conv_block_n(p.tiles_m, OC, 2 * c->sm_count, 128) : pick_conv_block_n(p.tiles_m, OC, c->sm_count);
     p.tiles_n = (OC + p.block_n - 1) / p.block_n;
+    // A small tile (few pixels, a narrow column block) takes as many stages as fit: with few tiles the layer is bound
+    // by the latency of its loads.  The MMA reads 128 rows of every chunk, beyond a tile's last one: bytes of the
+    // next stage or of B, whose accumulators are never stored.
+    p.a_stage = (uint32_t)B200_ALIGN(8 * B200_ALIGN(p.rows, 8) * 16, 1024);
+    p.b_stage = p.block_n * BLOCK_K;
+    p.stages = (half_cfg ? Cfg<128>::RING_BYTES : Cfg<256>::RING_BYTES) / (p.a_stage + p.b_stage);
+    if (p.stages > (uint32_t)MAX_STAGES) {
+        p.stages = MAX_STAGES;
+    }
     p.out = a.out;
     p.eltwise = a.eltwise;
     p.offsetC = a.offsetC;

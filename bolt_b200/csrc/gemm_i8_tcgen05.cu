@@ -37,7 +37,7 @@ namespace {
 using namespace tc;
 
 constexpr int MAX_BLOCK_N = 256;
-constexpr int MAX_STAGES = 8;        // the ring is as deep as shared memory allows for the tile width
+constexpr int MAX_STAGES = 24;       // the ring is as deep as shared memory allows for the tile
 #ifndef B200_EPI_WARPS_FAST
 #define B200_EPI_WARPS_FAST 16
 #endif
@@ -46,7 +46,6 @@ constexpr int EPI_WARPS_GENERAL = 8;
 constexpr uint32_t TMEM_COLS = 512;  // 2 accumulators x 256 columns
 constexpr uint32_t GROUP_M = 16;     // row blocks per raster group
 
-constexpr int SMEM_A_STAGE = BLOCK_M * BLOCK_K;        // 16 KiB
 constexpr int CONST_SLOTS = 1024;    // per-warp column constants: EPI_WARPS x (256 / column groups)
 
 struct __align__(16) SmemCtl {
@@ -71,6 +70,9 @@ constexpr size_t SMEM_RING_BYTES = (SMEM_BYTES - 1024 - sizeof(SmemCtl) - SMEM_S
 struct Params {
     uint32_t M, N, K;
     uint32_t block_n;       // multiple of 32, <= 256
+    // Rows of an A box.  128, except with fewer rows in all: then only those are loaded (in eights).  The MMA still reads
+    // 128 rows; the others are whatever lies behind in the ring, and so are their accumulators, which are never stored.
+    uint32_t a_rows;
     uint32_t stages;        // pipeline depth, <= MAX_STAGES
     uint32_t tiles_m, tiles_n, num_kb;
     void *C;
@@ -420,7 +422,8 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const uint32_t worker = PAIR ? (blockIdx.x >> 1) : blockIdx.x;
     const uint32_t workers = PAIR ? (gridDim.x >> 1) : gridDim.x;
-    uint8_t *smem_b = smem + p.stages * SMEM_A_STAGE;
+    const uint32_t a_stage = p.a_rows * BLOCK_K;
+    uint8_t *smem_b = smem + p.stages * a_stage;
     uint8_t *smem_staging = smem + SMEM_RING_BYTES;  // 1024-byte aligned
     SmemCtl *ctl = reinterpret_cast<SmemCtl *>(smem + SMEM_RING_BYTES + SMEM_STAGING_BYTES);
 
@@ -488,13 +491,13 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const int m0 = (int)((PAIR ? 2 * t.mb + rank : t.mb) * BLOCK_M);
                 const uint32_t my_rows = PAIR ? (t.units * 16) : (t.units * 32);  // B rows this CTA loads
                 const int n0 = (int)(t.n0 + rank * my_rows);
-                const uint32_t tile_bytes = (PAIR ? 2u : 1u) * (BLOCK_M + my_rows) * BLOCK_K;
+                const uint32_t tile_bytes = (PAIR ? 2u : 1u) * (p.a_rows + my_rows) * BLOCK_K;
                 for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
                     if (!mbar_wait(&ctl->empty[stage], phase ^ 1)) {
                         ok = false;
                         break;
                     }
-                    uint8_t *sa = smem_a + stage * SMEM_A_STAGE;
+                    uint8_t *sa = smem_a + stage * a_stage;
                     uint8_t *sb = smem_b + stage * b_stage;
                     if (PAIR) {
                         // both CTAs' bytes are expected by, and complete on, the leader's barrier
@@ -555,7 +558,7 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         break;
                     }
                     tcgen05_fence_after();
-                    const uint64_t da = make_desc_sw128(smem_u32(smem_a + stage * SMEM_A_STAGE));
+                    const uint64_t da = make_desc_sw128(smem_u32(smem_a + stage * a_stage));
                     const uint64_t db = make_desc_sw128(smem_u32(smem_b + stage * b_stage));
 #pragma unroll
                     for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
@@ -774,8 +777,8 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         }
                     }
                 }
-            } else if (c_begin >= c_end) {
-                release(acc);  // no columns of this tile: only the hand-back
+            } else if (c_begin >= c_end || m0 + quad * 32 >= p.M) {
+                release(acc);  // no columns or no rows of this tile: only the hand-back
             } else if (KIND >= 2) {
                 // u8 output, one 32-column chunk at a time (at most two per warp; the other warps of the scheduler
                 // cover the tensor-memory read latency, and 32 live accumulators keep the warp within its register
@@ -1148,7 +1151,10 @@ EE launch_gemm_tcgen05(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, con
         p.block_n = 256;
     }
     const uint32_t b_rows = pair ? p.block_n / 2 : p.block_n;
-    p.stages = (uint32_t)(SMEM_RING_BYTES / (SMEM_A_STAGE + B200_ALIGN((size_t)b_rows * BLOCK_K, 1024)));
+    // Few rows: small A boxes, and as many K blocks in flight as fit instead -- such a product is one pass over the
+    // weight, bound by the latency of its loads.
+    p.a_rows = M >= (uint32_t)BLOCK_M ? (uint32_t)BLOCK_M : B200_ALIGN(M, 8);
+    p.stages = (uint32_t)(SMEM_RING_BYTES / (p.a_rows * BLOCK_K + B200_ALIGN((size_t)b_rows * BLOCK_K, 1024)));
     if (p.stages > (uint32_t)MAX_STAGES) {
         p.stages = MAX_STAGES;
     }
@@ -1156,7 +1162,7 @@ EE launch_gemm_tcgen05(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, con
     p.num_kb = (K + BLOCK_K - 1) / BLOCK_K;
 
     CUtensorMap map_a, map_b;
-    if (!make_map(&map_a, A, K, M, K, BLOCK_M) ||
+    if (!make_map(&map_a, A, K, M, K, p.a_rows) ||
         !make_map(&map_b, B, K, B200_ALIGN(N, 16), Kp, b_rows)) {
         return NOT_SUPPORTED;
     }
