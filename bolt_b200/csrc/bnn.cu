@@ -18,7 +18,7 @@
 // long as both operands use the same one: word j of 8 takes bits j, j+8, j+16, j+24, one shift and one mask.
 //
 // Measured, 256 -> 256 channels, 3 x 3 on 28 x 28, batch 128, whole call: 519 us with XOR + popcount (16 per clock and
-// SM: 411 us of popcounts alone), 108 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
+// SM: 411 us of popcounts alone), 96 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
 #include <cuda_fp16.h>
 
 #include <cstring>
@@ -31,7 +31,8 @@ namespace {
 
 using namespace tc;
 
-constexpr int THREADS = 256;
+constexpr int WIDEN_THREADS = 256;                // widen, and convert the results
+constexpr int THREADS = WIDEN_THREADS + 32;       // + the warp that issues the MMAs
 constexpr int MAX_BN = 128;                       // output channels of a tile
 constexpr int STAGE_A = 2 * BLOCK_M * BLOCK_K;    // two row blocks: 256 pixels
 constexpr int STAGE = STAGE_A + MAX_BN * BLOCK_K; // 48 KiB; two stages, two CTAs per SM
@@ -127,44 +128,39 @@ struct BnnParams {
 };
 
 struct BnnCtl {
-    uint64_t done[2];
+    uint64_t full[2];       // a stage is widened (one arrival per warp)
+    uint64_t done[2];       // the MMAs reading a stage have completed
+    uint64_t drained;       // the accumulators have been read (one arrival per warp)
     uint32_t tmem_base;
     __align__(16) int corr[MAX_BN];      // XNOR: kbits - 2 popcount(w) of every channel of the tile
     __half2 scale[MAX_BN / 2], bias[MAX_BN / 2];
 };
 constexpr size_t BNN_SMEM = 1024 + 2 * (size_t)STAGE + sizeof(BnnCtl);
 
-// 32 bits -> 32 bytes of 0 / 1 (or of -1 / +1), two 16-byte chunks
-template <bool SIGNS>
-__device__ __forceinline__ uint32_t widen(uint32_t w, int j)
-{
-    const uint32_t t = (w >> j) & 0x01010101u;
-    if (!SIGNS) {
-        return t;
-    }
-    const uint32_t u = t ^ 0x01010101u;
-    return (u * 255u) | t;
-}
-template <bool SIGNS>
-__device__ __forceinline__ void store_word(uint8_t *tile, uint32_t row, uint32_t word, uint32_t w, bool valid)
+// 32 bits -> 32 bytes: the bit t becomes the byte t * mul + add.  (1, 0) leaves 0 / 1; (-254, -1) gives -1 / +1: the
+// complement of 254 t, which never carries into the next byte.
+struct Widen {
+    uint32_t mul, add;
+};
+template <bool PLAIN>
+__device__ __forceinline__ void store_word(uint8_t *tile, uint32_t row, uint32_t word, uint32_t w, const Widen &m)
 {
     uint32_t v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        v[j] = widen<SIGNS>(w, j);
-        if (SIGNS && !valid) {
-            v[j] = 0;   // beyond K (the activations are zero there too, but only one side has to be)
-        }
+        const uint32_t t = (w >> j) & 0x01010101u;
+        v[j] = PLAIN ? t : t * m.mul + m.add;
     }
     uint8_t *r = tile + row * 128;
     *reinterpret_cast<uint4 *>(r + (((2 * word) ^ (row & 7)) << 4)) = make_uint4(v[0], v[1], v[2], v[3]);
     *reinterpret_cast<uint4 *>(r + (((2 * word + 1) ^ (row & 7)) << 4)) = make_uint4(v[4], v[5], v[6], v[7]);
 }
 
-// Tile = up to 256 pixels x up to 128 channels; K in blocks of 4 words = 128 bytes.  256 threads: each widens the
-// word (threadIdx & 3) of rows threadIdx / 4, + 64, + 128, + 192 of the pixels and of rows + 0, + 64 of the weights;
-// the words of K block k+1 are fetched while block k is widened, and two stages let the MMAs of block k run beside
-// the widening of block k+1.  Two CTAs share an SM, so one's epilogue runs beside the other's MMAs.
+// Tile = up to 256 pixels x up to 128 channels; K in blocks of 4 words = 128 bytes.  256 threads widen: each the word
+// (threadIdx & 3) of rows threadIdx / 4, + 64, + 128, + 192 of the pixels and of rows + 0, + 64 of the weights; the
+// words of K block k+1 are fetched while block k is widened.  A ninth warp issues the MMAs, so that the widening warps
+// wait for nobody but the stage they need.  Two stages, and two CTAs share an SM: one's epilogue runs beside the
+// other's MMAs.
 template <bool XNOR>
 __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_constant__ BnnParams p)
 {
@@ -173,8 +169,11 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
     BnnCtl *ctl = reinterpret_cast<BnnCtl *>(smem + 2 * STAGE);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        mbar_init(&ctl->done[0], 1);
-        mbar_init(&ctl->done[1], 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&ctl->full[i], WIDEN_THREADS / 32);
+            mbar_init(&ctl->done[i], 1);
+        }
+        mbar_init(&ctl->drained, WIDEN_THREADS / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -186,180 +185,217 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t tmem_base = ctl->tmem_base;
-    const uint32_t idesc = make_idesc_i8(p.block_n);
     const uint32_t num_kb = (p.kw_words + 3) / 4;
     const uint32_t tiles = p.tiles_m * p.tiles_n;
-    const uint32_t npix = p.N * p.OH * p.OW;
-    const uint32_t plane = p.Hp * p.Wp;
-    const uint32_t word = threadIdx.x & 3, row0 = threadIdx.x >> 2;
-    const uint32_t a_rows = 2 * p.row_blocks, b_rows = (p.block_n + 63) / 64;   // rows of 64 this thread serves
-    uint32_t issued = 0, staged_n0 = 0xFFFFFFFFu;
     bool dead = false;
-    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const uint32_t m0 = (tile % p.tiles_m) * p.row_blocks * BLOCK_M, n0 = (tile / p.tiles_m) * p.block_n;
-        if (n0 != staged_n0) {
-            // constants of the tile's channels (the previous tile's epilogue is over: it ended with a barrier)
-            if (threadIdx.x < p.block_n) {
-                const uint32_t o = threadIdx.x;
-                const bool in = n0 + o < p.OC;
-                reinterpret_cast<__half *>(ctl->scale)[o] = in ? p.scale[n0 + o] : __half(0.f);
-                reinterpret_cast<__half *>(ctl->bias)[o] = in ? p.bias[n0 + o] : __half(0.f);
-            }
-            staged_n0 = n0;
-        }
-        // first word of this thread's pixels (tap 0, word 0) and weights
-        uint32_t xo[4], wo[2];
+
+    if (warp == WIDEN_THREADS / 32) {
+        // ------------------------------- MMA issuer ---------------------------------------------
+        if (lane == 0) {
+            const uint32_t idesc = make_idesc_i8(p.block_n);
+            uint32_t issued = 0, it = 0;
+            for (uint32_t tile = blockIdx.x; !dead && tile < tiles; tile += gridDim.x, ++it) {
+                if (it != 0 && !mbar_wait(&ctl->drained, (it - 1) & 1)) {
+                    dead = true;
+                    break;
+                }
+                for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
+                    const uint32_t s = issued & 1;
+                    if (!mbar_wait(&ctl->full[s], (issued >> 1) & 1)) {
+                        dead = true;
+                        break;
+                    }
+                    tcgen05_fence_after();
+                    uint8_t *sa = smem + s * STAGE;
+                    const uint64_t db = make_desc_sw128(smem_u32(sa + STAGE_A));
+                    for (uint32_t r = 0; r < p.row_blocks; ++r) {
+                        const uint64_t da = make_desc_sw128(smem_u32(sa + r * BLOCK_M * BLOCK_K));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t pix = m0 + row0 + 64 * i;
-            xo[i] = 0xFFFFFFFFu;
-            if ((uint32_t)i < a_rows && pix < npix) {
-                const uint32_t ow = pix % p.OW, t = pix / p.OW, oh = t % p.OH, n = t / p.OH;
-                xo[i] = (n * p.Cw * p.Hp + oh * p.sH) * p.Wp + ow * p.sW;
+                        for (uint32_t q = 0; q < 4; ++q) {
+                            umma_i8(tmem_base + r * MAX_BN, da + 2 * q, db + 2 * q, idesc, (kb | q) != 0 ? 1u : 0u);
+                        }
+                    }
+                    tcgen05_commit(&ctl->done[s]);
+                }
             }
         }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t o = row0 + 64 * i;
-            wo[i] = ((uint32_t)i < b_rows && o < p.block_n && n0 + o < p.OC) ? (n0 + o) * p.kw_words : 0xFFFFFFFFu;
-        }
-        // this thread's word of K block kb is k = 4 kb + word = (kh, kw, cw)
-        uint32_t k = word, cw = word % p.Cw, tap = word / p.Cw, kw = tap % p.FW, kh = tap / p.FW;
-        uint32_t xa[4], wa[2];
-        int ones[2] = {0, 0};   // set bits of this thread's words of its two channels
-        bool valid = false;
-        auto fetch = [&]() {
-            valid = k < p.kw_words;
-            const uint32_t off = cw * plane + kh * p.Wp + kw;
+        __syncwarp();
+    } else {
+        // ------------------------------- widening and epilogue ------------------------------------
+        const uint32_t npix = p.N * p.OH * p.OW;
+        const uint32_t plane = p.Hp * p.Wp;
+        const uint32_t word = threadIdx.x & 3, row0 = threadIdx.x >> 2;
+        const uint32_t a_rows = 2 * p.row_blocks;   // rows of 64 this thread serves
+        uint32_t issued = 0, staged_n0 = 0xFFFFFFFFu;
+        for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const uint32_t m0 = (tile % p.tiles_m) * p.row_blocks * BLOCK_M, n0 = (tile / p.tiles_m) * p.block_n;
+            if (n0 != staged_n0) {
+                // constants of the tile's channels (the previous tile's epilogue is over: it ended with a barrier)
+                if (threadIdx.x < p.block_n) {
+                    const uint32_t o = threadIdx.x;
+                    const bool in = n0 + o < p.OC;
+                    reinterpret_cast<__half *>(ctl->scale)[o] = in ? p.scale[n0 + o] : __half(0.f);
+                    reinterpret_cast<__half *>(ctl->bias)[o] = in ? p.bias[n0 + o] : __half(0.f);
+                }
+                staged_n0 = n0;
+            }
+            // first word of this thread's pixels (tap 0, word 0) and weights; the others read word 0 and drop it
+            const uint32_t *xp[4], *wp[2];
+            uint32_t xm = 0, wm = 0;   // which of them exist
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                xa[i] = (valid && xo[i] != 0xFFFFFFFFu) ? __ldg(p.xb + xo[i] + off) : 0u;
+                const uint32_t pix = m0 + row0 + 64 * i;
+                xp[i] = p.xb;
+                if ((uint32_t)i < a_rows && pix < npix) {
+                    const uint32_t ow = pix % p.OW, t = pix / p.OW, oh = t % p.OH, n = t / p.OH;
+                    xp[i] += (n * p.Cw * p.Hp + oh * p.sH) * p.Wp + ow * p.sW;
+                    xm |= 1u << i;
+                }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                wa[i] = (valid && wo[i] != 0xFFFFFFFFu) ? __ldg(p.wb + wo[i] + k) : 0u;
-            }
-            k += 4;
-            cw += 4;
-            while (cw >= p.Cw) {
-                cw -= p.Cw;
-                if (++kw == p.FW) {
-                    kw = 0;
-                    ++kh;
+                const uint32_t o = row0 + 64 * i;
+                wp[i] = p.wb;
+                if (o < p.block_n && n0 + o < p.OC) {
+                    wp[i] += (n0 + o) * p.kw_words;
+                    wm |= 1u << i;
                 }
             }
-        };
-        fetch();
-        for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
-            const uint32_t s = issued & 1;
-            uint8_t *sa = smem + s * STAGE, *sb = sa + STAGE_A;
-            const bool ok = issued < 2 || mbar_wait(&ctl->done[s], ((issued >> 1) + 1) & 1);
-            if (ok) {
+            // this thread's word of K block kb is k = 4 kb + word = (kh, kw, cw)
+            uint32_t k = word, cw = word % p.Cw, tap = word / p.Cw, kw = tap % p.FW, kh = tap / p.FW;
+            uint32_t xa[4], wa[2];
+            int ones[2] = {0, 0};   // set bits of this thread's words of its two channels
+            Widen mw = {1u, 0u};
+            auto fetch = [&]() {
+                const bool valid = k < p.kw_words;
+                const uint32_t off = valid ? cw * plane + kh * p.Wp + kw : 0u, wk = valid ? k : 0u;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t v = __ldg(xp[i] + off);
+                    xa[i] = (valid && (xm >> i & 1u)) ? v : 0u;
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t v = __ldg(wp[i] + wk);
+                    wa[i] = (valid && (wm >> i & 1u)) ? v : 0u;
+                }
+                if (XNOR) {
+                    // beyond K the weights are zeros (so are the activations, but only one side has to be)
+                    mw.mul = valid ? (uint32_t)-254 : 0u;
+                    mw.add = valid ? 0xFFFFFFFFu : 0u;
+                }
+                k += 4;
+                cw += 4;
+                while (cw >= p.Cw) {
+                    cw -= p.Cw;
+                    if (++kw == p.FW) {
+                        kw = 0;
+                        ++kh;
+                    }
+                }
+            };
+            fetch();
+            for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
+                const uint32_t s = issued & 1;
+                uint8_t *sa = smem + s * STAGE, *sb = sa + STAGE_A;
+                if (!dead && issued >= 2 && !mbar_wait(&ctl->done[s], ((issued >> 1) + 1) & 1)) {
+                    dead = true;
+                }
+                dead = __any_sync(0xffffffffu, dead);
+                if (dead) {
+                    continue;   // keeps meeting the barriers below without touching anything
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if ((uint32_t)i < a_rows) {
-                        store_word<false>(sa, row0 + 64 * i, word, xa[i], valid);
+                        store_word<true>(sa, row0 + 64 * i, word, xa[i], mw);
                     }
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     if (row0 + 64 * i < p.block_n) {
-                        store_word<XNOR>(sb, row0 + 64 * i, word, wa[i], valid);
+                        store_word<!XNOR>(sb, row0 + 64 * i, word, wa[i], mw);
                         if (XNOR) {
                             ones[i] += __popc(wa[i]);
                         }
                     }
                 }
                 fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&ctl->full[s]);
+                }
                 fetch();
             }
-            if (__syncthreads_or(!ok)) {
-                dead = true;
-                break;
+            if (XNOR) {
+                // four neighbouring lanes hold a channel's words
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    int t = ones[i] + __shfl_xor_sync(0xffffffffu, ones[i], 1);
+                    t += __shfl_xor_sync(0xffffffffu, t, 2);
+                    if (word == 0 && row0 + 64 * i < p.block_n) {
+                        ctl->corr[row0 + 64 * i] = (int)p.kbits - 2 * t;
+                    }
+                }
             }
-            if (threadIdx.x == 0) {
+            if (!dead) {
+                const uint32_t last = issued - 1;
+                dead = !mbar_wait(&ctl->done[last & 1], (last >> 1) & 1);
+            }
+            dead = __any_sync(0xffffffffu, dead);
+            asm volatile("bar.sync 1, %0;" ::"n"(WIDEN_THREADS) : "memory");   // the constants are there
+            if (!dead) {
                 tcgen05_fence_after();
-                const uint64_t db = make_desc_sw128(smem_u32(sb));
-                for (uint32_t r = 0; r < p.row_blocks; ++r) {
-                    const uint64_t da = make_desc_sw128(smem_u32(sa + r * BLOCK_M * BLOCK_K));
+                // int16 sum -> fp16 (round to nearest even), one fused multiply-add, 8 channels = 16 bytes; a lane is a
+                // pixel, so 32 lanes write 512 contiguous bytes.  Warp = lane quadrant x (row block, or half of the channels).
+                const uint32_t quad = warp & 3, half = warp >> 2, nch = p.block_n >> 5;
+                const uint32_t r = p.row_blocks == 2 ? half : 0u;
+                const uint32_t c_begin = p.row_blocks == 2 ? 0u : (half ? (nch + 1) / 2 : 0u);
+                const uint32_t c_end = p.row_blocks == 2 ? nch : (half ? nch : (nch + 1) / 2);
+                const uint32_t pix = m0 + r * BLOCK_M + quad * 32 + lane;
+                const uint32_t n = pix / (p.OH * p.OW);
+                const size_t oplane = (size_t)p.OH * p.OW;
+                __half *dst = p.out + (size_t)n * p.OC * oplane + (size_t)(pix - n * (uint32_t)oplane) * 8;
+                for (uint32_t c = c_begin; c < c_end; ++c) {
+                    uint32_t acc[32];
+                    tmem_ld32(tmem_base + ((quad * 32u) << 16) + r * MAX_BN + c * 32, acc);
+                    tmem_ld_wait(acc);
+                    if (pix < npix) {
 #pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        umma_i8(tmem_base + r * MAX_BN, da + 2 * q, db + 2 * q, idesc, (kb | q) != 0 ? 1u : 0u);
-                    }
-                }
-                tcgen05_commit(&ctl->done[s]);
-            }
-            __syncwarp();
-        }
-        if (dead) {
-            break;
-        }
-        if (XNOR) {
-            // four neighbouring lanes hold a channel's words
+                        for (int ob = 0; ob < 32; ob += 8) {
+                            const uint32_t oc = n0 + c * 32 + ob;
+                            if (oc < p.OC) {
+                                uint32_t h[4];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                int t = ones[i] + __shfl_xor_sync(0xffffffffu, ones[i], 1);
-                t += __shfl_xor_sync(0xffffffffu, t, 2);
-                if (word == 0 && row0 + 64 * i < p.block_n) {
-                    ctl->corr[row0 + 64 * i] = (int)p.kbits - 2 * t;
-                }
-            }
-        }
-        {
-            const uint32_t last = issued - 1;
-            const bool ok = mbar_wait(&ctl->done[last & 1], (last >> 1) & 1);
-            if (__syncthreads_or(!ok)) {
-                dead = true;
-                break;
-            }
-        }
-        tcgen05_fence_after();
-        // epilogue: int16 sum -> fp16 (round to nearest even), one fused multiply-add, 8 channels = 16 bytes; a lane is
-        // a pixel, so 32 lanes write 512 contiguous bytes.  Warp = lane quadrant x (row block, or half of the channels).
-        const uint32_t quad = warp & 3, half = warp >> 2, nch = p.block_n >> 5;
-        const uint32_t r = p.row_blocks == 2 ? half : 0u;
-        const uint32_t c_begin = p.row_blocks == 2 ? 0u : (half ? (nch + 1) / 2 : 0u);
-        const uint32_t c_end = p.row_blocks == 2 ? nch : (half ? nch : (nch + 1) / 2);
-        const uint32_t pix = m0 + r * BLOCK_M + quad * 32 + lane;
-        const uint32_t n = pix / (p.OH * p.OW);
-        const size_t oplane = (size_t)p.OH * p.OW;
-        __half *dst = p.out + (size_t)n * p.OC * oplane + (size_t)(pix - n * (uint32_t)oplane) * 8;
-        for (uint32_t c = c_begin; c < c_end; ++c) {
-            uint32_t acc[32];
-            tmem_ld32(tmem_base + ((quad * 32u) << 16) + r * MAX_BN + c * 32, acc);
-            tmem_ld_wait(acc);
-            if (pix < npix) {
-#pragma unroll
-                for (int ob = 0; ob < 32; ob += 8) {
-                    const uint32_t oc = n0 + c * 32 + ob;
-                    if (oc < p.OC) {
-                        uint32_t h[4];
-#pragma unroll
-                        for (int j = 0; j < 8; j += 2) {
-                            const uint32_t o = c * 32 + ob + j;
-                            int s0 = (int)acc[ob + j], s1 = (int)acc[ob + j + 1];
-                            if (XNOR) {
-                                const int2 co = *reinterpret_cast<const int2 *>(ctl->corr + o);
-                                s0 = 2 * s0 + co.x;
-                                s1 = 2 * s1 + co.y;
+                                for (int j = 0; j < 8; j += 2) {
+                                    const uint32_t o = c * 32 + ob + j;
+                                    int s0 = (int)acc[ob + j], s1 = (int)acc[ob + j + 1];
+                                    if (XNOR) {
+                                        const int2 co = *reinterpret_cast<const int2 *>(ctl->corr + o);
+                                        s0 = 2 * s0 + co.x;
+                                        s1 = 2 * s1 + co.y;
+                                    }
+                                    // int16 -> fp16 by way of binary32, which holds every int16 exactly
+                                    const __half2 hs = __floats2half2_rn((float)(short)s0, (float)(short)s1);
+                                    const __half2 v = __hfma2(hs, ctl->scale[o >> 1], ctl->bias[o >> 1]);
+                                    h[j >> 1] = *reinterpret_cast<const uint32_t *>(&v);
+                                }
+                                *reinterpret_cast<uint4 *>(dst + (size_t)oc * oplane) = make_uint4(h[0], h[1], h[2], h[3]);
                             }
-                            // int16 -> fp16 by way of binary32, which holds every int16 exactly
-                            const __half2 hs = __floats2half2_rn((float)(short)s0, (float)(short)s1);
-                            const __half2 v = __hfma2(hs, ctl->scale[o >> 1], ctl->bias[o >> 1]);
-                            h[j >> 1] = *reinterpret_cast<const uint32_t *>(&v);
                         }
-                        *reinterpret_cast<uint4 *>(dst + (size_t)oc * oplane) = make_uint4(h[0], h[1], h[2], h[3]);
                     }
                 }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&ctl->drained);
+                }
             }
+            asm volatile("bar.sync 1, %0;" ::"n"(WIDEN_THREADS) : "memory");   // the constants have been read
         }
-        tcgen05_fence_before();
-        __syncthreads();
-        tcgen05_fence_after();
     }
-    if (dead && threadIdx.x == 0) {
+    if (dead && lane == 0) {
         atomicExch(p.status, 41);
     }
     tcgen05_fence_before();
