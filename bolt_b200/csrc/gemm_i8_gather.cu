@@ -6,12 +6,12 @@
 // 1..33-sized products of Bolt's cover test (compute/blas_enhance/tests/test_mmm.cpp:165-171).
 //
 // One tile is 128 rows x block_n columns; a CTA is 256 threads, all of which load, convert and store; one of them
-// issues the MMAs.  Two 128-byte K blocks are in flight (the loads of block k+1 run while the MMAs of block k do)
-// and three CTAs share an SM, which is what hides the load latency: nothing here is specialised by warp, because
-// these products are bound by latency and by the load / store instructions, not by the tensor pipe.
+// issues the MMAs.  Two 128-byte K blocks are in flight (block k+1 is fetched and stored while the MMAs of block k
+// run) and two or three CTAs share an SM: nothing here is specialised by warp, because these products are bound by
+// latency and by the load / store instructions, not by the tensor pipe.
 //
 // Measured, 333 x 515 x 1001 u8 x s8 -> fp32 behind its dynamic quantization, whole calls: 111 us with the 16 x 16
-// CUDA-core kernel that stood here, 50 us with this one (about 40 us of both are the quantization and the host).
+// CUDA-core kernel that stood here, 38 us with this one (about 30 us of it are the quantization and the host).
 #include <cuda.h>
 
 #include <algorithm>
@@ -30,7 +30,6 @@ constexpr int THREADS = 256;
 constexpr int MAX_BN = 128;
 constexpr int STAGE_A = BLOCK_M * BLOCK_K;     // 16 KiB
 constexpr int EPI_PITCH = 36;                  // words per staged row: 16-byte aligned, conflict-free for 8-lane phases
-constexpr int CTAS_PER_SM = 3;
 
 struct Ctl {
     uint64_t done[2];       // the MMAs reading a stage have completed
@@ -47,6 +46,15 @@ enum Layout {
     F32_ROWS_K = 2,   // the same two in binary32, quantized while they are loaded
     F32_K_ROWS = 3
 };
+// Byte operands are fetched a K block ahead into registers, which two CTAs per SM leave room for; binary32 ones are not
+__host__ __device__ constexpr bool fetched_ahead(int la, int lb)
+{
+    return la < F32_ROWS_K && lb < F32_ROWS_K;
+}
+__host__ __device__ constexpr int ctas_per_sm(int la, int lb)
+{
+    return fetched_ahead(la, lb) ? 2 : 3;
+}
 struct Operand {
     const uint8_t *p;
     uint64_t ld;       // in elements
@@ -104,20 +112,31 @@ __device__ __forceinline__ uint4 shift_words(const uint8_t *p, uint32_t n, const
 }
 
 // quantizeF32ToU8 (avx512/quantize.cpp:135-178) with the zero point taken off again, and quantizeF32ToI8 (:195-233)
+// The low byte of the result holds it.  vcvtps2dq gives 0x80000000 for NaN and from 2^31 on, which the clamp turns
+// into the lower bound; below that, clamping before rounding is the same as after it, and adding 1.5 * 2^23 rounds
+// (to nearest even) and leaves the integer in the low mantissa bits.
+template <bool ZERO_POINT>
+__device__ __forceinline__ uint32_t quantize_bits(float x, float s)
+{
+    constexpr float lo = ZERO_POINT ? 1.0f : -127.0f, hi = ZERO_POINT ? 255.0f : 127.0f;
+    float f = __fmul_rn(x, s);
+    if (ZERO_POINT) {
+        f = __fadd_rn(f, 128.0f);
+    }
+    f = f < 2147483648.0f ? f : lo;
+    return __float_as_uint(__fadd_rn(fminf(fmaxf(f, lo), hi), 12582912.0f));
+}
 template <bool ZERO_POINT>
 __device__ __forceinline__ uint32_t quantize1(float x, float s)
 {
-    if (ZERO_POINT) {
-        return (uint32_t)(min(255, max(1, cvt_rne_x86(__fadd_rn(__fmul_rn(x, s), 128.0f)))) ^ 0x80);
-    }
-    return (uint32_t)(min(127, max(-127, cvt_rne_x86(__fmul_rn(x, s)))) & 0xFF);
+    return (quantize_bits<ZERO_POINT>(x, s) ^ (ZERO_POINT ? 0x80u : 0u)) & 0xFFu;
 }
 template <bool ZERO_POINT>
 __device__ __forceinline__ uint32_t quantize4(float4 v, float s)
 {
-    const uint32_t lo = __byte_perm(quantize1<ZERO_POINT>(v.x, s), quantize1<ZERO_POINT>(v.y, s), 0x0040);
-    const uint32_t hi = __byte_perm(quantize1<ZERO_POINT>(v.z, s), quantize1<ZERO_POINT>(v.w, s), 0x0040);
-    return __byte_perm(lo, hi, 0x5410);
+    const uint32_t lo = __byte_perm(quantize_bits<ZERO_POINT>(v.x, s), quantize_bits<ZERO_POINT>(v.y, s), 0x0040);
+    const uint32_t hi = __byte_perm(quantize_bits<ZERO_POINT>(v.z, s), quantize_bits<ZERO_POINT>(v.w, s), 0x0040);
+    return __byte_perm(lo, hi, 0x5410) ^ (ZERO_POINT ? 0x80808080u : 0u);
 }
 // the first n (0..4) of four floats; with aligned vectors the extents are multiples of 4
 __device__ __forceinline__ float4 load4f(const float *p, uint32_t n, int vec)
@@ -215,85 +234,102 @@ __device__ __forceinline__ void load_tile_f32(const Operand &o, uint32_t r0, uin
 
 // K block `kb` of rows [r0, r0 + rows_tile) into the 128-byte swizzled tile at `dst`: the 16-byte chunk c of row r
 // lies at r * 128 + ((c ^ (r & 7)) << 4).  Rows and bytes that do not exist become zeros; then every byte is XORed.
-template <int LAYOUT, uint32_t XOR>
-__device__ __forceinline__ void load_tile(const Operand &o, uint32_t r0, uint32_t rows_tile, uint32_t kb, uint8_t *dst)
+// In two steps: fetch() issues all of a thread's loads, put() shifts or transposes and stores, so that the loads of
+// the next K block run beside the MMAs of this one.
+constexpr int CHUNKS = BLOCK_M * 8 / THREADS;   // ROWS_K: a thread moves four 16-byte chunks at most
+struct Fragment {
+    uint32_t w[CHUNKS][5];
+};
+template <int LAYOUT>
+__device__ __forceinline__ void fetch(const Operand &o, uint32_t r0, uint32_t rows_tile, uint32_t kb, Fragment &f)
 {
-    const uint32_t k0 = kb * BLOCK_K;
     if (LAYOUT == ROWS_K) {
-        // a thread moves 16-byte chunks, all (at most four) on their way before the first is stored; eight neighbouring
-        // lanes cover one row's 128 bytes
-        constexpr int CH = BLOCK_M * 8 / THREADS;
-        const uint32_t c = threadIdx.x & 7, row0 = threadIdx.x >> 3, k = k0 + c * 16;
+        // eight neighbouring lanes cover one row's 128 bytes
+        const uint32_t c = threadIdx.x & 7, row0 = threadIdx.x >> 3, k = kb * BLOCK_K + c * 16;
         const uint8_t *p0 = o.p + (uint64_t)(r0 + row0) * o.ld + k;
         const uint64_t step = (uint64_t)(THREADS / 8) * o.ld;
         const uint32_t bytes = k < o.k ? min(16u, o.k - k) : 0u;
-        uint32_t n[CH];
-        uint4 v[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
+        auto count = [&](int i) {
             const uint32_t row = row0 + i * (THREADS / 8);
-            n[i] = (row < rows_tile && r0 + row < o.rows) ? bytes : 0u;
-        }
+            return (row < rows_tile && r0 + row < o.rows) ? bytes : 0u;
+        };
         if (o.vec == 16) {
 #pragma unroll
-            for (int i = 0; i < CH; ++i) {
-                v[i] = n[i] ? __ldg(reinterpret_cast<const uint4 *>(p0 + i * step)) : make_uint4(0, 0, 0, 0);
+            for (int i = 0; i < CHUNKS; ++i) {
+                const uint4 v = count(i) ? __ldg(reinterpret_cast<const uint4 *>(p0 + i * step)) : make_uint4(0, 0, 0, 0);
+                f.w[i][0] = v.x;
+                f.w[i][1] = v.y;
+                f.w[i][2] = v.z;
+                f.w[i][3] = v.w;
             }
         } else if (o.vec == 8) {
 #pragma unroll
-            for (int i = 0; i < CH; ++i) {
+            for (int i = 0; i < CHUNKS; ++i) {
                 const uint2 *p = reinterpret_cast<const uint2 *>(p0 + i * step);
-                const uint2 lo = n[i] ? __ldg(p) : make_uint2(0, 0);
-                const uint2 hi = n[i] == 16 ? __ldg(p + 1) : make_uint2(0, 0);
-                v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                const uint32_t n = count(i);
+                const uint2 lo = n ? __ldg(p) : make_uint2(0, 0);
+                const uint2 hi = n == 16 ? __ldg(p + 1) : make_uint2(0, 0);
+                f.w[i][0] = lo.x;
+                f.w[i][1] = lo.y;
+                f.w[i][2] = hi.x;
+                f.w[i][3] = hi.y;
             }
         } else {
-            uint32_t w[CH][5];
 #pragma unroll
-            for (int i = 0; i < CH; ++i) {
-                load_words(p0 + i * step, n[i], w[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < CH; ++i) {
-                v[i] = shift_words(p0 + i * step, n[i], w[i]);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-            const uint32_t row = row0 + i * (THREADS / 8);
-            if (row < rows_tile) {
-                *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) =
-                    make_uint4(v[i].x ^ XOR, v[i].y ^ XOR, v[i].z ^ XOR, v[i].w ^ XOR);
+            for (int i = 0; i < CHUNKS; ++i) {
+                load_words(p0 + i * step, count(i), f.w[i]);
             }
         }
     } else {
-        // a thread takes 4 rows x 16 k (sixteen 4-byte loads, lanes along the rows) and transposes in registers
-        for (uint32_t i = threadIdx.x; i < rows_tile * 2; i += THREADS) {
-            const uint32_t quads = rows_tile >> 2;
-            const uint32_t c = i / quads, row = (i - c * quads) * 4, k = k0 + c * 16;
-            const uint32_t left = r0 + row < o.rows ? o.rows - (r0 + row) : 0u;
-            const uint8_t *p = o.p + (uint64_t)k * o.ld + r0 + row;
-            uint32_t w[16];
-            if (o.vec == 4) {   // (then the number of rows is a multiple of 4 too)
+        // 4 rows x 16 k per thread: sixteen 4-byte loads, lanes along the rows
+        const uint32_t quads = rows_tile >> 2, c = threadIdx.x / quads, row = (threadIdx.x - c * quads) * 4, k = kb * BLOCK_K + c * 16;
+        const uint32_t left = (c < 8 && r0 + row < o.rows) ? o.rows - (r0 + row) : 0u;
+        const uint8_t *p = o.p + (uint64_t)k * o.ld + r0 + row;
+        if (o.vec == 4) {   // (then the number of rows is a multiple of 4 too)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    w[j] = (k + j < o.k && left != 0) ? __ldg(reinterpret_cast<const uint32_t *>(p + (uint64_t)j * o.ld)) : 0u;
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    w[j] = 0;
-#pragma unroll
-                    for (uint32_t t = 0; t < 4; ++t) {
-                        w[j] |= (k + j < o.k && t < left) ? (uint32_t)__ldg(p + (uint64_t)j * o.ld + t) << (8 * t) : 0u;
-                    }
-                }
+            for (int j = 0; j < 16; ++j) {
+                f.w[j >> 2][j & 3] = (k + j < o.k && left != 0) ? __ldg(reinterpret_cast<const uint32_t *>(p + (uint64_t)j * o.ld)) : 0u;
             }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                uint32_t w = 0;
+#pragma unroll
+                for (uint32_t t = 0; t < 4; ++t) {
+                    w |= (k + j < o.k && t < left) ? (uint32_t)__ldg(p + (uint64_t)j * o.ld + t) << (8 * t) : 0u;
+                }
+                f.w[j >> 2][j & 3] = w;
+            }
+        }
+    }
+}
+template <int LAYOUT, uint32_t XOR>
+__device__ __forceinline__ void put(const Operand &o, uint32_t r0, uint32_t rows_tile, uint32_t kb, const Fragment &f, uint8_t *dst)
+{
+    if (LAYOUT == ROWS_K) {
+        const uint32_t c = threadIdx.x & 7, row0 = threadIdx.x >> 3, k = kb * BLOCK_K + c * 16;
+        const uint32_t bytes = k < o.k ? min(16u, o.k - k) : 0u;
+        const uint8_t *p0 = o.p + (uint64_t)(r0 + row0) * o.ld + k;
+        const uint64_t step = (uint64_t)(THREADS / 8) * o.ld;
+#pragma unroll
+        for (int i = 0; i < CHUNKS; ++i) {
+            const uint32_t row = row0 + i * (THREADS / 8);
+            if (row < rows_tile) {
+                uint4 v = make_uint4(f.w[i][0], f.w[i][1], f.w[i][2], f.w[i][3]);
+                if (o.vec < 8) {
+                    v = shift_words(p0 + i * step, r0 + row < o.rows ? bytes : 0u, f.w[i]);
+                }
+                *reinterpret_cast<uint4 *>(dst + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(v.x ^ XOR, v.y ^ XOR, v.z ^ XOR, v.w ^ XOR);
+            }
+        }
+    } else {
+        const uint32_t quads = rows_tile >> 2, c = threadIdx.x / quads, row = (threadIdx.x - c * quads) * 4;
+        if (c < 8) {
             uint32_t t[4][4];   // [row][word of 4 k]
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const uint32_t a = __byte_perm(w[4 * q], w[4 * q + 1], 0x5140), b = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x5140);
-                const uint32_t d = __byte_perm(w[4 * q], w[4 * q + 1], 0x7362), e = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x7362);
+                const uint32_t a = __byte_perm(f.w[q][0], f.w[q][1], 0x5140), b = __byte_perm(f.w[q][2], f.w[q][3], 0x5140);
+                const uint32_t d = __byte_perm(f.w[q][0], f.w[q][1], 0x7362), e = __byte_perm(f.w[q][2], f.w[q][3], 0x7362);
                 t[0][q] = __byte_perm(a, b, 0x5410);
                 t[1][q] = __byte_perm(a, b, 0x7632);
                 t[2][q] = __byte_perm(d, e, 0x5410);
@@ -420,7 +456,7 @@ __device__ __forceinline__ uint64_t batch_index(uint64_t ic, const uint32_t (&c)
 // BATCH: A arrives as (or is made) signed by taking the zero point off, so that sum (a - 128) b needs no column sums:
 // it equals sum a b - 128 sum b in 32-bit arithmetic.
 template <int LA, int LB, bool BATCH>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
+__global__ void __launch_bounds__(THREADS, ctas_per_sm(LA, LB))
 gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant__ BatchParams bp)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -479,6 +515,12 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
             ob.p = p.b.p + batch_index(batch, bp.c_dims, bp.b_dims, bp.b_direct) * bp.b_bytes;
             C = reinterpret_cast<uint8_t *>(p.C) + batch * bp.c_bytes;
         }
+        constexpr bool AHEAD = fetched_ahead(LA, LB);
+        Fragment fa, fb;
+        if (AHEAD && num_kb != 0) {
+            fetch<LA>(oa, m0, BLOCK_M, 0, fa);
+            fetch<LB>(ob, n0, p.block_n, 0, fb);
+        }
         for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
             const uint32_t s = issued & 1;
             uint8_t *sa = smem + s * stage_bytes, *sb = sa + STAGE_A;
@@ -488,12 +530,22 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                 if constexpr (LA >= F32_ROWS_K) {
                     load_tile_f32<LA, true>(oa, m0, BLOCK_M, kb, sa, scale_a);
                 } else {
-                    load_tile<LA, BATCH ? 0x80808080u : 0u>(oa, m0, BLOCK_M, kb, sa);
+                    if (!AHEAD) {
+                        fetch<LA>(oa, m0, BLOCK_M, kb, fa);
+                    }
+                    put<LA, BATCH ? 0x80808080u : 0u>(oa, m0, BLOCK_M, kb, fa, sa);
                 }
                 if constexpr (LB >= F32_ROWS_K) {
                     load_tile_f32<LB, false>(ob, n0, p.block_n, kb, sb, scale_b);
                 } else {
-                    load_tile<LB, 0u>(ob, n0, p.block_n, kb, sb);
+                    if (!AHEAD) {
+                        fetch<LB>(ob, n0, p.block_n, kb, fb);
+                    }
+                    put<LB, 0u>(ob, n0, p.block_n, kb, fb, sb);
+                }
+                if (AHEAD && kb + 1 < num_kb) {
+                    fetch<LA>(oa, m0, BLOCK_M, kb + 1, fa);
+                    fetch<LB>(ob, n0, p.block_n, kb + 1, fb);
                 }
                 fence_proxy_async_smem();
             }
@@ -861,7 +913,7 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
     p.status = c->d_status;
     const uintptr_t c_align = ep.out_kind == 2 ? 4 : 16;
     p.vec_c = (N % 4 == 0) && (reinterpret_cast<uintptr_t>(C) % c_align == 0);
-    const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n, slots = (uint64_t)c->sm_count * CTAS_PER_SM;
+    const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n, slots = (uint64_t)c->sm_count * ctas_per_sm(ROWS_K, ROWS_K);
     const uint32_t grid = (uint32_t)(tiles < slots ? tiles : slots);
     if (a_transposed) {
         gemm_gather_kernel<K_ROWS, ROWS_K, false><<<grid, THREADS, SMEM_BYTES, st>>>(p, BatchParams());
@@ -934,7 +986,7 @@ Operand operand(const MatmulOperand &o, uint32_t rows, uint32_t K, bool rows_con
 
 // All products of a matmul call: at most one pass over the binary32 operands for their scales, then one kernel that
 // quantizes, multiplies and converts.  BERT-base attention of 32 x 128 tokens, scores and context (384 products of
-// 128 x 64 x 128 and of 128 x 128 x 64): 57 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
+// 128 x 64 x 128 and of 128 x 128 x 64): 53 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
 // floor is 15 us (each operand and result once); the operands are read a second time for their scales.
 EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
 {
@@ -1046,7 +1098,7 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
         p.tmem_cols = p.block_n > 64 ? 128u : p.block_n;
         cfg.dynamicSmemBytes = SMEM_BYTES;
         const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n * mb.batches;
-        const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)c->sm_count * CTAS_PER_SM);
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)c->sm_count * ctas_per_sm(la, lb));
         e = la == ROWS_K ? launch_batch_b<ROWS_K>(lb, grid, p, bp, cfg)
             : la == K_ROWS ? launch_batch_b<K_ROWS>(lb, grid, p, bp, cfg)
             : la == F32_ROWS_K ? launch_batch_b<F32_ROWS_K>(lb, grid, p, bp, cfg)
