@@ -40,9 +40,6 @@ namespace {
 
 using namespace tc;
 
-constexpr int EPI_WARPS = 8;
-constexpr int EPI_THREADS = EPI_WARPS * 32;
-constexpr int NUM_THREADS = 64 + EPI_THREADS;
 constexpr int SMEM_A_STAGE = BLOCK_M * BLOCK_K;      // of a full tile: 8 K-chunks x 128 pixels x 16 B
 constexpr int MAX_STAGES = 16;
 constexpr int MAX_CLASSES = 16;                      // border classes of a layer (3 x 3 pad 1: 9)
@@ -61,6 +58,9 @@ struct Cfg {
     static constexpr uint32_t RING_BYTES = STAGES * (SMEM_A_STAGE + NB * BLOCK_K);
     static constexpr int CLASS_PITCH = NB + 4;           // int32 per class row; +4 staggers the banks of different classes
     static constexpr int CTAS_PER_SM = NB == 256 ? 1 : 2;
+    static constexpr int EPI_WARPS = NB == 256 ? 16 : 8;  // sixteen per SM either way, four per scheduler
+    static constexpr int EPI_THREADS = EPI_WARPS * 32;
+    static constexpr int THREADS = 64 + EPI_THREADS;
 };
 
 template <int NB>
@@ -207,7 +207,7 @@ __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t
 }
 
 template <int KIND, int NB>
-__global__ void __launch_bounds__(NUM_THREADS, Cfg<NB>::CTAS_PER_SM)
+__global__ void __launch_bounds__(Cfg<NB>::THREADS, Cfg<NB>::CTAS_PER_SM)
 conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
     const __grid_constant__ ConvParams p)
 {
@@ -238,7 +238,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&ctl->tmem_full[a], 1);
-            mbar_init(&ctl->tmem_empty[a], EPI_WARPS);
+            mbar_init(&ctl->tmem_empty[a], CF::EPI_WARPS);
         }
         ctl->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -363,15 +363,16 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         }
         __syncwarp();
     } else {
-        // ------------------------------- epilogue warps 2..9 ------------------------------------
+        // ------------------------------- epilogue warps 2.. -------------------------------------
         const uint32_t quad = warp & 3;
-        const uint32_t half = (warp - 2) >> 2;
+        const uint32_t share = (warp - 2) >> 2;   // of the tile's 32-column chunks, two at most
         const uint32_t et = threadIdx.x - 64;
         const uint32_t nch = p.block_n >> 5;
         const uint32_t n_classes = p.n_rc * p.n_cc;
         const uint32_t taps = p.FH * p.FW;
-        const uint32_t c_begin = half ? ((nch + 1) >> 1) : 0u;
-        const uint32_t c_end = half ? nch : ((nch + 1) >> 1);
+        constexpr uint32_t SHARES = CF::EPI_WARPS / 4;
+        const uint32_t per = (nch + SHARES - 1) / SHARES;
+        const uint32_t c_begin = min(nch, share * per), c_end = min(nch, c_begin + per);
         uint32_t staged_n0 = 0xFFFFFFFFu;
         uint32_t it = 0;
         // this lane's pixel inside a tile (the same for every tile): image, row and column offsets
@@ -396,8 +397,8 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             if (n0 != staged_n0) {
                 // Constants of this column block (tiles run row-block fastest, so this happens tiles_n times
                 // per CTA): conversion factor and, per border class, the integer offset of every channel.
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");  // everyone is done with the old ones
-                for (uint32_t j = et; !dead && j < p.block_n; j += EPI_THREADS) {
+                asm volatile("bar.sync 1, %0;" ::"n"(CF::EPI_THREADS) : "memory");  // everyone is done with the old ones
+                for (uint32_t j = et; !dead && j < p.block_n; j += CF::EPI_THREADS) {
                     const uint32_t oc = n0 + j;
                     float factor = 0.f;
                     int boff = 0;
@@ -429,7 +430,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         ctl->offs[cls * CF::CLASS_PITCH + j] = v + boff;
                     }
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(CF::EPI_THREADS) : "memory");
                 staged_n0 = n0;
             }
             dead = __any_sync(0xffffffffu, dead);
@@ -481,47 +482,15 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                     }
                 }
             };
-            // two register buffers: the next chunk is on its way from tensor memory while this one is
-            // converted and stored; the accumulator is released as soon as its last chunk has arrived
-            if (NB != 256) {
-                // two CTAs per SM: the other CTA's warps cover the read latency, and the register budget of
-                // a half SM leaves room for one buffer only
-                uint32_t ra[32];
-                for (uint32_t c = c_begin; c < c_end; ++c) {
-                    tmem_ld32(tbase + c * 32, ra);
-                    tmem_ld_wait(ra);
-                    if (c + 1 == c_end) {
-                        release();
-                    }
-                    emit(c, ra);
-                }
-                if (c_begin >= c_end) {
-                    release();
-                }
-                continue;
-            }
-            uint32_t ra[32], rb[32];
-            if (c_begin < c_end) {
-                tmem_ld32(tbase + c_begin * 32, ra);
-            }
-            for (uint32_t c = c_begin; c < c_end; c += 2) {
+            // (the other warps of the scheduler cover the read latency)
+            uint32_t ra[32];
+            for (uint32_t c = c_begin; c < c_end; ++c) {
+                tmem_ld32(tbase + c * 32, ra);
                 tmem_ld_wait(ra);
-                const bool has1 = c + 1 < c_end;
-                if (has1) {
-                    tmem_ld32(tbase + (c + 1) * 32, rb);
-                } else {
+                if (c + 1 == c_end) {
                     release();
                 }
                 emit(c, ra);
-                if (has1) {
-                    tmem_ld_wait(rb);
-                    if (c + 2 < c_end) {
-                        tmem_ld32(tbase + (c + 2) * 32, ra);
-                    } else {
-                        release();
-                    }
-                    emit(c + 1, rb);
-                }
             }
             if (c_begin >= c_end) {
                 release();
@@ -805,7 +774,7 @@ cudaError_t launch_conv_kernel(uint32_t grid, cudaStream_t st, const CUtensorMap
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NUM_THREADS);
+    cfg.blockDim = dim3(Cfg<NB>::THREADS);
     cfg.dynamicSmemBytes = smem_bytes<NB>();
     cfg.stream = st;
     cudaLaunchAttribute at[1];
