@@ -117,6 +117,20 @@ struct ConvParams {
 // buffer of the dynamic u8 path (convolution_direct.cpp:2689-2693), and its largest magnitude in `top`.  KIND 2: u8 output with a known
 // output scale, the arithmetic of quantizeI32ToU8 with both scales given (avx512/quantize.cpp:372-414:
 // vcvtdq2ps, vmulps, vaddps 128, vcvtps2dq, vpmovusdb) fused behind the ReLU.
+// (p + 128) + 1.5 * 2^23 for two products, each step rounded by itself
+__device__ __forceinline__ void round_pair(float p0, float p1, uint32_t &b0, uint32_t &b1)
+{
+    asm("{\n\t.reg .b64 v, c;\n\t"
+        "mov.b64 v, {%2, %3};\n\t"
+        "mov.b64 c, {%4, %4};\n\t"
+        "add.rn.f32x2 v, v, c;\n\t"
+        "mov.b64 c, {%5, %5};\n\t"
+        "add.rn.f32x2 v, v, c;\n\t"
+        "mov.b64 {%0, %1}, v;\n\t}"
+        : "=r"(b0), "=r"(b1)
+        : "f"(p0), "f"(p1), "f"(128.0f), "f"(12582912.0f));
+}
+
 template <int KIND>
 __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t *offs, const float *colf, size_t base,
     uint32_t width, const uint32_t *r /*16 accumulators*/, int &top)
@@ -135,12 +149,13 @@ __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t
         for (int j = 0; j < 16; j += 4) {
             const int4 o = *reinterpret_cast<const int4 *>(offs + j);
             const float4 c4 = *reinterpret_cast<const float4 *>(colf + j);
-            const float cf[4] = {c4.x, c4.y, c4.z, c4.w};
-            const int v[4] = {(int)r[j] + o.x, (int)r[j + 1] + o.y, (int)r[j + 2] + o.z, (int)r[j + 3] + o.w};
+            // max(acc + offset, floor) is one instruction, and so are two of the additions
+            round_pair(__fmul_rn(__int2float_rn(__viaddmax_s32((int)r[j], o.x, floor_v)), c4.x),
+                __fmul_rn(__int2float_rn(__viaddmax_s32((int)r[j + 1], o.y, floor_v)), c4.y), bits[j], bits[j + 1]);
+            round_pair(__fmul_rn(__int2float_rn(__viaddmax_s32((int)r[j + 2], o.z, floor_v)), c4.z),
+                __fmul_rn(__int2float_rn(__viaddmax_s32((int)r[j + 3], o.w, floor_v)), c4.w), bits[j + 2], bits[j + 3]);
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                const float f = __fadd_rn(__fmul_rn(__int2float_rn(max(v[t], floor_v)), cf[t]), 128.0f);
-                bits[j + t] = __float_as_uint(__fadd_rn(f, 12582912.0f));
                 seen |= bits[j + t] ^ 0x4B400000u;
             }
             w[j >> 2] = __byte_perm(__byte_perm(bits[j], bits[j + 1], 0x0040), __byte_perm(bits[j + 2], bits[j + 3], 0x0040), 0x5410);
@@ -411,23 +426,54 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         }
                     }
                     ctl->colf[j] = factor;
-                    for (uint32_t cls = 0; cls < n_classes; ++cls) {
-                        int v = 0;
-                        if (oc < p.OC) {
-                            if (cls == 0) {
-                                v = p.offsetC[oc];
-                            } else {
-                                const uint32_t rc = cls / p.n_cc, cc = cls - rc * p.n_cc;
-                                int sum = 0;
-                                for (uint32_t kh = p.rc_lo[rc]; kh <= p.rc_hi[rc] && kh < p.FH; ++kh) {
-                                    for (uint32_t kw = p.cc_lo[cc]; kw <= p.cc_hi[cc] && kw < p.FW; ++kw) {
-                                        sum += p.tapsum[(size_t)oc * taps + kh * p.FW + kw];
-                                    }
+                    const bool in = oc < p.OC;
+                    ctl->offs[j] = (in ? p.offsetC[oc] : 0) + boff;
+                    if (n_classes == 1) {
+                        continue;
+                    }
+                    // border classes: -128 times the weights of the taps inside.  A 3 x 3 filter's nine sums are loaded
+                    // at once; loading them class by class (up to 60 loads, one latency after the other) took longer
+                    // than the products of most layers.
+                    const int32_t *ts = p.tapsum + (size_t)oc * taps;
+                    if (p.FH == 3 && p.FW == 3) {
+                        int t[9];
+#pragma unroll
+                        for (int k = 0; k < 9; ++k) {
+                            t[k] = in ? __ldg(ts + k) : 0;
+                        }
+                        for (uint32_t rc = 0; rc < p.n_rc; ++rc) {
+                            int row[3] = {0, 0, 0};   // of the filter rows inside, summed by column
+#pragma unroll
+                            for (int kh = 0; kh < 3; ++kh) {
+                                const bool inside = kh >= p.rc_lo[rc] && kh <= p.rc_hi[rc];
+#pragma unroll
+                                for (int kw = 0; kw < 3; ++kw) {
+                                    row[kw] += inside ? t[kh * 3 + kw] : 0;
                                 }
-                                v = -128 * sum;
+                            }
+                            for (uint32_t cc = 0; cc < p.n_cc; ++cc) {
+                                if ((rc | cc) != 0) {
+                                    int sum = 0;
+#pragma unroll
+                                    for (int kw = 0; kw < 3; ++kw) {
+                                        sum += (kw >= p.cc_lo[cc] && kw <= p.cc_hi[cc]) ? row[kw] : 0;
+                                    }
+                                    ctl->offs[(rc * p.n_cc + cc) * CF::CLASS_PITCH + j] = -128 * sum + boff;
+                                }
                             }
                         }
-                        ctl->offs[cls * CF::CLASS_PITCH + j] = v + boff;
+                    } else {
+                        for (uint32_t cls = 1; cls < n_classes; ++cls) {
+                            const uint32_t rc = cls / p.n_cc, cc = cls - rc * p.n_cc;
+                            int sum = 0;
+                            for (uint32_t kh = p.rc_lo[rc]; in && kh <= p.rc_hi[rc] && kh < p.FH; ++kh) {
+#pragma unroll 8
+                                for (uint32_t kw = p.cc_lo[cc]; kw <= min((uint32_t)p.cc_hi[cc], p.FW - 1); ++kw) {
+                                    sum += __ldg(ts + kh * p.FW + kw);
+                                }
+                            }
+                            ctl->offs[cls * CF::CLASS_PITCH + j] = -128 * sum + boff;
+                        }
                     }
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(CF::EPI_THREADS) : "memory");
@@ -468,6 +514,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                     mbar_arrive(&ctl->tmem_empty[acc]);
                 }
             };
+            const size_t image = (size_t)n * p.OC * plane, pix16 = pix * 16;
             auto emit = [&](uint32_t c, const uint32_t *rr) {
                 if (row_ok) {
 #pragma unroll
@@ -476,7 +523,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         const uint32_t ocb = n0 + col;
                         if (ocb < p.OC) {
                             const uint32_t width = min(16u, p.OC - ocb);
-                            const size_t base = ((size_t)n * p.OC + ocb) * plane + pix * width;
+                            const size_t base = image + (size_t)ocb * plane + (width == 16 ? pix16 : pix * width);
                             store_block16<KIND>(p, offs_px + col, ctl->colf + col, base, width, rr + hb * 16, top);
                         }
                     }
