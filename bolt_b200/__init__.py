@@ -119,6 +119,12 @@ class GemmEpilogue(C.Structure):
                 ("prefetch", C.c_void_p), ("prefetch_bytes", C.c_size_t)]
 
 
+class GemmCall(C.Structure):
+    """bolt_b200_gemm_call"""
+    _fields_ = [("N", C.c_uint32), ("M", C.c_uint32), ("K", C.c_uint32), ("A", C.c_void_p), ("packedB", C.c_void_p),
+                ("offsetC", C.c_void_p), ("C", C.c_void_p), ("epilogue", GemmEpilogue)]
+
+
 _vp, _u32, _u32p, _f32p = C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32), C.POINTER(C.c_float)
 _TDp = C.POINTER(TensorDesc)
 
@@ -152,6 +158,7 @@ SIGNATURES = {
     "matrix_matrix_multiply_transform_rhs_cuda_b200": (C.c_int, [_TDp, _vp, _TDp, _vp]),
     "matrix_matrix_multiply_tmp_bytes_cuda_b200": (C.c_int, [_u32] * 3 + [_u32] * 4 + [_u32p]),
     "mmm_cuda_b200": (C.c_int, [_u32, _u32, _u32, _u32, _u32, _vp, _vp, _vp, _vp, _f32p]),
+    "bolt_b200_gemm_u8s8_chain": (C.c_int, [C.POINTER(GemmCall), _u32]),
     "bolt_b200_gemm_u8s8_ex": (C.c_int, [_u32, _u32, _u32, _vp, _vp, _vp, _vp, C.POINTER(GemmEpilogue)]),
     "bolt_b200_quantize_f32_u8_dev": (C.c_int, [_vp, C.c_uint64, _vp, _vp]),
     "bolt_b200_col_factor": (C.c_int, [C.c_float, C.c_float, _vp, C.c_float, _vp, _u32, _vp]),

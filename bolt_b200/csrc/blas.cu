@@ -128,8 +128,9 @@ EE pack_weight(const void *src, bool src_is_nk, U32 N, U32 K, void *dst, size_t 
     return ret;
 }
 
+// after_skinny: in a chain of products, whether the previous one ran on the few-rows kernel; set for the next
 EE run_gemm(U32 N, U32 M, U32 K, bool a_t, const void *A, const void *B, const void *offsetC, void *C,
-    GemmEpilogue ep)
+    GemmEpilogue ep, bool *after_skinny = nullptr)
 {
     DeviceCtx *c = ctx();
     if (c == nullptr) {
@@ -157,7 +158,17 @@ EE run_gemm(U32 N, U32 M, U32 K, bool a_t, const void *A, const void *B, const v
     ep.offsetC = dOff;
     cudaStream_t st = tls().stream;
     EE ret;
-    if (gemm_tcgen05_eligible(M, N, K, dA, dB, Kp, a_t)) {
+    const bool preload = after_skinny != nullptr && *after_skinny;
+    if (after_skinny != nullptr) {
+        *after_skinny = false;
+    }
+    if (ep.scatter_n == 0 && gemm_skinny_preferred(M, N, K, c->sm_count) && gemm_tcgen05_eligible(M, N, K, dA, dB, Kp, a_t)) {
+        ret = launch_gemm_skinny(M, N, K, dA, dB, Kp, dC, ep, preload, st);
+        tls().last_gemm_tc = 1;
+        if (after_skinny != nullptr) {
+            *after_skinny = !sg.any_host();
+        }
+    } else if (gemm_tcgen05_eligible(M, N, K, dA, dB, Kp, a_t)) {
         ret = launch_gemm_tcgen05(M, N, K, dA, dB, Kp, dC, ep, st);
         tls().last_gemm_tc = 1;
     } else if (ep.scatter_n > 0) {
@@ -280,12 +291,9 @@ EE mmm_cuda_b200(U32 N, U32 M, U32 K, DataType dt, DataFormat adf, const void *A
     return run_gemm(N, M, K, adf == DF_TRANSPOSE, A, B, tmp, C, ep);
 }
 
-EE bolt_b200_gemm_u8s8_ex(U32 N, U32 M, U32 K, const void *A, const void *packedB, const I32 *offsetC,
-    void *C, const bolt_b200_gemm_epilogue *e)
+static EE gemm_ex(const bolt_b200_gemm_call &g, bool *after_skinny)
 {
-    if (e == nullptr) {
-        return NULL_POINTER;
-    }
+    const bolt_b200_gemm_epilogue *e = &g.epilogue;
     GemmEpilogue ep;
     std::memset(&ep, 0, sizeof(ep));
     if (e->out_dt == DT_I32) {
@@ -312,7 +320,28 @@ EE bolt_b200_gemm_u8s8_ex(U32 N, U32 M, U32 K, const void *A, const void *packed
     if (e->col_factor != nullptr && e->row_scale != nullptr) {
         return NOT_SUPPORTED;
     }
-    return run_gemm(N, M, K, false, A, packedB, offsetC, C, ep);
+    return run_gemm(g.N, g.M, g.K, false, g.A, g.packedB, g.offsetC, g.C, ep, after_skinny);
+}
+
+EE bolt_b200_gemm_u8s8_ex(U32 N, U32 M, U32 K, const void *A, const void *packedB, const I32 *offsetC,
+    void *C, const bolt_b200_gemm_epilogue *e)
+{
+    if (e == nullptr) {
+        return NULL_POINTER;
+    }
+    return gemm_ex(bolt_b200_gemm_call{N, M, K, A, packedB, offsetC, C, *e}, nullptr);
+}
+
+EE bolt_b200_gemm_u8s8_chain(const bolt_b200_gemm_call *calls, U32 n)
+{
+    if (calls == nullptr && n != 0) {
+        return NULL_POINTER;
+    }
+    bool after_skinny = false;
+    for (U32 i = 0; i < n; ++i) {
+        B200_EE(gemm_ex(calls[i], &after_skinny));
+    }
+    return SUCCESS;
 }
 
 EE bolt_b200_gemm_u8s8_scatter(U32 N, U32 M, U32 K, const void *A, const void *packedB, const I32 *offsetC,

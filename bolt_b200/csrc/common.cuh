@@ -238,6 +238,9 @@ EE launch_gemm_tcgen05(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, con
     uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st);
 bool gemm_tcgen05_eligible(uint32_t M, uint32_t N, uint32_t K, const void *A, const void *B,
     uint32_t Kp, bool a_transposed);
+bool gemm_skinny_preferred(uint32_t M, uint32_t N, uint32_t K, int sms);
+EE launch_gemm_skinny(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, const int8_t *B, uint32_t Kp, void *C,
+    const GemmEpilogue &ep, bool preload, cudaStream_t st);
 EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed,
     const int8_t *B, uint32_t Kp, void *C, const GemmEpilogue &ep, cudaStream_t st);
 

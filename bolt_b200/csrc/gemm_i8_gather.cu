@@ -19,6 +19,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "epilogue.cuh"
 #include "tcgen05.cuh"
 
 namespace b200 {
@@ -344,79 +345,6 @@ __device__ __forceinline__ void put(const Operand &o, uint32_t r0, uint32_t rows
     }
 }
 
-// conversion factor of column n (without per-row scales), in the order of the other kernels
-__device__ __forceinline__ float column_factor(const GemmEpilogue &ep, uint32_t n)
-{
-    if (ep.col_factor != nullptr) {
-        return ep.col_factor[n];
-    }
-    if (!ep.per_channel) {
-        return ep.factor;
-    }
-    const float sb = ep.col_scale ? ep.col_scale[n] : ep.sB;
-    if (ep.row_scale != nullptr) {
-        return sb;   // divided per element
-    }
-    return __fdiv_rn(ep.num, __fmul_rn(ep.sA_dev ? *ep.sA_dev : ep.sA, sb));
-}
-
-// what C holds in V consecutive columns of row m
-template <int V>
-__device__ __forceinline__ void read_c(const GatherParams &p, const void *C, uint32_t m, uint32_t n, int (&acc)[V])
-{
-    const int32_t *cin = reinterpret_cast<const int32_t *>(C) + (size_t)m * p.N + n;
-    if (V == 4) {
-        const int4 v = *reinterpret_cast<const int4 *>(cin);
-        acc[0] = v.x;
-        acc[1 % V] = v.y;
-        acc[2 % V] = v.z;
-        acc[3 % V] = v.w;
-    } else {
-        acc[0] = cin[0];
-    }
-}
-// V consecutive results of row m, columns n .. n+V-1
-template <int V>
-__device__ __forceinline__ void finish(const GatherParams &p, void *C, uint32_t m, uint32_t n, const int (&acc)[V], const float (&cf)[V])
-{
-    const GemmEpilogue &ep = p.ep;
-    const size_t o = (size_t)m * p.N + n;
-    if (ep.out_kind == 0) {
-        int32_t *out = reinterpret_cast<int32_t *>(C) + o;
-        if (V == 4) {
-            *reinterpret_cast<int4 *>(out) = make_int4(acc[0], acc[1 % V], acc[2 % V], acc[3 % V]);
-        } else {
-            out[0] = acc[0];
-        }
-        return;
-    }
-    float f[V];
-#pragma unroll
-    for (int j = 0; j < V; ++j) {
-        f[j] = cf[j];
-        if (ep.per_channel && ep.row_scale != nullptr) {
-            f[j] = __fdiv_rn(ep.num, __fmul_rn(ep.row_scale[m], cf[j]));
-        }
-    }
-    if (ep.out_kind == 1) {
-        float *out = reinterpret_cast<float *>(C) + o;
-        if (V == 4) {
-            *reinterpret_cast<float4 *>(out) = make_float4(acc_to_f32(acc[0], f[0]), acc_to_f32(acc[1 % V], f[1 % V]),
-                acc_to_f32(acc[2 % V], f[2 % V]), acc_to_f32(acc[3 % V], f[3 % V]));
-        } else {
-            out[0] = acc_to_f32(acc[0], f[0]);
-        }
-    } else {
-        uint8_t *out = reinterpret_cast<uint8_t *>(C) + o;
-        if (V == 4) {
-            *reinterpret_cast<uint32_t *>(out) = acc_to_u8(acc[0], f[0]) | (acc_to_u8(acc[1 % V], f[1 % V]) << 8) |
-                (acc_to_u8(acc[2 % V], f[2 % V]) << 16) | (acc_to_u8(acc[3 % V], f[3 % V]) << 24);
-        } else {
-            out[0] = (uint8_t)acc_to_u8(acc[0], f[0]);
-        }
-    }
-}
-
 // scale = max(given, 127 / max|x|), the dynamic scale of quantize (avx512/quantize.cpp:129-133), from the partial
 // maxima that absmax_pair_kernel left; called by a whole warp
 __device__ __forceinline__ float dynamic_scale(const unsigned *slots, uint32_t n, float given, uint32_t lane)
@@ -617,7 +545,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
 #pragma unroll
                             for (int u = 0; u < 4; ++u) {
                                 if (mq + i0 + 4 * u < p.M) {
-                                    read_c<4>(p, C, mq + i0 + 4 * u, n, acc[u]);
+                                    read_c<4>(p.N, C, mq + i0 + 4 * u, n, acc[u]);
                                 }
                             }
                         }
@@ -630,7 +558,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                                 acc[u][1] += v.y + off[1];
                                 acc[u][2] += v.z + off[2];
                                 acc[u][3] += v.w + off[3];
-                                finish<4>(p, C, mq + i, n, acc[u], cf);
+                                finish<4>(p.ep, p.N, C, mq + i, n, acc[u], cf);
                             }
                         }
                     }
@@ -646,7 +574,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
 #pragma unroll
                             for (int u = 0; u < 16; ++u) {
                                 if (mq + i0 + u < p.M) {
-                                    read_c<1>(p, C, mq + i0 + u, n, acc[u]);
+                                    read_c<1>(p.N, C, mq + i0 + u, n, acc[u]);
                                 }
                             }
                         }
@@ -654,7 +582,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                         for (int u = 0; u < 16; ++u) {
                             if (mq + i0 + u < p.M) {
                                 acc[u][0] += stg[(i0 + u) * EPI_PITCH + lane] + off;
-                                finish<1>(p, C, mq + i0 + u, n, acc[u], cf);
+                                finish<1>(p.ep, p.N, C, mq + i0 + u, n, acc[u], cf);
                             }
                         }
                     }
@@ -680,6 +608,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
 // Partial maxima of |a| and |b| (float bits): the first ga blocks take a, the others b; block i of an operand writes
 // slot i.  No initial value and no atomic: whoever needs the scale reduces the few hundred slots itself.
 constexpr int MAX_THREADS = 512;
+constexpr uint32_t MAX_BLOCK = MAX_THREADS * 32;   // elements a block takes at a time: 64 KiB
 __device__ __forceinline__ unsigned abs4(float4 v)
 {
     return max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
@@ -693,21 +622,29 @@ absmax_pair_kernel(const float *a, uint64_t na, unsigned *a_slots, uint32_t ga, 
     const float *x = first ? a : b;
     const uint64_t n = first ? na : nb;
     const uint32_t blk = first ? blockIdx.x : blockIdx.x - ga;
-    const uint64_t stride = (uint64_t)(first ? ga : gb) * MAX_THREADS;
-    const uint64_t n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / 4 : 0;
-    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    const uint32_t blocks = first ? ga : gb;
+    const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     unsigned m = 0;
-    uint64_t i = (uint64_t)blk * MAX_THREADS + threadIdx.x;
-    const uint64_t tid = i;
-    for (; i + 3 * stride < n4; i += 4 * stride) {
-        const float4 v0 = __ldg(x4 + i), v1 = __ldg(x4 + i + stride), v2 = __ldg(x4 + i + 2 * stride), v3 = __ldg(x4 + i + 3 * stride);
-        m = max(m, max(max(abs4(v0), abs4(v1)), max(abs4(v2), abs4(v3))));
-    }
-    for (; i < n4; i += stride) {
-        m = max(m, abs4(__ldg(x4 + i)));
-    }
-    for (uint64_t j = n4 * 4 + tid; j < n; j += stride) {
-        m = max(m, __float_as_uint(__ldg(x + j)) & 0x7FFFFFFFu);
+    // eight 16-byte loads per thread in flight
+    for (uint64_t i0 = (uint64_t)blk * MAX_BLOCK; i0 < n; i0 += (uint64_t)blocks * MAX_BLOCK) {
+        const uint64_t i1 = min(n, i0 + MAX_BLOCK);
+        if (aligned && i1 - i0 == MAX_BLOCK) {
+            const float4 *x4 = reinterpret_cast<const float4 *>(x + i0) + threadIdx.x;
+            float4 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                v[j] = __ldg(x4 + j * MAX_THREADS);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                m = max(m, abs4(v[j]));
+            }
+        } else {
+#pragma unroll 8
+            for (uint64_t i = i0 + threadIdx.x; i < i1; i += MAX_THREADS) {
+                m = max(m, __float_as_uint(__ldg(x + i)) & 0x7FFFFFFFu);
+            }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1051,13 +988,13 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
     all_batches(p.b, mb.b, bp.b_bytes);
     p.vec_c = (mb.N % 4 == 0) && ((reinterpret_cast<uintptr_t>(mb.C) | (mb.batches == 1 ? 0 : bp.c_bytes)) % (4 * esz) == 0);
 
-    // partial maxima: 64 KiB of operand per block at least, two blocks per SM at most, and no more slots than given
+    // partial maxima: a block per 64 KiB of an operand, four blocks per SM at most, and no more slots than given
     auto blocks_for = [&](const MatmulOperand &o) -> uint32_t {
         if (!o.f32) {
             return 0;
         }
-        uint64_t g = (o.elems + 4 * MAX_THREADS - 1) / (4 * MAX_THREADS);
-        g = std::min<uint64_t>(g, 2 * (uint64_t)c->sm_count);
+        uint64_t g = (o.elems + MAX_BLOCK - 1) / MAX_BLOCK;
+        g = std::min<uint64_t>(g, 4 * (uint64_t)c->sm_count);
         return (uint32_t)std::min<uint64_t>(g, o.max_slots);
     };
     const uint32_t ga = blocks_for(mb.a), gb = blocks_for(mb.b);

@@ -9,7 +9,7 @@ import ctypes as C
 
 import numpy as np
 
-from . import (CHECK_STATUS, DF_NORMAL, DF_TRANSPOSE, DT_F32, DT_I8, DT_I32, DT_U8_Q, GemmEpilogue, lib,
+from . import (CHECK_STATUS, DF_NORMAL, DF_TRANSPOSE, DT_F32, DT_I8, DT_I32, DT_U8_Q, GemmCall, GemmEpilogue, lib,
                matrix_matrix_multiply_transform_rhs, matrix_matrix_multiply_transform_rhs_bytes, tensor2df)
 
 
@@ -73,7 +73,7 @@ class LinearStack:
         self.launches_per_step = 3 + len(layers)
 
     # ---- pieces -------------------------------------------------------------------------
-    def _gemm(self, l, a_ptr, c_ptr, out_dt, out_scale, sA, d_sA=None, factor=None, warm=None):
+    def _epilogue(self, l, out_dt, out_scale, sA, d_sA=None, factor=None, warm=None):
         ep = GemmEpilogue()
         # the next layer's packed weight is asked into L2 while this layer computes
         ep.prefetch, ep.prefetch_bytes = (None, 0) if warm is None else (C.c_void_p(warm.packed.data_ptr()), warm.rhs_bytes)
@@ -83,6 +83,10 @@ class LinearStack:
         ep.d_sA = d_sA
         ep.row_scale = None
         ep.col_scale = None if l.uniform else C.c_void_p(l.w_scale.data_ptr())
+        return ep
+
+    def _gemm(self, l, a_ptr, c_ptr, out_dt, out_scale, sA):
+        ep = self._epilogue(l, out_dt, out_scale, sA)
         CHECK_STATUS(lib().bolt_b200_gemm_u8s8_ex(l.N, self.M, l.K, C.c_void_p(a_ptr), C.c_void_p(l.packed.data_ptr()),
                                                   C.c_void_p(l.offsetC_ptr), C.c_void_p(c_ptr), C.byref(ep)), "gemm")
 
@@ -93,21 +97,36 @@ class LinearStack:
         CHECK_STATUS(L.bolt_b200_quantize_f32_u8_dev(C.c_void_p(self.x_dev.data_ptr()), n,
                                                      C.c_void_p(self.act[0].data_ptr()), C.c_void_p(self.d_scale.data_ptr())))
 
-    def gemms(self):
-        """All layers, activations ping-ponging between two device buffers; needs calibrate() first."""
-        cur = 0
-        sA, d_sA = 1.0, C.c_void_p(self.d_scale.data_ptr())
-        last = len(self.layers) - 1
+    def _chain(self):
+        """The layers' calls, activations ping-ponging between two device buffers.  Kept between passes, and made anew
+        when a buffer or a scale is another one."""
         fac = getattr(self, "layer_factors", None)
-        for i, l in enumerate(self.layers):
-            f = fac[i] if (fac is not None and i > 0) else None  # layer 0 divides by the dynamic input scale
-            if i == last:
-                self._gemm(l, self.act[cur].data_ptr(), self.out_dev.data_ptr(), DT_F32, 1.0, sA, d_sA, f)
-            else:
-                self._gemm(l, self.act[cur].data_ptr(), self.act[1 - cur].data_ptr(), DT_U8_Q, self.out_scales[i], sA, d_sA, f,
-                           warm=self.layers[i + 1])
-                sA, d_sA = self.out_scales[i], None
-                cur = 1 - cur
+        key = [self.M, self.d_scale.data_ptr(), self.out_dev.data_ptr(), self.act[0].data_ptr(), self.act[1].data_ptr(), *self.out_scales]
+        key += [v for l in self.layers for v in (l.K, l.N, l.packed.data_ptr(), l.offsetC_ptr, l.uniform, l.w_scale.data_ptr(), float(l.w_scale_host[0]))]
+        key += [f.data_ptr() for f in fac or ()]
+        if getattr(self, "_calls_key", None) != key:
+            last = len(self.layers) - 1
+            calls = (GemmCall * len(self.layers))()
+            cur, sA, d_sA = 0, 1.0, C.c_void_p(self.d_scale.data_ptr())
+            for i, l in enumerate(self.layers):
+                f = fac[i] if (fac is not None and i > 0) else None  # layer 0 divides by the dynamic input scale
+                c = calls[i]
+                c.N, c.M, c.K, c.A, c.packedB, c.offsetC = l.N, self.M, l.K, self.act[cur].data_ptr(), l.packed.data_ptr(), l.offsetC_ptr
+                if i == last:
+                    c.C = self.out_dev.data_ptr()
+                    c.epilogue = self._epilogue(l, DT_F32, 1.0, sA, d_sA, f)
+                else:
+                    c.C = self.act[1 - cur].data_ptr()
+                    c.epilogue = self._epilogue(l, DT_U8_Q, self.out_scales[i], sA, d_sA, f, warm=self.layers[i + 1])
+                    sA, d_sA = self.out_scales[i], None
+                    cur = 1 - cur
+            self._calls, self._calls_key = calls, key
+        return self._calls
+
+    def gemms(self):
+        """All layers; needs calibrate() first."""
+        calls = self._chain()
+        CHECK_STATUS(lib().bolt_b200_gemm_u8s8_chain(calls, len(calls)), "gemm chain")
 
     def step(self):
         """One pass, device resident: input already in x_dev, result left in out_dev."""

@@ -287,6 +287,18 @@ typedef struct {
 } bolt_b200_gemm_epilogue;
 EE bolt_b200_gemm_u8s8_ex(U32 N, U32 M, U32 K, const void *A, const void *packedB,
     const I32 *offsetC, void *C, const bolt_b200_gemm_epilogue *ep);
+/* Several of them, one after the other in one call: the layers of a network.  A may be an earlier call's C; packedB,
+ * offsetC, col_scale and col_factor have to stay as they are for the whole chain (a layer's may be read while the
+ * layer before it still runs). */
+typedef struct {
+    U32 N, M, K;
+    const void *A;
+    const void *packedB;
+    const I32 *offsetC;
+    void *C;
+    bolt_b200_gemm_epilogue epilogue;
+} bolt_b200_gemm_call;
+EE bolt_b200_gemm_u8s8_chain(const bolt_b200_gemm_call *calls, U32 n);
 /* factor[n] = num / (sA * sB[n]) in the reference's operation order (fp32 multiply, fp32 divide;
  * fully_connected.cpp:396,409): num = 1 for fp32 output, the output scale for u8 output.  d_sA (device
  * scalar) overrides sA, col_scale (device [N]) overrides sB.  factor: device [N]. */
