@@ -105,6 +105,7 @@ struct ConvParams {
     float sI, sF, num;      // scaleO = sI * sF; factor = num / scaleO (num 1: fp32 out; output scale: fused u8)
     int relu;
     int *status;
+    int vec32;              // out and eltwise are 32-byte aligned
     MaxMail mail;           // KIND 0: where the largest |output| is reported
     // border classes: class = row_class * n_cc + col_class; class 0 has every tap inside
     uint32_t n_rc, n_cc;
@@ -176,46 +177,41 @@ __device__ __forceinline__ void store_block16(const ConvParams &p, const int32_t
         } else {
             *reinterpret_cast<uint2 *>(out) = make_uint2(w[0], w[1]);
         }
-    } else if (KIND == 1) {
-        float *out = reinterpret_cast<float *>(p.out) + base;
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-            if ((uint32_t)j < width) {
-                const int4 o = *reinterpret_cast<const int4 *>(offs + j);
-                const float4 c4 = *reinterpret_cast<const float4 *>(colf + j);
-                float4 v = make_float4(acc_to_f32((int)r[j] + o.x, c4.x), acc_to_f32((int)r[j + 1] + o.y, c4.y),
-                    acc_to_f32((int)r[j + 2] + o.z, c4.z), acc_to_f32((int)r[j + 3] + o.w, c4.w));
-                if (p.eltwise != nullptr) {
-                    const float4 e = *reinterpret_cast<const float4 *>(p.eltwise + base + j);
-                    v.x = __fadd_rn(v.x, e.x);
-                    v.y = __fadd_rn(v.y, e.y);
-                    v.z = __fadd_rn(v.z, e.z);
-                    v.w = __fadd_rn(v.w, e.w);
-                }
-                if (p.relu) {
-                    v.x = v.x > 0.f ? v.x : 0.f;
-                    v.y = v.y > 0.f ? v.y : 0.f;
-                    v.z = v.z > 0.f ? v.z : 0.f;
-                    v.w = v.w > 0.f ? v.w : 0.f;
-                }
-                *reinterpret_cast<float4 *>(out + j) = v;
-            }
-        }
     } else {
-        int32_t *out = reinterpret_cast<int32_t *>(p.out) + base;
+        // eight channels at a time: 32 bytes per lane
+        uint32_t *out = reinterpret_cast<uint32_t *>(p.out) + base;
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) {
+        for (int j = 0; j < 16; j += 8) {
             if ((uint32_t)j < width) {
-                const int4 o = *reinterpret_cast<const int4 *>(offs + j);
-                int4 v = make_int4((int)r[j] + o.x, (int)r[j + 1] + o.y, (int)r[j + 2] + o.z, (int)r[j + 3] + o.w);
-                if (p.relu) {
-                    v.x = max(v.x, 0);
-                    v.y = max(v.y, 0);
-                    v.z = max(v.z, 0);
-                    v.w = max(v.w, 0);
+                uint32_t w[8], e[8];
+                if (KIND == 1 && p.eltwise != nullptr) {
+                    load_8(p.eltwise + base + j, e, p.vec32);
                 }
-                top = max(top, max(max(magnitude(v.x), magnitude(v.y)), max(magnitude(v.z), magnitude(v.w))));
-                *reinterpret_cast<int4 *>(out + j) = v;
+#pragma unroll
+                for (int h = 0; h < 8; h += 4) {
+                    const int4 o = *reinterpret_cast<const int4 *>(offs + j + h);
+                    const float4 c4 = *reinterpret_cast<const float4 *>(colf + j + h);
+                    const int v[4] = {(int)r[j + h] + o.x, (int)r[j + h + 1] + o.y, (int)r[j + h + 2] + o.z, (int)r[j + h + 3] + o.w};
+                    const float cf[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        if (KIND == 1) {
+                            float f = acc_to_f32(v[t], cf[t]);
+                            if (p.eltwise != nullptr) {
+                                f = __fadd_rn(f, __uint_as_float(e[h + t]));
+                            }
+                            if (p.relu) {
+                                f = f > 0.f ? f : 0.f;
+                            }
+                            w[h + t] = __float_as_uint(f);
+                        } else {
+                            const int a = p.relu ? max(v[t], 0) : v[t];
+                            top = max(top, magnitude(a));
+                            w[h + t] = (uint32_t)a;
+                        }
+                    }
+                }
+                store_8(out + j, w, p.vec32);
             }
         }
     }
@@ -995,6 +991,8 @@ EE launch_conv_tcgen05(const ConvGeom &g, const ConvLaunch &a, cudaStream_t st)
     p.relu = a.relu;
     p.status = c->d_status;
     p.mail = a.mail;
+    // (a pixel's 16 channels are 64 bytes; a narrower last block of 8 keeps 32-byte multiples)
+    p.vec32 = ((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.eltwise)) % 32 == 0);
 
     // x as (c16, W, H, N, ICb): a box {.., TN, G} lands as [chunk][image][row][pixel][16 B]
     CUtensorMap map_x, map_w;

@@ -79,6 +79,7 @@ struct Params {
     GemmEpilogue ep;
     int *status;
     int vec_ok;             // rows of C are 16-byte aligned -> vector stores allowed
+    int vec32;              // ... and 32-byte aligned
     uint32_t prefetch_slice;  // bytes of ep.prefetch each CTA asks for (0: none)
     // scatter (u8 output through TMA stores only): every tile is stored into n_scatter destinations -- this GPU's
     // and its peers' copies of a wider [M][ld] matrix -- at column scatter_col0 + n; the tensor maps lie in
@@ -90,24 +91,13 @@ struct Params {
     uint32_t scatter_wide;
 };
 
-// Raster: groups of GROUP_M row blocks, inside a group the row block runs fastest.
-__device__ __forceinline__ void tile_coords(const Params &p, uint32_t tile, uint32_t &mb, uint32_t &nb)
-{
-    const uint32_t per_group = GROUP_M * p.tiles_n;
-    const uint32_t g = tile / per_group;
-    const uint32_t first = g * GROUP_M;
-    const uint32_t gm = min(GROUP_M, p.tiles_m - first);
-    const uint32_t r = tile - g * per_group;
-    nb = r / gm;
-    mb = first + (r - nb * gm);
-}
-
 // One tile of work: row block, first column, width in 32-column units (at most 8).
 struct Tile {
     uint32_t mb, n0, units;
 };
 // The tiles of one worker (a CTA, or a CTA pair), in the order in which all its roles visit them: tile
-// index = worker, worker + workers, ... in the grouped raster.
+// index = worker, worker + workers, ... in a raster of groups of GROUP_M row blocks, inside which the row block runs
+// fastest.
 // (Cutting the columns into equal spans per SM instead of whole tiles -- no partly empty last wave -- was
 // measured slower on the 4096 x 3072 x 768 shape: 13.5 us against 11.7 us per launch.)
 struct TileWalk {
@@ -242,36 +232,36 @@ __device__ __forceinline__ void stage_u8(uint8_t *stg, uint32_t lane, const uint
     *reinterpret_cast<uint4 *>(row + ((1 ^ sw) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
 }
 
-// KIND 0 s32, 1 f32, 2 u8: direct 16-byte stores of one row's 32 columns
+// KIND 0 s32, 1 f32: direct stores of one row's 32 columns.  A lane has a row, so a 16-byte store touches half a sector
+// in each of 32 lines; with 32 bytes the sectors are whole and there are half as many.
 template <int KIND, bool ROWS>
 __device__ __forceinline__ void store_chunk_fast(void *C, uint32_t N, const int32_t *offs, const float *colf, float num,
-    float rs, uint32_t m, uint32_t n0, uint32_t cl, const uint32_t (&r)[32])
+    float rs, uint32_t m, uint32_t n0, uint32_t cl, const uint32_t (&r)[32], bool vec32)
 {
-    const size_t row_off = (size_t)m * N + n0;
-    if (KIND == 1) {
-        float *out = reinterpret_cast<float *>(C) + row_off;
+    uint32_t *out = reinterpret_cast<uint32_t *>(C) + (size_t)m * N + n0;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            const int4 o = *reinterpret_cast<const int4 *>(offs + cl + j);
-            float4 c4 = *reinterpret_cast<const float4 *>(colf + cl + j);
-            if (ROWS) {
-                c4.x = __fdiv_rn(num, __fmul_rn(rs, c4.x));
-                c4.y = __fdiv_rn(num, __fmul_rn(rs, c4.y));
-                c4.z = __fdiv_rn(num, __fmul_rn(rs, c4.z));
-                c4.w = __fdiv_rn(num, __fmul_rn(rs, c4.w));
+    for (int j = 0; j < 32; j += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            const int4 o = *reinterpret_cast<const int4 *>(offs + cl + j + h);
+            v[h] = r[j + h] + (uint32_t)o.x;
+            v[h + 1] = r[j + h + 1] + (uint32_t)o.y;
+            v[h + 2] = r[j + h + 2] + (uint32_t)o.z;
+            v[h + 3] = r[j + h + 3] + (uint32_t)o.w;
+            if (KIND == 1) {
+                const float4 c4 = *reinterpret_cast<const float4 *>(colf + cl + j + h);
+                float cf[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    if (ROWS) {
+                        cf[t] = __fdiv_rn(num, __fmul_rn(rs, cf[t]));
+                    }
+                    v[h + t] = __float_as_uint(acc_to_f32((int)v[h + t], cf[t]));
+                }
             }
-            *reinterpret_cast<float4 *>(out + j) = make_float4(acc_to_f32((int)r[j] + o.x, c4.x),
-                acc_to_f32((int)r[j + 1] + o.y, c4.y), acc_to_f32((int)r[j + 2] + o.z, c4.z),
-                acc_to_f32((int)r[j + 3] + o.w, c4.w));
         }
-    } else {
-        int32_t *out = reinterpret_cast<int32_t *>(C) + row_off;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            const int4 o = *reinterpret_cast<const int4 *>(offs + cl + j);
-            *reinterpret_cast<int4 *>(out + j) =
-                make_int4((int)r[j] + o.x, (int)r[j + 1] + o.y, (int)r[j + 2] + o.z, (int)r[j + 3] + o.w);
-        }
+        store_8(out + j, v, vec32);
     }
 }
 
@@ -303,12 +293,13 @@ __device__ __forceinline__ void store_chunk(const Params &p, const int32_t *offs
         const int32_t *cin = reinterpret_cast<const int32_t *>(p.C) + row_off;
         if (full_vec) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-                int4 v = *reinterpret_cast<const int4 *>(cin + j);
-                acc[j] += v.x;
-                acc[j + 1] += v.y;
-                acc[j + 2] += v.z;
-                acc[j + 3] += v.w;
+            for (int j = 0; j < 32; j += 8) {
+                uint32_t v[8];
+                load_8(cin + j, v, p.vec32);
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    acc[j + t] += (int)v[t];
+                }
             }
         } else {
 #pragma unroll
@@ -323,8 +314,10 @@ __device__ __forceinline__ void store_chunk(const Params &p, const int32_t *offs
         int32_t *out = reinterpret_cast<int32_t *>(p.C) + row_off;
         if (full_vec) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-                *reinterpret_cast<int4 *>(out + j) = make_int4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            for (int j = 0; j < 32; j += 8) {
+                const uint32_t v[8] = {(uint32_t)acc[j], (uint32_t)acc[j + 1], (uint32_t)acc[j + 2], (uint32_t)acc[j + 3],
+                    (uint32_t)acc[j + 4], (uint32_t)acc[j + 5], (uint32_t)acc[j + 6], (uint32_t)acc[j + 7]};
+                store_8(out + j, v, p.vec32);
             }
         } else {
 #pragma unroll
@@ -355,8 +348,10 @@ __device__ __forceinline__ void store_chunk(const Params &p, const int32_t *offs
         }
         if (full_vec) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-                *reinterpret_cast<float4 *>(out + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
+            for (int j = 0; j < 32; j += 8) {
+                const uint32_t v[8] = {__float_as_uint(f[j]), __float_as_uint(f[j + 1]), __float_as_uint(f[j + 2]), __float_as_uint(f[j + 3]),
+                    __float_as_uint(f[j + 4]), __float_as_uint(f[j + 5]), __float_as_uint(f[j + 6]), __float_as_uint(f[j + 7])};
+                store_8(out + j, v, p.vec32);
             }
         } else {
 #pragma unroll
@@ -837,7 +832,7 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         release(acc);  // accumulator fully read: the MMA may reuse it
                     }
                     if (row_ok) {
-                        store_chunk_fast<KIND, ROWS>(p.C, p.N, offs, colf, ep.num, rs, m, n0 + c * 32, cl, ra);
+                        store_chunk_fast<KIND, ROWS>(p.C, p.N, offs, colf, ep.num, rs, m, n0 + c * 32, cl, ra, p.vec32);
                     }
                 }
             } else {
@@ -1126,6 +1121,7 @@ EE launch_gemm_tcgen05(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, con
     p.status = c->d_status;
     const size_t esz = ep.out_kind == 2 ? 1 : 4;
     p.vec_ok = ((N * esz) % 16 == 0) && (reinterpret_cast<uintptr_t>(C) % 16 == 0);
+    p.vec32 = ((N * esz) % 32 == 0) && (reinterpret_cast<uintptr_t>(C) % 32 == 0);
     // the fast epilogue needs whole, 16-byte aligned 32-column chunks and no read of C
     const bool rows = ep.per_channel && ep.row_scale != nullptr;
     const bool fast = p.vec_ok && (N % 32 == 0) && !(ep.out_kind != 2 && ep.accumulate) && !(rows && ep.out_kind == 0);
