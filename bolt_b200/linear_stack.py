@@ -171,6 +171,7 @@ class LinearStack:
                                                     C.c_void_p(self.layer_factors[i].data_ptr())), "col_factor")
             if not last:
                 sA = self.out_scales[i]
+        self._chain()
         torch.cuda.synchronize()
 
     def run_host(self, x_host, out_host):

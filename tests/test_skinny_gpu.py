@@ -1,0 +1,83 @@
+"""GPU parity of the few-rows GEMM at the edges of its blocks (rows in sixteens, columns in eights, K in 64-byte units,
+the batches of a warp), and of a chain of layers in one call: bit for bit against the oracle."""
+import ctypes as C
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(__file__))
+import oracle as O  # noqa: E402
+import bolt_b200 as B  # noqa: E402
+from bolt_b200 import synth  # noqa: E402
+from test_gather_gpu import product  # noqa: E402
+from util import dev_zeros, dptr, to_dev, to_host  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 2, 15, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("k,n", [(16, 1), (48, 7), (64, 8), (80, 33), (768, 24), (4112, 40), (32, 1185), (272, 1192), (64, 6148)])
+@pytest.mark.parametrize("out", ["s32", "f32", "u8"])
+def test_products(m, k, n, out):
+    got, ref = product(m, k, n, 0, out)
+    assert got.tobytes() == np.ascontiguousarray(ref).tobytes()
+
+
+def chain_layers(m, dims, seed):
+    layers = []
+    for i, (k, n) in enumerate(zip(dims[:-1], dims[1:])):
+        W = synth.s8(seed + i, (k, n))
+        desc = B.tensor2df(B.DT_I8, B.DF_NORMAL, k, n)
+        nbytes, rhs = B.matrix_matrix_multiply_transform_rhs_bytes(desc)
+        packed = dev_zeros(nbytes)
+        B.matrix_matrix_multiply_transform_rhs(desc, dptr(to_dev(W)), dptr(packed))
+        col = (np.abs(synth.normal(seed + 50 + i, (n,))) + np.float32(100)).astype(np.float32)
+        layers.append((k, n, packed, rhs, to_dev(col)))
+    return layers
+
+
+@pytest.mark.parametrize("m", [1, 16, 32, 40, 100])
+def test_chain_equals_single_calls(m):
+    """more layers than fit the GPU at once, few-rows and tensor-tile layers mixed (2048 and 7168 columns)"""
+    lib = B.lib()
+    dims = [256, 2048, 256, 7168, 128, 128, 1024, 64]
+    layers = chain_layers(m, dims, 700)
+    x = to_dev(synth.u8(7, (m, dims[0])))
+    results = []
+    for chained in (False, True):
+        bufs = [dev_zeros(m * n * 4) for _, n, _, _, _ in layers]
+        calls = (B.GemmCall * len(layers))()
+        a = x
+        for c, (k, n, packed, rhs, col), out in zip(calls, layers, bufs):
+            last = out is bufs[-1]
+            c.N, c.M, c.K, c.A, c.packedB, c.offsetC, c.C = n, m, k, a.data_ptr(), packed.data_ptr(), packed.data_ptr() + rhs, out.data_ptr()
+            c.epilogue.out_dt, c.epilogue.out_scale, c.epilogue.sA, c.epilogue.sB = (B.DT_F32 if last else B.DT_U8_Q), 0.6, 1.5, 1.0
+            c.epilogue.col_scale = col.data_ptr()
+            a = out
+        for _ in range(3):      # back to back, so that a call's first layer meets the previous call's last
+            if chained:
+                B.CHECK_STATUS(lib.bolt_b200_gemm_u8s8_chain(calls, len(calls)))
+            else:
+                for c in calls:
+                    B.CHECK_STATUS(lib.bolt_b200_gemm_u8s8_ex(c.N, c.M, c.K, c.A, c.packedB, c.offsetC, c.C, C.byref(c.epilogue)))
+        B.CHECK_STATUS(lib.bolt_b200_synchronize(), "synchronize")
+        results.append([to_host(b, np.uint8, m * n).tobytes() for b, (_, n, _, _, _) in zip(bufs[:-1], layers)] + [to_host(bufs[-1], np.float32, m * dims[-1]).tobytes()])
+    assert results[0] == results[1]
+    # the first layer's single call against the oracle's accumulators
+    k, n, packed, rhs, col = layers[0]
+    acc = O.port_gemm(to_host(x, np.uint8, m * k).reshape(m, k), synth.s8(700, (k, n)), O.port_offsetc(synth.s8(700, (k, n))))
+    fac = (np.float32(0.6) / (np.float32(1.5) * to_host(col, np.float32, n))).astype(np.float32)
+    r = np.rint((acc.astype(np.float32) * fac[None, :]).astype(np.float32)).astype(np.int64) + 128
+    assert results[0][0] == np.where(r < 0, 255, np.minimum(r, 255)).astype(np.uint8).tobytes()
+
+
+def test_chain_errors():
+    lib = B.lib()
+    assert lib.bolt_b200_gemm_u8s8_chain(None, 0) == B.SUCCESS
+    assert lib.bolt_b200_gemm_u8s8_chain(None, 1) == B.NULL_POINTER
+    calls = (B.GemmCall * 1)()
+    calls[0].N, calls[0].M, calls[0].K = 8, 2, 16
+    calls[0].epilogue.out_dt = B.DT_F32
+    assert lib.bolt_b200_gemm_u8s8_chain(calls, 1) == B.NULL_POINTER
