@@ -18,7 +18,7 @@
 // long as both operands use the same one: word j of 8 takes bits j, j+8, j+16, j+24, one shift and one mask.
 //
 // Measured, 256 -> 256 channels, 3 x 3 on 28 x 28, batch 128, whole call: 519 us with XOR + popcount (16 per clock and
-// SM: 411 us of popcounts alone), 96 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
+// SM: 411 us of popcounts alone), 94 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
 #include <cuda_fp16.h>
 
 #include <cstring>
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
                 }
                 staged_n0 = n0;
             }
-            // first word of this thread's pixels (tap 0, word 0) and weights; the others read word 0 and drop it
+            // first word of this thread's pixels (tap 0, word 0) and weights.  Rows that do not exist read some other
+            // words: their accumulators are never stored.
             const uint32_t *xp[4], *wp[2];
-            uint32_t xm = 0, wm = 0;   // which of them exist
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const uint32_t pix = m0 + row0 + 64 * i;
@@ -250,41 +250,35 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
                 if ((uint32_t)i < a_rows && pix < npix) {
                     const uint32_t ow = pix % p.OW, t = pix / p.OW, oh = t % p.OH, n = t / p.OH;
                     xp[i] += (n * p.Cw * p.Hp + oh * p.sH) * p.Wp + ow * p.sW;
-                    xm |= 1u << i;
                 }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const uint32_t o = row0 + 64 * i;
-                wp[i] = p.wb;
-                if (o < p.block_n && n0 + o < p.OC) {
-                    wp[i] += (n0 + o) * p.kw_words;
-                    wm |= 1u << i;
-                }
+                wp[i] = p.wb + ((o < p.block_n && n0 + o < p.OC) ? (n0 + o) * p.kw_words : 0u);
             }
             // this thread's word of K block kb is k = 4 kb + word = (kh, kw, cw)
             uint32_t k = word, cw = word % p.Cw, tap = word / p.Cw, kw = tap % p.FW, kh = tap / p.FW;
-            uint32_t xa[4], wa[2];
             int ones[2] = {0, 0};   // set bits of this thread's words of its two channels
-            Widen mw = {1u, 0u};
-            auto fetch = [&]() {
+            // The words of a K block.  Two sets: a block's words are asked for two blocks ahead, and nothing looks at them
+            // before they are widened.
+            struct Words {
+                uint32_t x[4], w[2];
+                Widen m;          // of the weights: zeros beyond K (there the activations are any words)
+            };
+            auto fetch = [&](Words &f) {
                 const bool valid = k < p.kw_words;
                 const uint32_t off = valid ? cw * plane + kh * p.Wp + kw : 0u, wk = valid ? k : 0u;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const uint32_t v = __ldg(xp[i] + off);
-                    xa[i] = (valid && (xm >> i & 1u)) ? v : 0u;
+                    f.x[i] = __ldg(xp[i] + off);
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    const uint32_t v = __ldg(wp[i] + wk);
-                    wa[i] = (valid && (wm >> i & 1u)) ? v : 0u;
+                    f.w[i] = __ldg(wp[i] + wk);
                 }
-                if (XNOR) {
-                    // beyond K the weights are zeros (so are the activations, but only one side has to be)
-                    mw.mul = valid ? (uint32_t)-254 : 0u;
-                    mw.add = valid ? 0xFFFFFFFFu : 0u;
-                }
+                f.m.mul = valid ? (XNOR ? (uint32_t)-254 : 1u) : 0u;
+                f.m.add = valid && XNOR ? 0xFFFFFFFFu : 0u;
                 k += 4;
                 cw += 4;
                 while (cw >= p.Cw) {
@@ -295,29 +289,29 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
                     }
                 }
             };
-            fetch();
-            for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
+            auto block = [&](Words &f) {
                 const uint32_t s = issued & 1;
                 uint8_t *sa = smem + s * STAGE, *sb = sa + STAGE_A;
                 if (!dead && issued >= 2 && !mbar_wait(&ctl->done[s], ((issued >> 1) + 1) & 1)) {
                     dead = true;
                 }
                 dead = __any_sync(0xffffffffu, dead);
+                ++issued;
                 if (dead) {
-                    continue;   // keeps meeting the barriers below without touching anything
+                    return;   // keeps meeting the barriers below without touching anything
                 }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     if ((uint32_t)i < a_rows) {
-                        store_word<true>(sa, row0 + 64 * i, word, xa[i], mw);
+                        store_word<true>(sa, row0 + 64 * i, word, f.x[i], f.m);
                     }
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     if (row0 + 64 * i < p.block_n) {
-                        store_word<!XNOR>(sb, row0 + 64 * i, word, wa[i], mw);
+                        store_word<false>(sb, row0 + 64 * i, word, f.w[i], f.m);
                         if (XNOR) {
-                            ones[i] += __popc(wa[i]);
+                            ones[i] += f.m.mul != 0 ? __popc(f.w[i]) : 0;
                         }
                     }
                 }
@@ -326,7 +320,16 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
                 if (lane == 0) {
                     mbar_arrive(&ctl->full[s]);
                 }
-                fetch();
+                fetch(f);
+            };
+            Words f0, f1;
+            fetch(f0);
+            fetch(f1);
+            for (uint32_t kb = 0; kb < num_kb; kb += 2) {
+                block(f0);
+                if (kb + 1 < num_kb) {
+                    block(f1);
+                }
             }
             if (XNOR) {
                 // four neighbouring lanes hold a channel's words
@@ -578,8 +581,8 @@ EE bnn_run(const TensorDesc *inputDesc, const void *input, const TensorDesc *fil
     {
         const size_t words = g.xb_bytes / 4;
         size_t blocks = (words + 255) / 256;
-        if (blocks > (size_t)c->sm_count * 16) {
-            blocks = (size_t)c->sm_count * 16;
+        if (blocks > (size_t)c->sm_count * 64) {   // (16 made one round and a half of the 28 x 28 x 256 batch)
+            blocks = (size_t)c->sm_count * 64;
         }
         bnn_binarize_pad_kernel<<<(uint32_t)blocks, 256, 0, st>>>(d_in, g.in.n, g.in.c, g.in.h, g.in.w, g.Hp, g.Wp, g.pt,
             g.pl, g.Cw, xnor ? 0.0f : 0.5f, d_xb);
