@@ -18,7 +18,7 @@
 // long as both operands use the same one: word j of 8 takes bits j, j+8, j+16, j+24, one shift and one mask.
 //
 // Measured, 256 -> 256 channels, 3 x 3 on 28 x 28, batch 128, whole call: 519 us with XOR + popcount (16 per clock and
-// SM: 411 us of popcounts alone), 94 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
+// SM: 411 us of popcounts alone), 90 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
 #include <cuda_fp16.h>
 
 #include <cstring>
@@ -165,7 +165,7 @@ template <bool XNOR>
 __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_constant__ BnnParams p)
 {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_1024(smem_raw);
     BnnCtl *ctl = reinterpret_cast<BnnCtl *>(smem + 2 * STAGE);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {

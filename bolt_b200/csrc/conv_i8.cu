@@ -224,7 +224,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 {
     using CF = Cfg<NB>;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_1024(smem_raw);
     uint8_t *smem_a = smem;
     uint8_t *smem_b = smem + p.stages * p.a_stage;
     SmemCtl<NB> *ctl = reinterpret_cast<SmemCtl<NB> *>(smem + CF::RING_BYTES);

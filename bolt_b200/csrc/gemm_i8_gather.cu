@@ -350,8 +350,16 @@ __device__ __forceinline__ void put(const Operand &o, uint32_t r0, uint32_t rows
 __device__ __forceinline__ float dynamic_scale(const unsigned *slots, uint32_t n, float given, uint32_t lane)
 {
     unsigned m = 0;
-    for (uint32_t i = lane; i < n; i += 32) {
-        m = max(m, slots[i]);
+    for (uint32_t i = lane; i < n; i += 8 * 32) {   // (the loads of a round go out together)
+        unsigned v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = i + 32 * j < n ? slots[i + 32 * j] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            m = max(m, v[j]);
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -388,7 +396,7 @@ __global__ void __launch_bounds__(THREADS, ctas_per_sm(LA, LB))
 gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant__ BatchParams bp)
 {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_1024(smem_raw);
     const uint32_t stage_bytes = STAGE_A + p.block_n * BLOCK_K;   // both tiles stay 1024-byte aligned
     Ctl *ctl = reinterpret_cast<Ctl *>(smem + 2 * (size_t)(STAGE_A + MAX_BN * BLOCK_K));
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -923,7 +931,7 @@ Operand operand(const MatmulOperand &o, uint32_t rows, uint32_t K, bool rows_con
 
 // All products of a matmul call: at most one pass over the binary32 operands for their scales, then one kernel that
 // quantizes, multiplies and converts.  BERT-base attention of 32 x 128 tokens, scores and context (384 products of
-// 128 x 64 x 128 and of 128 x 128 x 64): 53 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
+// 128 x 64 x 128 and of 128 x 128 x 64): 49 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
 // floor is 15 us (each operand and result once); the operands are read a second time for their scales.
 EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
 {

@@ -410,7 +410,7 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     constexpr uint32_t SLOTS = CONST_SLOTS / EW;        // constants per warp: 64 (16 warps) or 128 (8 warps)
     extern __shared__ uint8_t smem_raw[];
     // 128-byte swizzled tiles need 1024-byte aligned bases
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_1024(smem_raw);
     uint8_t *smem_a = smem;
     const uint32_t b_rows = PAIR ? (p.block_n >> 1) : p.block_n;  // rows of a full B tile this CTA holds
     const uint32_t b_stage = (b_rows * BLOCK_K + 1023u) & ~1023u;  // every stage stays 1024-byte aligned

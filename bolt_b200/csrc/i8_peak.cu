@@ -20,7 +20,7 @@ constexpr uint32_t PROBE_BATCH = 32;  // MMAs per commit
 __global__ void __launch_bounds__(128, 1) i8_mma_rate_kernel(uint32_t iters, int *status)
 {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *smem = align_1024(smem_raw);
     uint8_t *smem_a = smem;                                  // 128 rows x 128 B
     uint8_t *smem_b = smem + BLOCK_M * BLOCK_K;              // 256 rows x 128 B
     __shared__ uint64_t bar[2];

@@ -24,6 +24,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
+// The first 1024-byte boundary of the block's dynamic shared memory.  An offset, not a rounded pointer value: behind a
+// cast to an integer the compiler no longer knows the address space and accesses everything through generic loads and
+// stores, with their latency and 64-bit addresses, and spills.  Whole calls: 24 GEMMs of a 4096-token stack 303.8 ->
+// 295.6 us, 1-bit convolution 93.6 -> 89.6, batched attention 51.3 -> 48.7, 22 convolutions 420 -> 416.
+__device__ __forceinline__ uint8_t *align_1024(uint8_t *smem)
+{
+    return smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);
+}
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
