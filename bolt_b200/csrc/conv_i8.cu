@@ -29,6 +29,7 @@
 // constants; one launch per call.  Weights are pre-packed [OC][K] and loaded like the GEMM's B operand
 // (128-byte swizzle).  Warp roles, the tensor-memory double buffering and the bounded waits are those of
 // gemm_i8_tcgen05.cu.
+#include <algorithm>
 #include <cstring>
 #include <optional>
 
@@ -672,33 +673,109 @@ bool get4d(const TensorDesc *d, Conv4d *o)
     return true;
 }
 
-uint32_t pick_conv_block_n(uint32_t tiles_m, uint32_t OC, int sms, uint32_t max_bn = 256)
+// ---- tile choice --------------------------------------------------------------------------------------------
+// What a K block of 128 bytes costs a CTA, in cycles: its operands come in at about 50 bytes per cycle, a TMA request (one
+// line of up to 128 bytes: a run of pixels of one image row and channel group, or a weight row; with a stride along W
+// every single pixel) takes about 1.5, and the MMAs twice the column block.  Found on the 22 ResNet-50-shaped layers.
+// The former choice, the fewest tiles whatever their shape, took 2 x 2 pixels of 32 images where 14 x 14 maps tile
+// badly (512 runs of 32 bytes per K block instead of 64 of 256) and left most SMs idle with one image: 22 layers, batch
+// 64, 416 -> 387 us; 3 x 3 on 14 x 14, 256 channels, 24.3 -> 15.1, with stride 2 28.9 -> 17.9.
+struct TileShape {
+    uint32_t tw, th, tn, block_n;
+};
+struct TileProblem {
+    uint32_t N, OH, OW, OC, sH, sW, num_kb;
+    bool merged;          // stride 1 along W: a row of a tile is one run
+    bool off_grid;        // its taps start it off the 128-byte grid
+    uint32_t max_n;       // widest column block
+    uint32_t slots;       // CTAs the device holds
+};
+uint32_t div_up(uint32_t a, uint32_t b)
 {
-    uint32_t best = 32;
-    double best_cost = 1e30;
-    for (uint32_t bn = max_bn; bn >= 32; bn -= 32) {
-        if (bn > B200_ALIGN(OC, 32) && bn != 32) {
-            continue;
+    return (a + b - 1) / b;
+}
+bool pick_tile(const TileProblem &q, TileShape *best)
+{
+    const uint32_t widest = std::min<uint32_t>(q.max_n, B200_ALIGN(q.OC, 32));
+    const double per_slot = 1.0 / q.slots;
+    const uint32_t tw_max = q.merged ? 16u : 128u;
+    uint64_t least = ~0ull;
+    auto consider = [&](uint32_t tw, uint32_t th, const uint32_t *block_n, uint32_t n_blocks) {
+        if (tw * q.sW > 256 || th * q.sH > 256 || tw * th > 128) {
+            return;   // a TMA box, the rows of an MMA
         }
-        const uint64_t tiles = (uint64_t)tiles_m * ((OC + bn - 1) / bn);
-        const uint64_t waves = (tiles + sms - 1) / sms;
-        const double cost = (double)waves * (bn + 48.0);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = bn;
+        uint32_t tn = 128 / (tw * th);
+        tn = tn < q.N ? tn : q.N;
+        const uint32_t groups = div_up(q.N, tn);
+        tn = div_up(q.N, groups);   // images spread evenly
+        const uint64_t tiles_m = (uint64_t)div_up(q.OW, tw) * div_up(q.OH, th) * groups;
+        const uint32_t runs = th * tn * 8;
+        const uint32_t requests = q.merged ? runs * ((tw * 16 + (q.off_grid ? 16 : 0) + 127) / 128) : runs * tw;
+        const uint32_t bytes = runs * tw * (q.merged ? 16 : 32);
+        // (a pixel count that is no multiple of 8 needs a box per channel group)
+        const uint32_t extra = (tw * th * tn) % 8 != 0 ? 250 : 0;
+        for (uint32_t i = 0; i < n_blocks; ++i) {
+            const uint32_t bn = block_n[i];
+            uint32_t kb = (requests + bn) * 3 / 2;
+            kb = std::max(kb, (bytes + bn * 128) / 50);
+            kb = std::max(kb, 2 * bn) + extra;
+            const uint64_t epilogue = 14 * bn + 600;   // beside the next tile's K blocks
+            const uint64_t waves = (uint64_t)((double)(tiles_m * div_up(q.OC, bn)) * per_slot + (1.0 - 1e-9));
+            const uint64_t cost = waves * std::max((uint64_t)q.num_kb * kb, epilogue) + epilogue;
+            if (cost < least) {
+                least = cost;
+                *best = TileShape{tw, th, tn, bn};
+            }
+        }
+    };
+    // Widths and heights that split the map evenly, and rows of 16 or 8 pixels that overhang it; a few column blocks
+    // first, all of them for the shape that wins.  (This runs on every call: two microseconds.)
+    uint32_t w[12], h[12], nw = 0, nh = 0;
+    auto add = [](uint32_t *list, uint32_t &n, uint32_t v) {
+        if (n < 12 && (n == 0 || list[n - 1] != v)) {
+            list[n++] = v;
+        }
+    };
+    add(w, nw, std::min<uint32_t>((uint32_t)B200_ALIGN(q.OW, 8), tw_max));
+    add(w, nw, 8);
+    for (uint32_t v = std::min(tw_max, q.OW); nw < 12 && v >= 1; --v) {
+        if (div_up(q.OW, div_up(q.OW, v)) == v) {
+            add(w, nw, v);
         }
     }
-    return best;
+    for (uint32_t v = std::min(128u, q.OH); nh < 12 && v >= 1; --v) {
+        if (div_up(q.OH, div_up(q.OH, v)) == v) {
+            add(h, nh, v);
+        }
+    }
+    if (nh == 12) {   // a tall map: powers of two below
+        for (uint32_t i = 0, v = 64; i < 7; ++i, v >>= 1) {
+            h[5 + i] = v;
+        }
+    }
+    const uint32_t first[3] = {widest, std::min(widest, 128u), 32u};
+    for (uint32_t i = 0; i < nw; ++i) {
+        for (uint32_t j = 0; j < nh; ++j) {
+            consider(w[i], h[j], first, 3);
+        }
+    }
+    if (least == ~0ull) {
+        return false;
+    }
+    uint32_t all[8], n_all = 0;
+    for (uint32_t bn = widest; bn >= 32; bn -= 32) {
+        all[n_all++] = bn;
+    }
+    consider(best->tw, best->th, all, n_all);
+    return true;
 }
 
 // Two CTAs per SM pay where a tile is short and narrow: at most 64 output channels, or at most 128 behind a K
 // of one or two blocks.  Measured on the 22 ResNet-50-shaped layers at batch 64 (u8 output): 3x3 64->64 @56
 // 38.9 -> 28.3 us, 1x1 256->128 @56 28.7 -> 25.0 us, 1x1 64->64 and 256->64 @56 22.5 -> 20.5 us; wider or longer
 // layers lose (3x3 512->512 @14 s2 32.8 -> 51.2 us), the 256-wide tile reads the activations half as often.
-bool conv_prefers_half(uint32_t tiles_m, uint32_t OC, uint32_t num_kb, int sms)
+bool conv_prefers_half(uint32_t OC, uint32_t num_kb)
 {
-    (void)tiles_m;
-    (void)sms;
     return OC <= 64 || (OC <= 128 && num_kb <= 2);
 }
 
@@ -894,51 +971,32 @@ EE launch_conv_tcgen05(const ConvGeom &g, const ConvLaunch &a, cudaStream_t st)
     p.OH = OH;
     p.OW = OW;
     p.OC = OC;
-    // Tile: TW x TH pixels of TN images, at most 128 in all; the shape that needs the fewest tiles, wider rows
-    // first among equals.  With stride 1 along W a row of TW pixels is TW*16 contiguous bytes; the (c16, w)
-    // dimensions are then merged so that TMA moves one 16*TW-byte run per row instead of TW 16-byte ones (a
-    // TMA box is at most 256 elements wide, hence TW <= 16 on that path).
+    // Tile: TW x TH pixels of TN images, at most 128 in all.  With stride 1 along W a row of TW pixels is TW*16
+    // contiguous bytes; the (c16, w) dimensions are then merged so that TMA moves one 16*TW-byte run per row instead
+    // of TW 16-byte ones (a TMA box is at most 256 elements wide, hence TW <= 16 on that path).
     // A tile whose pixel count is a multiple of 8 lets one TMA request bring all 8 channel groups of a
     // 128-byte K block (the groups then lie 128-byte aligned behind one another in shared memory); any other
-    // count needs a request per group, eight times as many.  So such shapes are preferred even when they
-    // overhang the image (TW may exceed OW by up to 7 columns: the overhang reads zeros and is not stored).
+    // count needs a request per group, eight times as many.  A tile may overhang the image: the overhang reads
+    // zeros and is not stored.
     const bool merged_w = (sW == 1);
-    uint64_t best_tiles = ~0ull;
-    uint32_t btw = 0, bth = 0, btn = 0;
-    const uint32_t tw_max = merged_w ? 16u : 128u;
-    const uint32_t ow8 = (uint32_t)B200_ALIGN(OW, 8);
-    for (uint32_t tw = (ow8 < tw_max ? ow8 : tw_max); tw >= 1; --tw) {
-        if (tw * sW > 256) {
-            continue;
-        }
-        for (uint32_t th = (OH < 128 / tw ? OH : 128 / tw); th >= 1; --th) {
-            if (th * sH > 256) {
-                continue;
-            }
-            uint32_t tn = 128 / (tw * th);
-            tn = tn < N ? tn : N;
-            if (tn == 0) {
-                continue;
-            }
-            uint64_t tiles = (uint64_t)((OW + tw - 1) / tw) * ((OH + th - 1) / th) * ((N + tn - 1) / tn);
-            if ((tw * th * tn) % 8 != 0) {
-                tiles *= 4;  // weight of the eightfold request count
-            }
-            if (tiles < best_tiles) {
-                best_tiles = tiles;
-                btw = tw;
-                bth = th;
-                btn = tn;
-            }
-        }
-    }
-    if (btw == 0) {
+    p.total_chunks = FH * FW * g.ICb;
+    p.num_kb = (p.total_chunks + 7) / 8;
+    // which configuration: two CTAs per SM with column blocks of at most 128 channels, or one with up to 256
+    static const int force_half = [] {
+        const char *e = getenv("BOLT_B200_CONV_HALF");
+        return (e == nullptr || e[0] == '\0') ? -1 : atoi(e);
+    }();
+    const bool half_cfg = force_half >= 0 ? force_half != 0 : conv_prefers_half(OC, p.num_kb);
+    TileShape shape;
+    if (!pick_tile(TileProblem{N, OH, OW, OC, sH, sW, p.num_kb, merged_w, FW > 1, half_cfg ? 128u : 256u,
+                       (uint32_t)c->sm_count * (half_cfg ? 2 : 1)}, &shape)) {
         return NOT_SUPPORTED;
     }
-    p.TW = btw;
-    p.TH = bth;
-    p.TN = btn;
-    p.rows = btw * bth * btn;
+    p.TW = shape.tw;
+    p.TH = shape.th;
+    p.TN = shape.tn;
+    p.block_n = shape.block_n;
+    p.rows = p.TW * p.TH * p.TN;
     p.tiles_w = (OW + p.TW - 1) / p.TW;
     p.tiles_h = (OH + p.TH - 1) / p.TH;
     p.tiles_n_img = (N + p.TN - 1) / p.TN;
@@ -959,16 +1017,7 @@ EE launch_conv_tcgen05(const ConvGeom &g, const ConvLaunch &a, cudaStream_t st)
     if (p.rows % 8 != 0) {
         p.G = 1;  // chunks of a box follow each other without gaps; only whole 128-byte units may be merged
     }
-    p.total_chunks = FH * FW * g.ICb;
-    p.num_kb = (p.total_chunks + 7) / 8;
     p.tiles_m = p.tiles_n_img * p.tiles_w * p.tiles_h;
-    // which configuration: two CTAs per SM with column blocks of at most 128 channels, or one with up to 256
-    static const int force_half = [] {
-        const char *e = getenv("BOLT_B200_CONV_HALF");
-        return (e == nullptr || e[0] == '\0') ? -1 : atoi(e);
-    }();
-    const bool half_cfg = force_half >= 0 ? force_half != 0 : conv_prefers_half(p.tiles_m, OC, p.num_kb, c->sm_count);
-    p.block_n = half_cfg ? pick_conv_block_n(p.tiles_m, OC, 2 * c->sm_count, 128) : pick_conv_block_n(p.tiles_m, OC, c->sm_count);
     p.tiles_n = (OC + p.block_n - 1) / p.block_n;
     // A small tile (few pixels, a narrow column block) takes as many stages as fit: with few tiles the layer is bound
     // by the latency of its loads.  The MMA reads 128 rows of every chunk, beyond a tile's last one: bytes of the
