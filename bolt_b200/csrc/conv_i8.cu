@@ -230,7 +230,7 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     uint8_t *smem_b = smem + p.stages * p.a_stage;
     SmemCtl<NB> *ctl = reinterpret_cast<SmemCtl<NB> *>(smem + CF::RING_BYTES);
 
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = warp_index();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t num_tiles = p.tiles_m * p.tiles_n;
     const uint32_t chunk_bytes = p.rows * 16;   // one 16-byte K chunk of all the tile's pixels
@@ -282,20 +282,24 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
                 uint32_t n, oh0, ow0, n0;
                 decode(tile, n, oh0, ow0, n0);
                 for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
-                    if (!mbar_wait(&ctl->empty[stage], phase ^ 1)) {
+                    if (!mbar_wait_warp(&ctl->empty[stage], phase ^ 1)) {
                         ok = false;
                         break;
                     }
                     const uint32_t q0 = kb * 8;
                     const uint32_t nq = min(8u, p.total_chunks - q0);
-                    mbar_expect_tx(&ctl->full[stage], nq * chunk_bytes + p.block_n * BLOCK_K);
+                    if (leader) {
+                        mbar_expect_tx(&ctl->full[stage], nq * chunk_bytes + p.block_n * BLOCK_K);
+                        tma_load_2d(&map_w, &ctl->full[stage], smem_b + stage * p.b_stage, (int)(kb * BLOCK_K), (int)n0);
+                    }
                     for (uint32_t j = 0; j < nq; j += p.G) {
                         const uint32_t q = q0 + j;
                         const uint32_t tap = q / p.ICb;
@@ -305,21 +309,22 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         // taps outside the image start at negative or too large coordinates and read zeros
                         const int x = (int)(ow0 * p.sW + kw * p.dW) - p.pl;
                         const int y = (int)(oh0 * p.sH + kh * p.dH) - p.pt;
-                        if (p.merged_w) {
+                        if (!leader) {
+                        } else if (p.merged_w) {
                             // a row of TW pixels is TW * 16 contiguous bytes: one wide request per row
                             tma_load_4d(&map_x, &ctl->full[stage], dst, x * 16, y, (int)n, (int)cb);
                         } else {
                             tma_load_5d(&map_x, &ctl->full[stage], dst, 0, x, y, (int)n, (int)cb);
                         }
                     }
-                    tma_load_2d(&map_w, &ctl->full[stage], smem_b + stage * p.b_stage, (int)(kb * BLOCK_K), (int)n0);
+                    __syncwarp();
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
             }
-            if (!ok) {
+            if (!ok && leader) {
                 atomicExch(p.status, 11);
                 atomicExch(&ctl->abort_flag, 1u);
             }
@@ -327,7 +332,8 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ---------------------------------------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();   // (commits follow the MMAs of the thread that issues them)
             const uint32_t idesc = make_idesc_i8(p.block_n);
             uint32_t stage = 0, phase = 0;
             uint32_t it = 0;
@@ -335,14 +341,14 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
             for (uint32_t tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++it) {
                 const uint32_t acc = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
-                if (!mbar_wait(&ctl->tmem_empty[acc], acc_phase ^ 1)) {
+                if (!mbar_wait_warp(&ctl->tmem_empty[acc], acc_phase ^ 1)) {
                     ok = false;
                     break;
                 }
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + acc * CF::MAX_N;
                 for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
-                    if (!mbar_wait(&ctl->full[stage], phase)) {
+                    if (!mbar_wait_warp(&ctl->full[stage], phase)) {
                         ok = false;
                         break;
                     }
@@ -355,9 +361,14 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                         // beyond the tile's pixels read the next chunk's bytes: their accumulators are never
                         // stored.  An odd last chunk pairs with stale bytes, which meet zero weights.
                         const uint64_t da = make_desc_noswizzle(a_addr + k * 2 * chunk_stride, chunk_stride, 128);
-                        umma_i8(tmem_d, da, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        if (leader) {
+                            umma_i8(tmem_d, da, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                        }
                     }
-                    tcgen05_commit(&ctl->empty[stage]);
+                    if (leader) {
+                        tcgen05_commit(&ctl->empty[stage]);
+                    }
+                    __syncwarp();
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
@@ -366,9 +377,12 @@ conv_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
                 if (!ok) {
                     break;
                 }
-                tcgen05_commit(&ctl->tmem_full[acc]);
+                if (leader) {
+                    tcgen05_commit(&ctl->tmem_full[acc]);
+                }
+                __syncwarp();
             }
-            if (!ok) {
+            if (!ok && leader) {
                 atomicExch(p.status, 12);
                 atomicExch(&ctl->abort_flag, 1u);
             }

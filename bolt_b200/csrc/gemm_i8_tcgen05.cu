@@ -422,7 +422,7 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     uint8_t *smem_staging = smem + SMEM_RING_BYTES;  // 1024-byte aligned
     SmemCtl *ctl = reinterpret_cast<SmemCtl *>(smem + SMEM_RING_BYTES + SMEM_STAGING_BYTES);
 
-    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t warp = warp_index();
     const uint32_t lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -473,7 +473,8 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             // this CTA's slice of the memory a later kernel will read, requested once the pipeline is filled
@@ -488,13 +489,14 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const int n0 = (int)(t.n0 + rank * my_rows);
                 const uint32_t tile_bytes = (PAIR ? 2u : 1u) * (p.a_rows + my_rows) * BLOCK_K;
                 for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
-                    if (!mbar_wait(&ctl->empty[stage], phase ^ 1)) {
+                    if (!mbar_wait_warp(&ctl->empty[stage], phase ^ 1)) {
                         ok = false;
                         break;
                     }
                     uint8_t *sa = smem_a + stage * a_stage;
                     uint8_t *sb = smem_b + stage * b_stage;
-                    if (PAIR) {
+                    if (!leader) {
+                    } else if (PAIR) {
                         // both CTAs' bytes are expected by, and complete on, the leader's barrier
                         const uint32_t bar = mapa_shared(smem_u32(&ctl->full[stage]), 0);
                         if (rank == 0) {
@@ -507,6 +509,7 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         tma_load_2d(&map_a, &ctl->full[stage], sa, (int)(kb * BLOCK_K), m0);
                         tma_load_2d(&map_b, &ctl->full[stage], sb, (int)(kb * BLOCK_K), n0);
                     }
+                    __syncwarp();
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
@@ -515,14 +518,14 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         const size_t off = (size_t)blockIdx.x * p.prefetch_slice;
                         if (off < p.ep.prefetch_bytes) {
                             const size_t n = min((size_t)p.prefetch_slice, p.ep.prefetch_bytes - off) & ~(size_t)15;
-                            if (n != 0) {
+                            if (n != 0 && leader) {
                                 prefetch_l2_bulk(reinterpret_cast<const uint8_t *>(p.ep.prefetch) + off, (uint32_t)n);
                             }
                         }
                     }
                 }
             }
-            if (!ok) {
+            if (!ok && leader) {
                 atomicExch(p.status, 1);
                 atomicExch(&ctl->abort_flag, 1u);
             }
@@ -530,7 +533,8 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- MMA issuer ---------------------------------------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const bool leader = elect_one();   // (commits follow the MMAs of the thread that issues them)
             uint32_t stage = 0, phase = 0;
             uint32_t it = 0;
             bool ok = true;
@@ -541,36 +545,39 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const uint32_t idesc = make_idesc_i8(t.units * 32, PAIR ? 2 * BLOCK_M : BLOCK_M);
                 const uint32_t acc = it & 1;
                 const uint32_t acc_phase = (it >> 1) & 1;
-                if (!mbar_wait(&ctl->tmem_empty[acc], acc_phase ^ 1)) {
+                if (!mbar_wait_warp(&ctl->tmem_empty[acc], acc_phase ^ 1)) {
                     ok = false;
                     break;
                 }
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + acc * MAX_BLOCK_N;
                 for (uint32_t kb = 0; kb < p.num_kb; ++kb) {
-                    if (!mbar_wait(&ctl->full[stage], phase)) {
+                    if (!mbar_wait_warp(&ctl->full[stage], phase)) {
                         ok = false;
                         break;
                     }
                     tcgen05_fence_after();
                     const uint64_t da = make_desc_sw128(smem_u32(smem_a + stage * a_stage));
                     const uint64_t db = make_desc_sw128(smem_u32(smem_b + stage * b_stage));
+                    if (leader) {
 #pragma unroll
-                    for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                        // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the
-                        // 16-byte units of the descriptor's start-address field
+                        for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                            // advancing K inside the 128-byte swizzle row: +32 bytes = +2 in the
+                            // 16-byte units of the descriptor's start-address field
+                            if (PAIR) {
+                                umma_i8_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            } else {
+                                umma_i8(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            }
+                        }
+                        // frees the stage (in both CTAs) once these MMAs retire
                         if (PAIR) {
-                            umma_i8_pair(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            tcgen05_commit_pair(&ctl->empty[stage]);
                         } else {
-                            umma_i8(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                            tcgen05_commit(&ctl->empty[stage]);
                         }
                     }
-                    // frees the stage (in both CTAs) once these MMAs retire
-                    if (PAIR) {
-                        tcgen05_commit_pair(&ctl->empty[stage]);
-                    } else {
-                        tcgen05_commit(&ctl->empty[stage]);
-                    }
+                    __syncwarp();
                     if (++stage == p.stages) {
                         stage = 0;
                         phase ^= 1;
@@ -579,13 +586,15 @@ gemm_u8s8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 if (!ok) {
                     break;
                 }
-                if (PAIR) {
+                if (!leader) {
+                } else if (PAIR) {
                     tcgen05_commit_pair(&ctl->tmem_full[acc]);
                 } else {
                     tcgen05_commit(&ctl->tmem_full[acc]);
                 }
+                __syncwarp();
             }
-            if (!ok) {
+            if (!ok && leader) {
                 atomicExch(p.status, 2);
                 atomicExch(&ctl->abort_flag, 1u);
             }
