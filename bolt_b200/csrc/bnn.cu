@@ -18,7 +18,7 @@
 // long as both operands use the same one: word j of 8 takes bits j, j+8, j+16, j+24, one shift and one mask.
 //
 // Measured, 256 -> 256 channels, 3 x 3 on 28 x 28, batch 128, whole call: 519 us with XOR + popcount (16 per clock and
-// SM: 411 us of popcounts alone), 90 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
+// SM: 411 us of popcounts alone), 86 us with this; 26 us is the tensor pipe's share, 15 us the bytes.
 #include <cuda_fp16.h>
 
 #include <cstring>
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = align_1024(smem_raw);
     BnnCtl *ctl = reinterpret_cast<BnnCtl *>(smem + 2 * STAGE);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&ctl->full[i], WIDEN_THREADS / 32);
@@ -192,17 +192,18 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
 
     if (warp == WIDEN_THREADS / 32) {
         // ------------------------------- MMA issuer ---------------------------------------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();   // (commits follow the MMAs of the thread that issues them)
             const uint32_t idesc = make_idesc_i8(p.block_n);
             uint32_t issued = 0, it = 0;
             for (uint32_t tile = blockIdx.x; !dead && tile < tiles; tile += gridDim.x, ++it) {
-                if (it != 0 && !mbar_wait(&ctl->drained, (it - 1) & 1)) {
+                if (it != 0 && !mbar_wait_warp(&ctl->drained, (it - 1) & 1)) {
                     dead = true;
                     break;
                 }
                 for (uint32_t kb = 0; kb < num_kb; ++kb, ++issued) {
                     const uint32_t s = issued & 1;
-                    if (!mbar_wait(&ctl->full[s], (issued >> 1) & 1)) {
+                    if (!mbar_wait_warp(&ctl->full[s], (issued >> 1) & 1)) {
                         dead = true;
                         break;
                     }
@@ -213,10 +214,15 @@ __global__ void __launch_bounds__(THREADS, 2) bnn_conv_kernel(const __grid_const
                         const uint64_t da = make_desc_sw128(smem_u32(sa + r * BLOCK_M * BLOCK_K));
 #pragma unroll
                         for (uint32_t q = 0; q < 4; ++q) {
-                            umma_i8(tmem_base + r * MAX_BN, da + 2 * q, db + 2 * q, idesc, (kb | q) != 0 ? 1u : 0u);
+                            if (leader) {
+                                umma_i8(tmem_base + r * MAX_BN, da + 2 * q, db + 2 * q, idesc, (kb | q) != 0 ? 1u : 0u);
+                            }
                         }
                     }
-                    tcgen05_commit(&ctl->done[s]);
+                    if (leader) {
+                        tcgen05_commit(&ctl->done[s]);
+                    }
+                    __syncwarp();
                 }
             }
         }

@@ -11,7 +11,7 @@
 // latency and by the load / store instructions, not by the tensor pipe.
 //
 // Measured, 333 x 515 x 1001 u8 x s8 -> fp32 behind its dynamic quantization, whole calls: 111 us with the 16 x 16
-// CUDA-core kernel that stood here, 38 us with this one (about 30 us of it are the quantization and the host).
+// CUDA-core kernel that stood here, 37 us with this one (about 30 us of it are the quantization and the host).
 #include <cuda.h>
 
 #include <algorithm>
@@ -399,7 +399,7 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
     uint8_t *smem = align_1024(smem_raw);
     const uint32_t stage_bytes = STAGE_A + p.block_n * BLOCK_K;   // both tiles stay 1024-byte aligned
     Ctl *ctl = reinterpret_cast<Ctl *>(smem + 2 * (size_t)(STAGE_A + MAX_BN * BLOCK_K));
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         mbar_init(&ctl->done[0], 1);
@@ -489,14 +489,19 @@ gemm_gather_kernel(const __grid_constant__ GatherParams p, const __grid_constant
                 dead = true;
                 break;
             }
-            if (threadIdx.x == 0) {
+            if (warp == 0) {
+                const bool leader = elect_one();   // the same lane every time
                 tcgen05_fence_after();
                 const uint64_t da = make_desc_sw128(smem_u32(sa)), db = make_desc_sw128(smem_u32(sb));
                 const uint32_t steps = (min((uint32_t)BLOCK_K, p.K - kb * BLOCK_K) + UMMA_K - 1) / UMMA_K;
                 for (uint32_t k = 0; k < steps; ++k) {
-                    umma_i8(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                    if (leader) {
+                        umma_i8(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
+                    }
                 }
-                tcgen05_commit(&ctl->done[s]);
+                if (leader) {
+                    tcgen05_commit(&ctl->done[s]);
+                }
             }
             __syncwarp();
         }
@@ -931,7 +936,7 @@ Operand operand(const MatmulOperand &o, uint32_t rows, uint32_t K, bool rows_con
 
 // All products of a matmul call: at most one pass over the binary32 operands for their scales, then one kernel that
 // quantizes, multiplies and converts.  BERT-base attention of 32 x 128 tokens, scores and context (384 products of
-// 128 x 64 x 128 and of 128 x 128 x 64): 49 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
+// 128 x 64 x 128 and of 128 x 128 x 64): 47 us against 8.0 ms for a pack and a GEMM launch per product.  Its memory
 // floor is 15 us (each operand and result once); the operands are read a second time for their scales.
 EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
 {

@@ -194,15 +194,22 @@ cudaError_t launch(const SkinnyParams &p, bool pdl, cudaStream_t st)
 
 }  // namespace
 
-// Few rows and a weight of at most 32 MiB and 6144 columns: beyond that the TMA kernel streams as fast.  Measured, us per
-// product in a graph of forty, this kernel against that one: 16 x 768 x 3072 3.0 / 4.6, 16 x 3072 x 768 3.2 / 8.6,
-// 16 x 4096 x 4096 5.6 / 10.9, 16 x 8192 x 4096 10.9 / 18.8, 16 x 1024 x 16384 7.0 / 6.2, 16 x 4096 x 12288 17.9 / 13.1;
-// 32 x 768 x 3072 3.4 / 4.5, 32 x 8192 x 4096 17.7 / 18.8.  From 33 rows on it only pays with 8 columns per CTA:
-// 48 x 3072 x 768 5.1 / 8.6, 64 x 256 x 1024 2.7 / 3.5, but 64 x 768 x 3072 6.1 / 4.5.
+// Few rows, and a weight of at most 32 MiB and 6144 columns: beyond that the TMA kernel streams as fast.  Measured, us per
+// product in a graph of forty, this kernel against that one (whose time does not depend on so few rows): 16 rows x 768 x
+// 3072 3.0 / 4.0, 3072 x 768 3.2 / 7.1, 4096 x 4096 5.6 / 8.9, 8192 x 4096 10.9 / 15.1, 1024 x 16384 7.0 / 5.8, 4096 x 12288
+// 17.9 / 12.2.  With 32 rows 768 x 3072 3.4 / 4.0, 1024 x 4096 3.6 / 4.4, 8192 x 2048 7.8 / 14.6, but 4096 x 4096 9.3 / 8.9,
+// 8192 x 4096 17.7 / 15.1.  From 33 rows on it only pays with 8 columns per CTA: 48 x 3072 x 768 5.1 / 7.1, 64 x 256 x 1024
+// 2.7 / 3.2, but 64 x 768 x 3072 6.1 / 4.0.
 bool gemm_skinny_preferred(uint32_t M, uint32_t N, uint32_t K, int sms)
 {
-    const bool rows = M <= 32 || (M <= 64 && N <= 8 * (uint32_t)sms);
-    return rows && N <= 6144 && (uint64_t)N * K <= (32ull << 20);
+    const uint64_t weight = (uint64_t)N * K;
+    if (M <= 16) {
+        return N <= 6144 && weight <= (32ull << 20);
+    }
+    if (M <= 32) {
+        return weight <= (12ull << 20) ? N <= 6144 : (N <= 2048 && weight <= (32ull << 20));
+    }
+    return M <= 64 && N <= 8 * (uint32_t)sms && weight <= (32ull << 20);
 }
 
 // The operands satisfy gemm_tcgen05_eligible.  preload: see SkinnyParams.

@@ -184,7 +184,7 @@ U32 global_index(uint64_t ic, const TensorDesc &c, const TensorDesc &x)
 // kernel never packs and keeps the host out of it, but it converts an fp32 operand again for every tile row / column
 // of the other one and fills the tensor pipe a quarter as well.  Measured (fp32 in and out, us per call, one launch
 // against one by one): 1 x 512^3 37 / 75, 1 x 1024^3 73 / 83, 1 x 2048^3 209 / 112; 4 x 512^3 42 / 123,
-// 4 x 1024^3 112 / 145, 4 x 2048^3 903 / 272; 384 x (128 x 64 x 128 and 128 x 128 x 64) 57 / 8000 for the pair.
+// 4 x 1024^3 112 / 145, 4 x 2048^3 903 / 272; 384 x (128 x 64 x 128 and 128 x 128 x 64) 47 / 8000 for the pair.
 bool one_launch(const Plan &p)
 {
     const uint64_t M = p.a.dims[1 - p.kDimA], N = p.b.dims[1 - p.kDimB], K = p.a.dims[p.kDimA];
