@@ -101,9 +101,14 @@ class LinearStack:
         """The layers' calls, activations ping-ponging between two device buffers.  Kept between passes, and made anew
         when a buffer or a scale is another one."""
         fac = getattr(self, "layer_factors", None)
-        key = [self.M, self.d_scale.data_ptr(), self.out_dev.data_ptr(), self.act[0].data_ptr(), self.act[1].data_ptr(), *self.out_scales]
-        key += [v for l in self.layers for v in (l.K, l.N, l.packed.data_ptr(), l.offsetC_ptr, l.uniform, l.w_scale.data_ptr(), float(l.w_scale_host[0]))]
-        key += [f.data_ptr() for f in fac or ()]
+        key = [self.M, self.d_scale.data_ptr(), self.out_dev.data_ptr(), self.act[0].data_ptr(), self.act[1].data_ptr(),
+               float(self.layers[0].w_scale_host[0]), *self.out_scales]
+        for l in self.layers:
+            key += (l.packed.data_ptr(), l.offsetC_ptr, l.uniform, l.w_scale.data_ptr())
+        if fac is not None:
+            key += [f.data_ptr() for f in fac]
+        else:
+            key += [float(l.w_scale_host[0]) for l in self.layers]
         if getattr(self, "_calls_key", None) != key:
             last = len(self.layers) - 1
             calls = (GemmCall * len(self.layers))()
