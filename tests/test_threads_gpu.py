@@ -1,0 +1,69 @@
+"""Several host threads, each with a stream of its own, through the calls whose scale is found on the device: the reported
+maxima and the shared pool behind them must not mix.  Every thread's bytes and scales against its own serial run."""
+import ctypes as C
+import os
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(__file__))
+import bolt_b200 as B  # noqa: E402
+from bolt_b200 import synth  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+THREADS, ROUNDS = 70, 12     # more threads than the pool has entries
+
+
+class Work:
+    def __init__(self, t):
+        import torch
+
+        self.n = 1000 + 517 * t
+        self.x = torch.from_numpy((synth.normal(t, (self.n,)) * np.float32(0.1 + t)).astype(np.float32)).cuda()
+        self.acc = torch.from_numpy(synth.integers(t + 500, (self.n,), -1000 * (t + 1), 1000 * (t + 1)).astype(np.int32)).cuda()
+        self.q, self.r = (torch.empty(self.n, dtype=torch.uint8, device="cuda") for _ in range(2))
+        self.a = torch.from_numpy(synth.normal(t + 900, (2, 24, 32)) * np.float32(1 + t)).cuda()
+        self.b = torch.from_numpy(synth.normal(t + 901, (2, 32, 40))).cuda()
+        self.c = torch.empty((2, 24, 40), dtype=torch.uint8, device="cuda")
+        ad, bd = B.tensor_nd(B.DT_F32, (2, 24, 32)), B.tensor_nd(B.DT_F32, (2, 32, 40))
+        cd = B.matmul_infer_output_size(ad, 0, bd, 0)
+        cd.dt = B.DT_U8_Q
+        self.nb = B.matmul_infer_forward_tmp_bytes(ad, 0, bd, 0, cd, -1.0)
+        self.tmp = torch.empty(self.nb, dtype=torch.uint8, device="cuda")
+        self.ad, self.bd, self.cd = ad, bd, cd
+
+    def run(self):
+        p = lambda t: C.c_void_p(t.data_ptr())
+        sq, sr = [-1.0], [-1.0, 40.0]
+        B.quantize(B.tensor1d(B.DT_F32, self.n), p(self.x), B.tensor1d(B.DT_U8_Q, self.n), p(self.q), sq)
+        B.quantize(B.tensor1d(B.DT_I32, self.n), p(self.acc), B.tensor1d(B.DT_U8_Q, self.n), p(self.r), sr)
+        sm = B.matmul(self.ad, 0, p(self.a), -1.0, self.bd, 0, p(self.b), -1.0, None, None, self.nb, p(self.tmp), self.cd, p(self.c), -1.0)
+        B.CHECK_STATUS(B.lib().bolt_b200_synchronize(), "synchronize")
+        return (sq[0], sr[0], float(sm), self.q.cpu().numpy().tobytes(), self.r.cpu().numpy().tobytes(), self.c.cpu().numpy().tobytes())
+
+
+def test_threads_and_streams_do_not_mix():
+    import torch
+
+    works = [Work(t) for t in range(THREADS)]
+    expect = [w.run() for w in works]
+    torch.cuda.synchronize()
+    bad = []
+
+    def body(t):
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            B.CHECK_STATUS(B.lib().bolt_b200_set_stream(C.c_void_p(st.cuda_stream)))
+            for i in range(ROUNDS):
+                if works[t].run() != expect[t]:
+                    bad.append((t, i))
+            B.CHECK_STATUS(B.lib().bolt_b200_set_stream(None))
+
+    ts = [threading.Thread(target=body, args=(t,)) for t in range(THREADS)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad[:10]
