@@ -1277,14 +1277,17 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
     if (tmpBytes < need) {
         return NOT_MATCH;
     }
+    const size_t out_elems = (size_t)g.out.n * g.out.c * g.out.h * g.out.w;
+    const size_t in_elems = (size_t)g.in.n * g.in.c * g.in.h * g.in.w;
+    if (out_elems == 0 || in_elems == 0 || g.K == 0) {
+        return NOT_SUPPORTED;  // no tile covers an empty tensor (pick_tile divides by these extents)
+    }
     DeviceCtx *c = ctx();
     if (c == nullptr) {
         return UNKNOWN;
     }
     cudaStream_t st = tls().stream;
     F32 *sc = reinterpret_cast<F32 *>(scale);
-    const size_t out_elems = (size_t)g.out.n * g.out.c * g.out.h * g.out.w;
-    const size_t in_elems = (size_t)g.in.n * g.in.c * g.in.h * g.in.w;
     const size_t ts_off = filter_tapsum_off(g.f.n, g.OCr, g.K);
     const size_t w_bytes = ts_off + 4 * (size_t)g.f.n * g.taps;
 
