@@ -559,14 +559,17 @@ EE bnn_run(const TensorDesc *inputDesc, const void *input, const TensorDesc *fil
     if (tmpBytes < need) {
         return NOT_MATCH;
     }
+    const size_t in_elems = (size_t)g.in.n * g.in.c * g.in.h * g.in.w;
+    const size_t out_elems = (size_t)g.out.n * g.out.c * g.out.h * g.out.w;
+    if (in_elems == 0 || out_elems == 0) {
+        return NOT_SUPPORTED;  // pick_tile divides by the channel blocks, and the kernel's walk over K by the words of a tap
+    }
     DeviceCtx *c = ctx();
     if (c == nullptr) {
         return UNKNOWN;
     }
     cudaStream_t st = tls().stream;
     const bool xnor = g.f.dt == DT_BIN11;
-    const size_t in_elems = (size_t)g.in.n * g.in.c * g.in.h * g.in.w;
-    const size_t out_elems = (size_t)g.out.n * g.out.c * g.out.h * g.out.w;
     const size_t w_words = (size_t)g.f.n * g.taps * g.Cw;
     Stage sg;
     const __half *d_in = reinterpret_cast<const __half *>(sg.in(input, in_elems * 2));

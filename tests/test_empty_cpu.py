@@ -30,3 +30,9 @@ def convolution_code(n, ic, oc, out_dt=B.DT_F32, hw=8, binary=False):
 @pytest.mark.parametrize("out_dt", [B.DT_F32, B.DT_U8_Q])
 def test_convolution_without_images_or_channels(n, ic, oc, out_dt):
     assert convolution_code(n, ic, oc, out_dt) == B.NOT_SUPPORTED
+
+
+@pytest.mark.parametrize("n,ic,oc", [(0, 32, 64), (1, 32, 0), (1, 0, 64), (0, 0, 0)])
+def test_one_bit_convolution_without_images_or_channels(n, ic, oc):
+    """(without input channels the kernel's walk over the words of a tap would not end)"""
+    assert convolution_code(n, ic, oc, binary=True) == B.NOT_SUPPORTED
