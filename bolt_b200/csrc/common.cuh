@@ -126,9 +126,10 @@ struct DeviceCtx {
     unsigned *d_scratch_u = nullptr;
     std::mutex mu;       // guards the staging workspace (one staged call at a time)
     std::mutex twin_mu;  // guards twins
-    std::mutex mail_mu;     // guards mail_free
+    std::mutex mail_mu;     // guards mail_free and mails
     std::condition_variable mail_cv;
     std::vector<MaxMail *> mail_free;
+    int mails = 0;          // in the pool or in use
     std::map<const void *, WeightTwin> twins;  // host packed weight -> device copy
     // growable staging workspace for host-pointer calls
     char *ws = nullptr;
@@ -151,22 +152,36 @@ inline void count_launch(int n = 1)
     g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed);
 }
 
-// One MaxMail for the duration of a call (found on a stream that is not being captured: the host has to wait).
+// One MaxMail for the duration of a call (found on a stream that is not being captured: the host has to wait):
+// ok(), launch a kernel with mail(), launched() if that succeeded, wait().
 class MaxLease {
 public:
     explicit MaxLease(DeviceCtx *c);
     ~MaxLease();
+    MaxLease(const MaxLease &) = delete;
+    MaxLease &operator=(const MaxLease &) = delete;
+    bool ok() const
+    {
+        return m_ != nullptr;
+    }
     const MaxMail &mail() const
     {
         return *m_;
     }
-    // the maximum that the kernel launched on `st` with this mail reports
-    EE wait(cudaStream_t st, int *maximum);
+    // from here on the mail belongs to a kernel on `st`, until that is seen to have reported
+    void launched(cudaStream_t st)
+    {
+        in_flight_ = true;
+        st_ = st;
+    }
+    // the maximum that the kernel reports
+    EE wait(int *maximum);
 
 private:
     DeviceCtx *c_;
-    MaxMail *m_;
-    bool lost_ = false;   // the kernel did not report: its words may be half counted and are not used again
+    MaxMail *m_ = nullptr;
+    cudaStream_t st_ = nullptr;
+    bool in_flight_ = false;
 };
 bool capturing(cudaStream_t st);
 

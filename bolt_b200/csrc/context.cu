@@ -1,6 +1,4 @@
 // context.cu -- per-device state, the staging of host pointers, and the runtime entry points.
-#include <sched.h>
-
 #include <cstring>
 
 #include "common.cuh"
@@ -93,6 +91,7 @@ DeviceCtx *ctx()
             m->seq = 0;
             c->mail_free.push_back(m);
         }
+        c->mails = MAX_MAILS;
         __atomic_store_n(&g_ctx[dev], c, __ATOMIC_RELEASE);
     } else {
         int cur = -1;
@@ -114,67 +113,6 @@ EE raise_smem_limit(DeviceCtx *c, KernelFamily f, const void *const *kernels, in
     }
     c->smem_raised[f] = true;
     return SUCCESS;
-}
-
-MaxLease::MaxLease(DeviceCtx *c) : c_(c)
-{
-    std::unique_lock<std::mutex> g(c->mail_mu);
-    c->mail_cv.wait(g, [&] { return !c->mail_free.empty(); });
-    m_ = c->mail_free.back();
-    c->mail_free.pop_back();
-    if (++m_->seq == 0) {
-        m_->seq = 1;
-    }
-}
-
-MaxLease::~MaxLease()
-{
-    if (lost_) {
-        return;
-    }
-    {
-        std::lock_guard<std::mutex> g(c_->mail_mu);
-        c_->mail_free.push_back(m_);
-    }
-    c_->mail_cv.notify_one();
-}
-
-EE MaxLease::wait(cudaStream_t st, int *maximum)
-{
-    auto arrived = [&] {
-        const unsigned long long v = *m_->h_mail;
-        *maximum = (int)(unsigned)v;
-        return (uint32_t)(v >> 32) == m_->seq;
-    };
-    for (uint32_t spin = 1;; ++spin) {
-        if (arrived()) {
-            return SUCCESS;
-        }
-        __builtin_ia32_pause();
-        if ((spin & 0x3FFF) == 0) {   // some hundred microseconds: is the stream still at work?
-            const cudaError_t e = cudaStreamQuery(st);
-            if (e == cudaErrorNotReady) {
-                cudaGetLastError();
-                sched_yield();
-                continue;
-            }
-            if (e == cudaSuccess && arrived()) {
-                return SUCCESS;
-            }
-            lost_ = true;
-            return e == cudaSuccess ? UNKNOWN : cuda_ee(e);
-        }
-    }
-}
-
-bool capturing(cudaStream_t st)
-{
-    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
-        cudaGetLastError();
-        return true;   // the legacy stream beside another stream's capture
-    }
-    return s != cudaStreamCaptureStatusNone;
 }
 
 bool is_device_ptr(const void *p)

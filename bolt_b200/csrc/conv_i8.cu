@@ -1359,6 +1359,9 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
             return UNKNOWN;   // the scale has to reach the host
         }
         lease.emplace(c);
+        if (!lease->ok()) {
+            return UNKNOWN;
+        }
         a.mail = lease->mail();
     }
 
@@ -1391,6 +1394,9 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
         ret = launch_conv_tcgen05(g, a, st);
     }
     B200_EE(ret);
+    if (find_max) {
+        lease->launched(st);
+    }
     if (fused_u8) {
         sc[1] = ext_out_scale;
     } else if (f32_staged) {
@@ -1399,7 +1405,7 @@ EE conv_i8_run(const TensorDesc *inputDesc, void *input, void *eltwiseInput, con
         sc[1] = s;
     } else if (out_u8) {
         int mx = 0;
-        B200_EE(lease->wait(st, &mx));
+        B200_EE(lease->wait(&mx));
         F32 scales[2] = {-1, scaleO};
         B200_EE(quantize_i32_u8_device(reinterpret_cast<const int32_t *>(a.out), out_elems, mx, reinterpret_cast<uint8_t *>(d_out), scales));
         sc[1] = scales[0];

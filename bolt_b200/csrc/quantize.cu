@@ -70,13 +70,23 @@ __global__ void __launch_bounds__(MAX_TPB) absmax_kernel(const T *__restrict__ x
         }
     }
 }
+// A launch judged by its own status, not by the thread's last error: that may be an earlier call's.
+template <typename... P, typename... A>
+cudaError_t launch(uint32_t grid, uint32_t block, cudaStream_t st, void (*kernel)(P...), A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    count_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 template <typename T>
-void launch_absmax(DeviceCtx *c, const T *x, uint64_t n, const MaxMail &m, cudaStream_t st)
+cudaError_t launch_absmax(DeviceCtx *c, const T *x, uint64_t n, const MaxMail &m, cudaStream_t st)
 {
     // a block takes 16 KiB at least; four blocks per SM at most (all resident)
     const uint64_t blocks = (n + 8 * MAX_TPB - 1) / (8 * MAX_TPB), cap = 4 * (uint64_t)c->sm_count;
-    absmax_kernel<T><<<(uint32_t)(blocks < cap ? blocks : cap), MAX_TPB, 0, st>>>(x, n, m);
-    count_launch();
+    return launch((uint32_t)(blocks < cap ? blocks : cap), MAX_TPB, st, absmax_kernel<T>, x, n, m);
 }
 
 // 127 / absmax on the device (quantize.cpp:63-67), for pipelines that never leave the stream
@@ -165,9 +175,7 @@ EE launch_to8(const SrcT *x, uint64_t n, uint8_t *q, Op op, cudaStream_t st)
     if (blocks > 0x7FFFFFFFull) {
         return NOT_SUPPORTED;
     }
-    to8_kernel<SrcT, Op><<<(uint32_t)blocks, TPB, 0, st>>>(x, n, q, op);
-    count_launch();
-    B200_CUDA(cudaGetLastError());
+    B200_CUDA(launch((uint32_t)blocks, TPB, st, to8_kernel<SrcT, Op>, x, n, q, op));
     return SUCCESS;
 }
 
@@ -287,9 +295,12 @@ EE absmax_host(const T *d_x, uint64_t n, int *mx)
         return SUCCESS;
     }
     MaxLease lease(c);
-    launch_absmax(c, d_x, n, lease.mail(), st);
-    B200_CUDA(cudaGetLastError());
-    return lease.wait(st, mx);
+    if (!lease.ok()) {
+        return UNKNOWN;
+    }
+    B200_CUDA(launch_absmax(c, d_x, n, lease.mail(), st));
+    lease.launched(st);
+    return lease.wait(mx);
 }
 EE absmax_f32_host(const float *d_x, uint64_t n, float *mx)
 {
@@ -409,6 +420,7 @@ EE quantize_cuda_b200(const TensorDesc *dDesc, const void *data, TensorDesc *qDe
     } else if (sdt == DT_U8_Q) {
         u8_to_i8_kernel<<<grid, TPB, 0, st>>>(reinterpret_cast<const uint8_t *>(d_src), n, d_q);
         count_launch();
+        B200_CUDA(cudaGetLastError());
     } else {
         float raw = 0;  // quantize.cpp:320-326 / 369-375
         if (scale[0] < 0 && scale[1] > 0) {
@@ -426,7 +438,6 @@ EE quantize_cuda_b200(const TensorDesc *dDesc, const void *data, TensorDesc *qDe
         }
         count_launch();
     }
-    B200_CUDA(cudaGetLastError());
     return sg.finish();
 }
 
@@ -443,7 +454,7 @@ EE bolt_b200_absmax_scale_f32(const F32 *data, uint64_t n, F32 *d_scale)
     unsigned *bits = c->d_scratch_u + 2;
     B200_CUDA(cudaMemsetAsync(bits, 0, 4, st));
     if (n > 0) {
-        launch_absmax(c, data, n, MaxMail{bits, nullptr, nullptr, 0}, st);
+        B200_CUDA(launch_absmax(c, data, n, MaxMail{bits, nullptr, nullptr, 0}, st));
     }
     finalize_scale_kernel<<<1, 1, 0, st>>>(bits, d_scale);
     count_launch();
