@@ -296,6 +296,12 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
     if (tmp == nullptr || tmpBytes < need) {
         return NOT_MATCH;
     }
+    if (p.loopsC == 0) {
+        return SUCCESS;  // an empty batch
+    }
+    if (p.loopsA == 0 || p.loopsB == 0) {
+        return NOT_MATCH;  // products of operands that do not exist
+    }
     const uint64_t nA = elems(p.a), nB = elems(p.b), nC = elems(p.c);
     const size_t bias_bytes = (bias != nullptr && biasDesc != nullptr) ? (size_t)elems(*biasDesc) * bytes_of(biasDesc->dt) : 0;
     cudaStream_t st = tls().stream;

@@ -1,0 +1,46 @@
+"""Host paths of the library against a CUDA runtime without a device (fake_gpu.py)."""
+import ctypes as C
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(__file__))
+import bolt_b200 as B  # noqa: E402
+import fake_gpu  # noqa: E402
+
+F, U, I = B.DT_F32, B.DT_U8_Q, B.DT_I8
+
+
+def matmul_code(lib, a_shape, b_shape, c_shape, a_dt=F, b_dt=F, c_dt=F, c_scale=-1.0, bias=0, ta=0, tb=0):
+    a, b, c = B.tensor_nd(a_dt, a_shape), B.tensor_nd(b_dt, b_shape), B.tensor_nd(c_dt, c_shape)
+    buf = [np.zeros(max(int(np.prod(s)), 1) * 4 + 4096, np.uint8) for s in (a_shape, b_shape, c_shape)]
+    pa, pb, pc = (C.c_void_p(x.ctypes.data) for x in buf)
+    tmp, bvec = np.zeros(1 << 22, np.uint8), np.zeros(max(bias, 1), np.float32)
+    s = C.c_float(c_scale)
+    bd = B.tensor1d(F, bias)
+    r = lib.matmul_cuda_b200(C.byref(a), ta, pa, 5.0, C.byref(b), tb, pb, 5.0, C.byref(bd) if bias else None,
+                             C.c_void_p(bvec.ctypes.data) if bias else None, tmp.size, C.c_void_p(tmp.ctypes.data), C.byref(c), pc, C.byref(s))
+    return r, s.value
+
+
+@pytest.mark.parametrize("m", [1, 4])
+@pytest.mark.parametrize("a_dt,b_dt", [(F, F), (None, None)])
+@pytest.mark.parametrize("c_dt,c_scale,bias", [(F, -1.0, 0), (F, -1.0, 8), (U, -1.0, 0), (U, 3.0, 0)])
+def test_matmul_without_products(m, a_dt, b_dt, c_dt, c_scale, bias):
+    """an empty batch is a success that launches nothing and leaves no error behind for the thread's next call"""
+    lib = fake_gpu.load()
+    a_dt, b_dt = a_dt or (I if m == 1 else U), b_dt or (U if m == 1 else I)
+    assert matmul_code(lib, (0, m, 16), (0, 16, 8), (0, m, 8), a_dt, b_dt, c_dt, c_scale, bias) == (B.SUCCESS, c_scale)
+    assert lib.fake_last_error() == 0 and fake_gpu.launches(lib) == []
+
+
+@pytest.mark.parametrize("m", [1, 4])
+@pytest.mark.parametrize("a,b", [((0,), (1,)), ((1,), (0,)), ((0,), (0,)), ((3, 0), (3, 1))])
+def test_matmul_products_without_operands(m, a, b):
+    """C has products but an operand has none: there is nothing to read"""
+    lib = fake_gpu.load()
+    c = tuple(max(x, y) for x, y in zip(a, b)) if a != b else (2,)
+    assert matmul_code(lib, a + (m, 16), b + (16, 8), c + (m, 8))[0] == B.NOT_MATCH
+    assert lib.fake_last_error() == 0 and fake_gpu.launches(lib) == []
