@@ -89,10 +89,10 @@ cudaError_t launch_absmax(DeviceCtx *c, const T *x, uint64_t n, const MaxMail &m
     return launch((uint32_t)(blocks < cap ? blocks : cap), MAX_TPB, st, absmax_kernel<T>, x, n, m);
 }
 
-// 127 / absmax on the device (quantize.cpp:63-67), for pipelines that never leave the stream
-__global__ void finalize_scale_kernel(const unsigned *bits, float *scale)
+// the absmax at *scale becomes 127 / absmax (quantize.cpp:63-67), for pipelines that never leave the stream
+__global__ void finalize_scale_kernel(float *scale)
 {
-    const float mx = __uint_as_float(*bits);
+    const float mx = *scale;
     *scale = (mx == 0.f) ? 1.0f : __fdiv_rn(127.0f, mx);
 }
 
@@ -451,14 +451,13 @@ EE bolt_b200_absmax_scale_f32(const F32 *data, uint64_t n, F32 *d_scale)
         return NULL_POINTER;
     }
     cudaStream_t st = tls().stream;
-    unsigned *bits = c->d_scratch_u + 2;
+    // the maximum is found in the caller's own word: a shared one would mix calls on several streams
+    unsigned *bits = reinterpret_cast<unsigned *>(d_scale);
     B200_CUDA(cudaMemsetAsync(bits, 0, 4, st));
     if (n > 0) {
         B200_CUDA(launch_absmax(c, data, n, MaxMail{bits, nullptr, nullptr, 0}, st));
     }
-    finalize_scale_kernel<<<1, 1, 0, st>>>(bits, d_scale);
-    count_launch();
-    B200_CUDA(cudaGetLastError());
+    B200_CUDA(launch(1, 1, st, finalize_scale_kernel, d_scale));
     return SUCCESS;
 }
 

@@ -28,6 +28,7 @@ def load():
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
         lib.fake_launch_name.restype = C.c_char_p
+        lib.fake_max_words.restype = C.c_void_p
         lib.bolt_b200_set_pointer_mode(1)
         _lib = lib
     _lib.fake_refuse_programmatic(0)

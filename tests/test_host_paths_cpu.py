@@ -44,3 +44,14 @@ def test_matmul_products_without_operands(m, a, b):
     c = tuple(max(x, y) for x, y in zip(a, b)) if a != b else (2,)
     assert matmul_code(lib, a + (m, 16), b + (16, 8), c + (m, 8))[0] == B.NOT_MATCH
     assert lib.fake_last_error() == 0 and fake_gpu.launches(lib) == []
+
+
+def test_device_scale_counts_in_the_callers_memory():
+    """calls on several streams run at the same time: what one counts in, no other may"""
+    lib = fake_gpu.load()
+    x, scales = np.zeros(64, np.float32), np.zeros(2, np.float32)
+    words = []
+    for i in range(2):
+        assert lib.bolt_b200_absmax_scale_f32(C.c_void_p(x.ctypes.data), x.size, C.c_void_p(scales.ctypes.data + 4 * i)) == B.SUCCESS
+        words.append(lib.fake_max_words())
+    assert words[0] != words[1]

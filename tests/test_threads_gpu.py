@@ -11,6 +11,7 @@ import pytest
 sys.path.insert(0, os.path.dirname(__file__))
 import bolt_b200 as B  # noqa: E402
 from bolt_b200 import synth  # noqa: E402
+from test_stack_gpu import make_stack  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 THREADS, ROUNDS = 70, 12     # more threads than the pool has entries
@@ -62,6 +63,43 @@ def test_threads_and_streams_do_not_mix():
             B.CHECK_STATUS(B.lib().bolt_b200_set_stream(None))
 
     ts = [threading.Thread(target=body, args=(t,)) for t in range(THREADS)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad, bad[:10]
+
+
+def test_stacks_on_streams_do_not_mix():
+    """The device-resident input scale: stacks whose inputs differ by orders of magnitude, each on a stream of its own."""
+    import torch
+
+    stacks, expect = [], []
+    for t in range(4):
+        st, _ = make_stack(48, [512, 256, 64], False, 300 + 10 * t)
+        st.x_dev.copy_(torch.from_numpy((synth.normal(400 + t, (48 * 512,)) * np.float32(10.0 ** (2 * t - 3))).astype(np.float32)))
+        st.calibrate()
+        st.step()
+        B.CHECK_STATUS(B.lib().bolt_b200_synchronize(), "synchronize")
+        stacks.append(st)
+        expect.append((st.d_scale[:1].clone(), st.out_dev.clone()))
+    torch.cuda.synchronize()
+    bad = []
+
+    def body(t):
+        st, (scale, out) = stacks[t], expect[t]
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            B.CHECK_STATUS(B.lib().bolt_b200_set_stream(C.c_void_p(stream.cuda_stream)))
+            for i in range(200):
+                st.step()
+                if i % 10 == 9:
+                    stream.synchronize()
+                    if not (torch.equal(st.d_scale[:1], scale) and torch.equal(st.out_dev, out)):
+                        bad.append((t, i))
+            B.CHECK_STATUS(B.lib().bolt_b200_set_stream(None))
+
+    ts = [threading.Thread(target=body, args=(t,)) for t in range(len(stacks))]
     for t in ts:
         t.start()
     for t in ts:
