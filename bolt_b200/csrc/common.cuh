@@ -122,8 +122,7 @@ struct DeviceCtx {
     int sm_count = 148;
     int *d_status = nullptr;      // device-side error word
     void *d_scatter_maps = nullptr;  // 8 tensor maps of a scatter GEMM (allocated on first use)
-    float *d_scratch = nullptr;   // small device scratch for reductions (absmax etc.)
-    unsigned *d_scratch_u = nullptr;
+    unsigned *d_scratch_u = nullptr;   // the words of the MaxMails
     std::mutex mu;       // guards the staging workspace (one staged call at a time)
     std::mutex twin_mu;  // guards twins
     std::mutex mail_mu;     // guards mail_free and mails

@@ -69,16 +69,17 @@ DeviceCtx *ctx()
         if (cudaGetDeviceProperties(&prop, dev) == cudaSuccess) {
             c->sm_count = prop.multiProcessorCount;
         }
-        if (cudaMalloc(&c->d_status, 256) != cudaSuccess ||
-            cudaMemset(c->d_status, 0, 256) != cudaSuccess ||
-            cudaMalloc(&c->d_scratch, 4096) != cudaSuccess) {
-            delete c;
-            return nullptr;
-        }
-        c->d_scratch_u = reinterpret_cast<unsigned *>(c->d_scratch);
-        cudaMemset(c->d_scratch, 0, 4096);
+        // Kernels count in this memory from their first launch on, on any stream: it has to be clear before that, and
+        // cudaMemset neither waits nor is ordered against streams that do not block on the legacy one.
         void *h = nullptr, *hd = nullptr;
-        if (cudaHostAlloc(&h, 64 * MAX_MAILS, cudaHostAllocMapped) != cudaSuccess || cudaHostGetDevicePointer(&hd, h, 0) != cudaSuccess) {
+        if (cudaMalloc(&c->d_status, 256) != cudaSuccess || cudaMemset(c->d_status, 0, 256) != cudaSuccess ||
+            cudaMalloc(&c->d_scratch_u, 4096) != cudaSuccess || cudaMemset(c->d_scratch_u, 0, 4096) != cudaSuccess ||
+            cudaStreamSynchronize(nullptr) != cudaSuccess ||
+            cudaHostAlloc(&h, 64 * MAX_MAILS, cudaHostAllocMapped) != cudaSuccess || cudaHostGetDevicePointer(&hd, h, 0) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(c->d_status);
+            cudaFree(c->d_scratch_u);
+            cudaFreeHost(h);
             delete c;
             return nullptr;
         }

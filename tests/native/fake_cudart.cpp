@@ -31,7 +31,7 @@ struct Names {
 };
 std::vector<std::string> launched;
 void *max_words = nullptr;   // where the last absmax_kernel was to count
-bool refuse_programmatic = false;
+bool refuse_programmatic = false, refuse_fills = false;
 struct Call {
     dim3 grid, block;
     size_t smem;
@@ -106,6 +106,10 @@ void fake_refuse_programmatic(int on)
 {
     refuse_programmatic = on != 0;
 }
+void fake_refuse_fills(int on)
+{
+    refuse_fills = on != 0;
+}
 void fake_set_last_error(int e)
 {
     last = (cudaError_t)e;
@@ -131,6 +135,10 @@ cudaError_t cudaFree(void *p)
     std::free(p);
     return cudaSuccess;
 }
+cudaError_t cudaFreeHost(void *p)
+{
+    return cudaFree(p);
+}
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned)
 {
     return cudaMalloc(p, n);
@@ -142,6 +150,9 @@ cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned)
 }
 cudaError_t cudaMemset(void *p, int v, size_t n)
 {
+    if (refuse_fills && n > 1024) {   // (the words of the maxima, not the smaller status)
+        return fail(cudaErrorNotSupported);
+    }
     fills.push_back(Fill{p, v, n});
     return cudaSuccess;
 }

@@ -55,3 +55,24 @@ def test_device_scale_counts_in_the_callers_memory():
         assert lib.bolt_b200_absmax_scale_f32(C.c_void_p(x.ctypes.data), x.size, C.c_void_p(scales.ctypes.data + 4 * i)) == B.SUCCESS
         words.append(lib.fake_max_words())
     assert words[0] != words[1]
+
+
+def test_the_words_of_reported_maxima_are_cleared_before_the_first_call_uses_them():
+    """cudaMemset returns before the memory is set and streams that do not block on the legacy one run past it"""
+    lib = fake_gpu.fresh()
+    x, q, s = np.zeros(64, np.float32), np.zeros(64, np.uint8), (C.c_float * 1)(-1.0)
+    d, o = B.tensor1d(F, 64), B.tensor1d(U, 64)
+    assert lib.quantize_cuda_b200(C.byref(d), C.c_void_p(x.ctypes.data), C.byref(o), C.c_void_p(q.ctypes.data), s, 0) == B.SUCCESS
+    assert lib.fake_unordered_fills() == 0
+    assert (C.c_uint * 2).from_address(lib.fake_max_words())[:] == [0, 0]
+
+
+def test_a_device_whose_words_cannot_be_cleared_is_refused():
+    lib = fake_gpu.fresh()
+    lib.fake_refuse_fills(1)
+    x, q, s = np.zeros(64, np.float32), np.zeros(64, np.uint8), (C.c_float * 1)(-1.0)
+    d, o = B.tensor1d(F, 64), B.tensor1d(U, 64)
+    call = lambda: lib.quantize_cuda_b200(C.byref(d), C.c_void_p(x.ctypes.data), C.byref(o), C.c_void_p(q.ctypes.data), s, 0)
+    assert call() == B.UNKNOWN and fake_gpu.launches(lib) == []
+    lib.fake_refuse_fills(0)
+    assert call() == B.SUCCESS
