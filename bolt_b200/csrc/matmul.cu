@@ -2,8 +2,8 @@
 // CUDA_B200: both operands may arrive as fp32 and are quantized per call (dynamic scale 127 / absmax, or the
 // scale the tensor carries), and the result is written as fp32 (accumulator / (scaleA * scaleB)) or requantized
 // to u8.  All products of a call run in one launch that quantizes its operands while it loads them
-// (launch_matmul_batch); a single large product, and a result of one column, take the quantize / pack / multiply
-// kernels one after the other.
+// (launch_matmul_batch); a single large product, a result of one column and one that lies over its operands take the
+// quantize / pack / multiply kernels one after the other.
 //
 // The x86 convention applies (matmul.cpp:373-398): u8 activations with zero point 128 times s8, except
 // when the result is a vector, where A becomes s8 and B u8.  Leading (batch) dimensions broadcast as in
@@ -194,6 +194,12 @@ bool one_launch(const Plan &p)
     return N != 1 && M * N <= (1ull << 30) / K;
 }
 
+bool overlap(const void *a, size_t na, const void *b, size_t nb)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+}
+
 // the scratch of the batched kernel: an operand's partial maxima lie where its quantized copy would
 MatmulOperand batch_operand(const void *data, const TensorDesc &d, bool f32, int transposed, F32 scale, uint64_t loops, uint64_t loopsC, char *scratch)
 {
@@ -358,7 +364,10 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
         return NOT_MATCH;
     }
 
-    const bool fused = one_launch(p);
+    // The batched kernel reads A and B while it writes C.  A result over its own operands (fp32 in, fp32 out) needs the
+    // quantized copies of the other way.
+    const bool in_place = !p.stageC && (overlap(C, c_bytes, A, (size_t)nA * bytes_of(p.a.dt)) || overlap(C, c_bytes, B, (size_t)nB * bytes_of(p.b.dt)));
+    const bool fused = !in_place && one_launch(p);
     // (the tmp bytes count 1 KiB more than what is laid out in it)
     char *t = fused ? reinterpret_cast<char *>(B200_ALIGN(reinterpret_cast<uintptr_t>(tmp), 16)) : reinterpret_cast<char *>(tmp);
     char *slotsA = t, *slotsB = t + (p.quantA ? B200_ALIGN(nA, 256) : 0);
@@ -441,7 +450,11 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
         const char *pb = reinterpret_cast<const char *>(B) + ib * b2;
         char *pc = reinterpret_cast<char *>(prod) + ic * c2;
         EE ret;
-        if (p.b.dims[1 - p.kDimB] == 1) {
+        if (p.a.dims[1 - p.kDimA] == 1) {
+            ret = b200_matrix_vector_multiply(
+                desc2d(p.qb, p.dfB == DF_TRANSPOSE ? DF_NORMAL : DF_TRANSPOSE, p.b.dims[1], p.b.dims[0]), pb,
+                desc1d(p.qa, p.a.dims[p.kDimA]), pa, p.mmm_bytes, t, desc1d(p.qc, p.c.dims[0]), pc, scalePtr, CUDA_B200);
+        } else if (p.b.dims[1 - p.kDimB] == 1) {
             ret = b200_matrix_vector_multiply(desc2d(p.qa, p.dfA, p.a.dims[1], p.a.dims[0]), pa,
                 desc1d(p.qb, p.b.dims[p.kDimB]), pb, p.mmm_bytes, t, desc1d(p.qc, p.c.dims[1]), pc, scalePtr, CUDA_B200);
         } else {

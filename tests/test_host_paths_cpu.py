@@ -13,10 +13,13 @@ import fake_gpu  # noqa: E402
 F, U, I = B.DT_F32, B.DT_U8_Q, B.DT_I8
 
 
-def matmul_code(lib, a_shape, b_shape, c_shape, a_dt=F, b_dt=F, c_dt=F, c_scale=-1.0, bias=0, ta=0, tb=0):
+def matmul_code(lib, a_shape, b_shape, c_shape, a_dt=F, b_dt=F, c_dt=F, c_scale=-1.0, bias=0, ta=0, tb=0, over=None, shift=0):
+    """over: C lies over A (0) or B (1), `shift` bytes behind its start"""
     a, b, c = B.tensor_nd(a_dt, a_shape), B.tensor_nd(b_dt, b_shape), B.tensor_nd(c_dt, c_shape)
     buf = [np.zeros(max(int(np.prod(s)), 1) * 4 + 4096, np.uint8) for s in (a_shape, b_shape, c_shape)]
     pa, pb, pc = (C.c_void_p(x.ctypes.data) for x in buf)
+    if over is not None:
+        pc = C.c_void_p(buf[over].ctypes.data + shift)
     tmp, bvec = np.zeros(1 << 22, np.uint8), np.zeros(max(bias, 1), np.float32)
     s = C.c_float(c_scale)
     bd = B.tensor1d(F, bias)
@@ -76,3 +79,22 @@ def test_a_device_whose_words_cannot_be_cleared_is_refused():
     assert call() == B.UNKNOWN and fake_gpu.launches(lib) == []
     lib.fake_refuse_fills(0)
     assert call() == B.SUCCESS
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 24, 24), (24, 24, 24), (40, 16, 32)])
+@pytest.mark.parametrize("over", [0, 1])
+def test_matmul_over_its_operands_copies_them_first(m, n, k, over):
+    lib = fake_gpu.load()
+    size = (m * k, k * n)[over] * 4
+    args = (lib, (1, m, k), (1, k, n), (1, m, n))
+    batched = lambda: any("absmax_pair_kernel" in x for x in fake_gpu.launches(lib))
+    for shift in (0, size - 4):
+        lib.fake_forget_launches()
+        assert matmul_code(*args, over=over, shift=shift)[0] == B.SUCCESS
+        assert not batched()
+    lib.fake_forget_launches()
+    assert matmul_code(*args, over=over, shift=size)[0] == B.SUCCESS      # right behind: no overlap
+    assert batched()
+    lib.fake_forget_launches()
+    assert matmul_code(*args, c_dt=U, over=over)[0] == B.SUCCESS          # goes through the scratch anyway
+    assert batched()

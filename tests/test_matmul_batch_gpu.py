@@ -12,6 +12,7 @@ import oracle as O  # noqa: E402
 import bolt_b200 as B  # noqa: E402
 from bolt_b200 import synth  # noqa: E402
 from test_matmul_gpu import matmul_gpu  # noqa: E402
+from util import dev_zeros, dptr, to_dev, to_host  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 F, U, I = B.DT_F32, B.DT_U8_Q, B.DT_I8
@@ -56,6 +57,21 @@ def test_broadcast_bias_and_scale_edges():
     check((a, F, -1.0, 0, b, F, -1.0, 0, synth.normal(8, (40,)), F, -1.0))
     check((a, F, 500.0, 0, b, F, -1.0, 0, None, F, -1.0))              # a given scale above the dynamic one wins
     check((np.zeros_like(a), F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0))
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 640, 640), (128, 128, 128), (300, 96, 96)])
+@pytest.mark.parametrize("over", [0, 1])
+def test_result_over_its_operands(m, k, n, over):
+    a, b = synth.normal(21, (3, m, k)), synth.normal(22, (3, k, n))
+    d_a, d_b = to_dev(a), to_dev(b)
+    ad, bd, cd = B.tensor_nd(F, a.shape), B.tensor_nd(F, b.shape), B.tensor_nd(F, (3, m, n))
+    tmp_bytes = B.matmul_infer_forward_tmp_bytes(ad, 0, bd, 0, cd, -1.0)
+    d_c = (d_a, d_b)[over]
+    if d_c.numel() < 3 * m * n * 4:
+        pytest.skip("C is larger than the operand")
+    B.matmul(ad, 0, dptr(d_a), -1.0, bd, 0, dptr(d_b), -1.0, None, None, tmp_bytes, dptr(dev_zeros(tmp_bytes)), cd, dptr(d_c), -1.0)
+    ref, _ = O.port_matmul(a, F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0)
+    assert to_host(d_c, np.float32, 3 * m * n).tobytes() == np.ascontiguousarray(ref).tobytes()
 
 
 def test_single_large_product_goes_one_by_one():
