@@ -13,7 +13,7 @@
 // In a chain of layers (bolt_b200_gemm_u8s8_chain) the kernel of layer i+1 starts while layer i runs and has its weight
 // fragments, offsets and factors in registers when layer i's result arrives.  That is safe because this kernel lets
 // its successor start only after its own wait: whoever starts then knows that everything before layer i is complete,
-// and the chain's weights are constant.
+// and the chain's weights are constant.  A layer with its input scale in device memory waits first.
 #include <cstdlib>
 
 #include "common.cuh"
@@ -235,7 +235,8 @@ EE launch_gemm_skinny(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, cons
         const char *e = getenv("BOLT_B200_NO_PDL");
         return !(e != nullptr && e[0] != '\0' && e[0] != '0');
     }();
-    p.preload = preload && pdl ? 1 : 0;
+    // (d_sA is no constant of the chain: an earlier layer may just be writing it)
+    p.preload = preload && pdl && ep.sA_dev == nullptr ? 1 : 0;
     // 8 columns per CTA, 16 where that makes more CTAs than SMs
     const bool wide = (N + 7) / 8 > (uint32_t)c->sm_count;
     cudaError_t e;

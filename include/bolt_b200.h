@@ -287,9 +287,9 @@ typedef struct {
 } bolt_b200_gemm_epilogue;
 EE bolt_b200_gemm_u8s8_ex(U32 N, U32 M, U32 K, const void *A, const void *packedB,
     const I32 *offsetC, void *C, const bolt_b200_gemm_epilogue *ep);
-/* Several of them, one after the other in one call: the layers of a network.  A may be an earlier call's C; packedB,
- * offsetC, col_scale and col_factor have to stay as they are for the whole chain (a layer's may be read while the
- * layer before it still runs). */
+/* Several of them, one after the other in one call: the layers of a network.  A, row_scale and d_sA may be an earlier
+ * call's C; packedB, offsetC, col_scale and col_factor have to stay as they are for the whole chain (a layer's may be
+ * read while the layer before it still runs). */
 typedef struct {
     U32 N, M, K;
     const void *A;

@@ -73,6 +73,30 @@ def test_chain_equals_single_calls(m):
     assert results[0][0] == np.where(r < 0, 255, np.minimum(r, 255)).astype(np.uint8).tobytes()
 
 
+@pytest.mark.parametrize("m", [1, 16])
+def test_input_scale_from_an_earlier_call(m):
+    """d_sA may be what an earlier call of the chain writes.  That call has a long K, so that a later one that
+    did not wait for it would read what the buffer held before."""
+    lib, k0, k, n = B.lib(), 16384, 256, 512
+    (_, _, w0, r0, _), (_, _, w1, r1, _), (_, _, w2, r2, col) = chain_layers(m, [k0, 8], 900) + chain_layers(m, [k, n], 910) + chain_layers(m, [k, n], 920)
+    x0, x = synth.u8(31, (m, k0)), synth.u8(32, (m, k))
+    d_x0, d_x, d_s, d_mid, d_out = to_dev(x0), to_dev(x), dev_zeros(m * 8 * 4), dev_zeros(m * n * 4), dev_zeros(m * n * 4)
+    calls = (B.GemmCall * 3)()
+    for c, (M, K, N, a, w, r, out) in zip(calls, ((m, k, n, d_x, w1, r1, d_mid), (m, k0, 8, d_x0, w0, r0, d_s), (m, k, n, d_x, w2, r2, d_out))):
+        c.N, c.M, c.K, c.A, c.packedB, c.offsetC, c.C = N, M, K, a.data_ptr(), w.data_ptr(), w.data_ptr() + r, out.data_ptr()
+        c.epilogue.out_dt, c.epilogue.out_scale, c.epilogue.sA, c.epilogue.sB = B.DT_F32, 1.0, 1.0, 1.0
+    calls[2].epilogue.d_sA, calls[2].epilogue.col_scale = d_s.data_ptr(), col.data_ptr()
+    acc0 = O.port_gemm(x0, synth.s8(900, (k0, 8)), O.port_offsetc(synth.s8(900, (k0, 8))))
+    acc = O.port_gemm(x, synth.s8(920, (k, n)), O.port_offsetc(synth.s8(920, (k, n))))
+    fac = (np.float32(1) / (np.float32(acc0[0, 0]) * to_host(col, np.float32, n))).astype(np.float32)
+    ref = (acc.astype(np.float32) * fac[None, :]).astype(np.float32).tobytes()
+    for _ in range(20):
+        d_s.fill_(0x3F)
+        B.CHECK_STATUS(lib.bolt_b200_gemm_u8s8_chain(calls, 3))
+        B.CHECK_STATUS(lib.bolt_b200_synchronize(), "synchronize")
+        assert to_host(d_out, np.float32, m * n).tobytes() == ref
+
+
 def test_chain_errors():
     lib = B.lib()
     assert lib.bolt_b200_gemm_u8s8_chain(None, 0) == B.SUCCESS
