@@ -208,6 +208,39 @@ __device__ __forceinline__ int magnitude(int x)
 }
 #endif
 
+#ifdef __CUDACC__
+// Programmatic stream serialization (a kernel's set-up runs beside the end of the kernel in front of it): on unless
+// BOLT_B200_NO_PDL is set in the environment, or the runtime has refused it where it took the plain launch.
+bool programmatic_launches();
+void refuse_programmatic_launches();
+template <typename... P, typename... A>
+cudaError_t launch_programmatic(const cudaLaunchConfig_t &plain, void (*kernel)(P...), const A &...args)
+{
+    if (!programmatic_launches()) {
+        return cudaLaunchKernelEx(&plain, kernel, args...);
+    }
+    cudaLaunchAttribute at[2];
+    unsigned n = 0;
+    for (; n < plain.numAttrs && n < 1; ++n) {
+        at[n] = plain.attrs[n];
+    }
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = plain;
+    cfg.attrs = at;
+    cfg.numAttrs = n + 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess && !capturing(plain.stream)) {
+        cudaGetLastError();
+        e = cudaLaunchKernelEx(&plain, kernel, args...);
+        if (e == cudaSuccess) {
+            refuse_programmatic_launches();
+        }
+    }
+    return e;
+}
+#endif
+
 // cudaFuncAttributeMaxDynamicSharedMemorySize for every kernel of a family, once per device
 // (the calling thread's device must be current, which ctx() guarantees)
 EE raise_smem_limit(DeviceCtx *c, KernelFamily f, const void *const *kernels, int n, size_t bytes);

@@ -1,4 +1,5 @@
 // context.cu -- per-device state, the staging of host pointers, and the runtime entry points.
+#include <cstdlib>
 #include <cstring>
 
 #include "common.cuh"
@@ -101,6 +102,25 @@ DeviceCtx *ctx()
         }
     }
     return g_ctx[dev];
+}
+
+namespace {
+std::atomic<bool> &programmatic()
+{
+    static std::atomic<bool> on{[] {
+        const char *e = getenv("BOLT_B200_NO_PDL");
+        return !(e != nullptr && e[0] != '\0' && e[0] != '0');
+    }()};
+    return on;
+}
+}  // namespace
+bool programmatic_launches()
+{
+    return programmatic().load(std::memory_order_relaxed);
+}
+void refuse_programmatic_launches()
+{
+    programmatic().store(false, std::memory_order_relaxed);
 }
 
 EE raise_smem_limit(DeviceCtx *c, KernelFamily f, const void *const *kernels, int n, size_t bytes)

@@ -894,40 +894,15 @@ struct ConvLaunch {
     MaxMail mail;
 };
 
-// Launch with programmatic stream serialization (the kernel's set-up overlaps the tail of the previous kernel);
-// if the attribute is refused outside a stream capture, launch without it from then on.
-std::atomic<int> g_conv_pdl{-1};
 template <int KIND, int NB>
 cudaError_t launch_conv_kernel(uint32_t grid, cudaStream_t st, const CUtensorMap &mx, const CUtensorMap &mw, const ConvParams &p)
 {
-    int pdl = g_conv_pdl.load(std::memory_order_relaxed);
-    if (pdl < 0) {
-        const char *e = getenv("BOLT_B200_NO_PDL");
-        pdl = (e != nullptr && e[0] != '\0' && e[0] != '0') ? 0 : 1;
-        g_conv_pdl.store(pdl, std::memory_order_relaxed);
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(Cfg<NB>::THREADS);
     cfg.dynamicSmemBytes = smem_bytes<NB>();
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, conv_u8s8_tcgen05_kernel<KIND, NB>, mx, mw, p);
-    if (e != cudaSuccess && pdl) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(st, &cap);
-        if (cap == cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            g_conv_pdl.store(0, std::memory_order_relaxed);
-            cfg.numAttrs = 0;
-            e = cudaLaunchKernelEx(&cfg, conv_u8s8_tcgen05_kernel<KIND, NB>, mx, mw, p);
-        }
-    }
-    return e;
+    return launch_programmatic(cfg, conv_u8s8_tcgen05_kernel<KIND, NB>, mx, mw, p);
 }
 
 // run the implicit-GEMM kernel (all pointers device)

@@ -15,7 +15,6 @@
 #include <cuda.h>
 
 #include <algorithm>
-#include <cstdlib>
 #include <cstring>
 
 #include "common.cuh"
@@ -877,25 +876,24 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
 
 namespace {
 
-template <int LA, int LB>
-cudaError_t launch_batch(uint32_t grid, const GatherParams &p, const BatchParams &bp, const cudaLaunchConfig_t &base)
+// its set-up runs beside the reduction in front of it, if there is one
+template <typename... P, typename... A>
+cudaError_t launch_behind(bool reduction, const cudaLaunchConfig_t &cfg, void (*kernel)(P...), const A &...args)
 {
-    cudaLaunchConfig_t cfg = base;
-    cfg.gridDim = dim3(grid);
-    return cudaLaunchKernelEx(&cfg, gemm_gather_kernel<LA, LB, true>, p, bp);
+    return reduction ? launch_programmatic(cfg, kernel, args...) : cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 template <int LA>
-cudaError_t launch_batch_b(int lb, uint32_t grid, const GatherParams &p, const BatchParams &bp, const cudaLaunchConfig_t &base)
+cudaError_t launch_batch(int lb, bool reduction, const cudaLaunchConfig_t &cfg, const GatherParams &p, const BatchParams &bp)
 {
     switch (lb) {
         case ROWS_K:
-            return launch_batch<LA, ROWS_K>(grid, p, bp, base);
+            return launch_behind(reduction, cfg, gemm_gather_kernel<LA, ROWS_K, true>, p, bp);
         case K_ROWS:
-            return launch_batch<LA, K_ROWS>(grid, p, bp, base);
+            return launch_behind(reduction, cfg, gemm_gather_kernel<LA, K_ROWS, true>, p, bp);
         case F32_ROWS_K:
-            return launch_batch<LA, F32_ROWS_K>(grid, p, bp, base);
+            return launch_behind(reduction, cfg, gemm_gather_kernel<LA, F32_ROWS_K, true>, p, bp);
         default:
-            return launch_batch<LA, F32_K_ROWS>(grid, p, bp, base);
+            return launch_behind(reduction, cfg, gemm_gather_kernel<LA, F32_K_ROWS, true>, p, bp);
     }
 }
 template <int LA>
@@ -905,14 +903,6 @@ void batch_kernels(const void **ks)
     ks[1] = (const void *)gemm_gather_kernel<LA, K_ROWS, true>;
     ks[2] = (const void *)gemm_gather_kernel<LA, F32_ROWS_K, true>;
     ks[3] = (const void *)gemm_gather_kernel<LA, F32_K_ROWS, true>;
-}
-bool programmatic_launch()
-{
-    static const bool on = [] {
-        const char *e = getenv("BOLT_B200_NO_PDL");
-        return !(e != nullptr && e[0] != '\0' && e[0] != '0');
-    }();
-    return on;
 }
 Operand operand(const MatmulOperand &o, uint32_t rows, uint32_t K, bool rows_contiguous)
 {
@@ -1024,11 +1014,7 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(THREADS);
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = (ga + gb) && programmatic_launch() ? 1 : 0;   // its set-up runs beside the reduction
+    const bool reduction = ga + gb != 0;
     const int la = (mb.a.f32 ? 2 : 0) + (mb.a.transposed ? 1 : 0);
     const int lb = (mb.b.f32 ? 2 : 0) + (mb.b.transposed ? 0 : 1);
     cudaError_t e;
@@ -1037,10 +1023,10 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
         cfg.gridDim = dim3((uint32_t)std::min<uint64_t>(work, 8 * (uint64_t)c->sm_count));
         cfg.dynamicSmemBytes = mvm_smem;
         const int af = mb.a.f32 ? 1 : 0;
-        e = lb == ROWS_K ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<ROWS_K>, p, bp, af)
-            : lb == K_ROWS ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<K_ROWS>, p, bp, af)
-            : lb == F32_ROWS_K ? cudaLaunchKernelEx(&cfg, mvm_batch_kernel<F32_ROWS_K>, p, bp, af)
-                               : cudaLaunchKernelEx(&cfg, mvm_batch_kernel<F32_K_ROWS>, p, bp, af);
+        e = lb == ROWS_K ? launch_behind(reduction, cfg, mvm_batch_kernel<ROWS_K>, p, bp, af)
+            : lb == K_ROWS ? launch_behind(reduction, cfg, mvm_batch_kernel<K_ROWS>, p, bp, af)
+            : lb == F32_ROWS_K ? launch_behind(reduction, cfg, mvm_batch_kernel<F32_ROWS_K>, p, bp, af)
+                               : launch_behind(reduction, cfg, mvm_batch_kernel<F32_K_ROWS>, p, bp, af);
     } else {
         p.tiles_m = (mb.M + BLOCK_M - 1) / BLOCK_M;
         p.block_n = pick_bn((uint64_t)p.tiles_m * mb.batches, mb.N, c->sm_count);
@@ -1048,11 +1034,11 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
         p.tmem_cols = p.block_n > 64 ? 128u : p.block_n;
         cfg.dynamicSmemBytes = SMEM_BYTES;
         const uint64_t tiles = (uint64_t)p.tiles_m * p.tiles_n * mb.batches;
-        const uint32_t grid = (uint32_t)std::min<uint64_t>(tiles, (uint64_t)c->sm_count * ctas_per_sm(la, lb));
-        e = la == ROWS_K ? launch_batch_b<ROWS_K>(lb, grid, p, bp, cfg)
-            : la == K_ROWS ? launch_batch_b<K_ROWS>(lb, grid, p, bp, cfg)
-            : la == F32_ROWS_K ? launch_batch_b<F32_ROWS_K>(lb, grid, p, bp, cfg)
-                               : launch_batch_b<F32_K_ROWS>(lb, grid, p, bp, cfg);
+        cfg.gridDim = dim3((uint32_t)std::min<uint64_t>(tiles, (uint64_t)c->sm_count * ctas_per_sm(la, lb)));
+        e = la == ROWS_K ? launch_batch<ROWS_K>(lb, reduction, cfg, p, bp)
+            : la == K_ROWS ? launch_batch<K_ROWS>(lb, reduction, cfg, p, bp)
+            : la == F32_ROWS_K ? launch_batch<F32_ROWS_K>(lb, reduction, cfg, p, bp)
+                               : launch_batch<F32_K_ROWS>(lb, reduction, cfg, p, bp);
         tls().last_gemm_tc = 1;
     }
     count_launch();

@@ -14,8 +14,6 @@
 // fragments, offsets and factors in registers when layer i's result arrives.  That is safe because this kernel lets
 // its successor start only after its own wait: whoever starts then knows that everything before layer i is complete,
 // and the chain's weights are constant.  A layer with its input scale in device memory waits first.
-#include <cstdlib>
-
 #include "common.cuh"
 #include "epilogue.cuh"
 
@@ -174,7 +172,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, MT == 1 ? 2 : 1) gemm_skinny_k
 }
 
 template <int MT, int NT, int UNITS>
-cudaError_t launch(const SkinnyParams &p, bool pdl, cudaStream_t st)
+cudaError_t launch(const SkinnyParams &p, cudaStream_t st)
 {
     const uint32_t units = (p.K + 63) / 64;
     uint32_t warps = (units + UNITS - 1) / UNITS;   // one batch of loads per warp, if sixteen warps can do it
@@ -184,12 +182,7 @@ cudaError_t launch(const SkinnyParams &p, bool pdl, cudaStream_t st)
     cfg.blockDim = dim3(warps * 32);
     cfg.dynamicSmemBytes = warps * NT * MT * 128 * sizeof(int);
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<MT, NT, UNITS>, p);
+    return launch_programmatic(cfg, gemm_skinny_kernel<MT, NT, UNITS>, p);
 }
 
 }  // namespace
@@ -231,21 +224,17 @@ EE launch_gemm_skinny(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, cons
     p.ep = ep;
     const uintptr_t c_align = ep.out_kind == 2 ? 4 : 16;
     p.vec_c = (N % 4 == 0) && (reinterpret_cast<uintptr_t>(C) % c_align == 0);
-    static const bool pdl = [] {
-        const char *e = getenv("BOLT_B200_NO_PDL");
-        return !(e != nullptr && e[0] != '\0' && e[0] != '0');
-    }();
     // (d_sA is no constant of the chain: an earlier layer may just be writing it)
-    p.preload = preload && pdl && ep.sA_dev == nullptr ? 1 : 0;
+    p.preload = preload && ep.sA_dev == nullptr ? 1 : 0;
     // 8 columns per CTA, 16 where that makes more CTAs than SMs
     const bool wide = (N + 7) / 8 > (uint32_t)c->sm_count;
     cudaError_t e;
     if (M <= 16) {
-        e = wide ? launch<1, 2, 2>(p, pdl, st) : launch<1, 1, 3>(p, pdl, st);
+        e = wide ? launch<1, 2, 2>(p, st) : launch<1, 1, 3>(p, st);
     } else if (M <= 32) {
-        e = wide ? launch<2, 2, 2>(p, pdl, st) : launch<2, 1, 3>(p, pdl, st);
+        e = wide ? launch<2, 2, 2>(p, st) : launch<2, 1, 3>(p, st);
     } else {
-        e = launch<4, 1, 2>(p, pdl, st);   // (narrow: gemm_skinny_preferred)
+        e = launch<4, 1, 2>(p, st);   // (narrow: gemm_skinny_preferred)
     }
     count_launch();
     B200_CUDA(e);

@@ -1000,55 +1000,24 @@ bool gemm_tcgen05_eligible(uint32_t M, uint32_t N, uint32_t K, const void *A, co
 
 namespace {
 
-// One launch, with programmatic stream serialization unless BOLT_B200_NO_PDL is set in the environment
-// (or the runtime refuses the attribute, in which case the plain launch is used from then on).
 // PAIR launches clusters of two CTAs.
-std::atomic<int> g_pdl{-1};
-
 template <int KIND, bool ROWS, int EW, bool PAIR>
 cudaError_t launch_one(uint32_t grid, cudaStream_t st, const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc,
     const Params &p)
 {
-    int pdl = g_pdl.load(std::memory_order_relaxed);
-    if (pdl < 0) {
-        const char *e = getenv("BOLT_B200_NO_PDL");
-        pdl = (e != nullptr && e[0] != '\0' && e[0] != '0') ? 0 : 1;
-        g_pdl.store(pdl, std::memory_order_relaxed);
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(64 + EW * 32);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    int n = 0;
-    if (PAIR) {
-        at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = 2;
-        at[n].val.clusterDim.y = 1;
-        at[n].val.clusterDim.z = 1;
-        ++n;
-    }
-    const int base = n;
-    if (pdl) {
-        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = n;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_u8s8_tcgen05_kernel<KIND, ROWS, EW, PAIR>, ma, mb, mc, p);
-    if (e != cudaSuccess && pdl) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(st, &cap);
-        if (cap == cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            g_pdl.store(0, std::memory_order_relaxed);
-            cfg.numAttrs = base;
-            e = cudaLaunchKernelEx(&cfg, gemm_u8s8_tcgen05_kernel<KIND, ROWS, EW, PAIR>, ma, mb, mc, p);
-        }
-    }
-    return e;
+    cfg.numAttrs = PAIR ? 1 : 0;
+    return launch_programmatic(cfg, gemm_u8s8_tcgen05_kernel<KIND, ROWS, EW, PAIR>, ma, mb, mc, p);
 }
 
 template <bool PAIR>

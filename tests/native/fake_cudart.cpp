@@ -31,6 +31,7 @@ struct Names {
 };
 std::vector<std::string> launched;
 void *max_words = nullptr;   // where the last absmax_kernel was to count
+int refused = 0;
 bool refuse_programmatic = false, refuse_fills = false;
 struct Call {
     dim3 grid, block;
@@ -105,6 +106,10 @@ void *fake_max_words(void)
 void fake_refuse_programmatic(int on)
 {
     refuse_programmatic = on != 0;
+}
+int fake_refused(void)
+{
+    return refused;
 }
 void fake_refuse_fills(int on)
 {
@@ -275,6 +280,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void
 {
     for (unsigned i = 0; i < c->numAttrs; ++i) {
         if (refuse_programmatic && c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization) {
+            ++refused;
             return fail(cudaErrorNotSupported);
         }
     }

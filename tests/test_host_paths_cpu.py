@@ -98,3 +98,28 @@ def test_matmul_over_its_operands_copies_them_first(m, n, k, over):
     lib.fake_forget_launches()
     assert matmul_code(*args, c_dt=U, over=over)[0] == B.SUCCESS          # goes through the scratch anyway
     assert batched()
+
+
+def gemm_codes(lib, m, n, k, chained):
+    a, w, out = np.zeros(m * k, np.uint8), np.zeros((n + 16) * (k + 16), np.int8), np.zeros(m * n, np.float32)
+    w16 = (w.ctypes.data + 15) & ~15
+    calls = (B.GemmCall * 2)()
+    for c in calls:
+        c.N, c.M, c.K, c.A, c.packedB, c.offsetC, c.C = n, m, k, (a.ctypes.data + 15) & ~15, w16, w16, out.ctypes.data
+        c.epilogue.out_dt, c.epilogue.out_scale, c.epilogue.sA, c.epilogue.sB = F, 1.0, 1.0, 1.0
+    if chained:
+        return [lib.bolt_b200_gemm_u8s8_chain(calls, 2)]
+    return [lib.bolt_b200_gemm_u8s8_ex(c.N, c.M, c.K, c.A, c.packedB, c.offsetC, c.C, C.byref(c.epilogue)) for c in calls]
+
+
+@pytest.mark.parametrize("call", [
+    lambda lib: gemm_codes(lib, 8, 64, 64, False), lambda lib: gemm_codes(lib, 8, 64, 64, True), lambda lib: gemm_codes(lib, 256, 64, 64, False),
+    lambda lib: [matmul_code(lib, (2, m, 16), (2, 16, 8), (2, m, 8))[0] for m in (1, 4)]])
+def test_programmatic_serialization_refused(call):
+    """a runtime that does not take the launch attribute gets the plain launch, from then on at once"""
+    lib = fake_gpu.fresh()
+    lib.fake_refuse_programmatic(1)
+    assert set(call(lib)) == {B.SUCCESS} and lib.fake_last_error() == 0
+    n = lib.fake_refused()
+    assert n >= 1
+    assert set(call(lib)) == {B.SUCCESS} and lib.fake_refused() == n
