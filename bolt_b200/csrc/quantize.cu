@@ -416,7 +416,6 @@ EE quantize_cuda_b200(const TensorDesc *dDesc, const void *data, TensorDesc *qDe
         } else {
             B200_EE((launch_to8<float, F32ToI8>(reinterpret_cast<const float *>(d_src), n, d_q, F32ToI8{*scale}, st)));
         }
-        count_launch();
     } else if (sdt == DT_U8_Q) {
         u8_to_i8_kernel<<<grid, TPB, 0, st>>>(reinterpret_cast<const uint8_t *>(d_src), n, d_q);
         count_launch();
@@ -436,7 +435,6 @@ EE quantize_cuda_b200(const TensorDesc *dDesc, const void *data, TensorDesc *qDe
         } else {
             B200_EE((launch_to8<int32_t, I32ToI8>(reinterpret_cast<const int32_t *>(d_src), n, d_q, I32ToI8{raw}, st)));
         }
-        count_launch();
     }
     return sg.finish();
 }

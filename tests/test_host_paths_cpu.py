@@ -123,3 +123,21 @@ def test_programmatic_serialization_refused(call):
     n = lib.fake_refused()
     assert n >= 1
     assert set(call(lib)) == {B.SUCCESS} and lib.fake_refused() == n
+
+
+@pytest.mark.parametrize("src,dst", [(F, U), (F, I), (U, I), (B.DT_I32, U), (B.DT_I32, I)])
+@pytest.mark.parametrize("scale", [-1.0, 3.0])
+def test_every_launch_is_counted_once(src, dst, scale):
+    lib = fake_gpu.load()
+    x, q, s = np.zeros(64, np.float32), np.zeros(64, np.uint8), (C.c_float * 2)(scale, 2.0)
+    d, o = B.tensor1d(src, 64), B.tensor1d(dst, 64)
+    before = lib.bolt_b200_launch_count()
+    assert lib.quantize_cuda_b200(C.byref(d), C.c_void_p(x.ctypes.data), C.byref(o), C.c_void_p(q.ctypes.data), s, 1) == B.SUCCESS
+    assert lib.bolt_b200_launch_count() - before == lib.fake_launches() != 0
+    before, _ = lib.bolt_b200_launch_count(), lib.fake_forget_launches()
+    for m, n in ((1, 8), (4, 8), (4, 1)):
+        for c_dt, c_scale, bias in ((F, -1.0, n), (U, -1.0, 0), (U, 3.0, 0)):
+            assert matmul_code(lib, (2, m, 16), (2, 16, n), (2, m, n), c_dt=c_dt, c_scale=c_scale, bias=bias)[0] == B.SUCCESS
+    assert set(gemm_codes(lib, 8, 64, 64, True) + gemm_codes(lib, 256, 64, 64, False) + gemm_codes(lib, 8, 64, 63, False)) == {B.SUCCESS}
+    assert lib.bolt_b200_absmax_scale_f32(C.c_void_p(x.ctypes.data), x.size, s) == B.SUCCESS
+    assert lib.bolt_b200_launch_count() - before == lib.fake_launches()
