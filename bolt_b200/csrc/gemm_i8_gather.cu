@@ -1023,6 +1023,7 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
         cfg.gridDim = dim3((uint32_t)std::min<uint64_t>(work, 8 * (uint64_t)c->sm_count));
         cfg.dynamicSmemBytes = mvm_smem;
         const int af = mb.a.f32 ? 1 : 0;
+        tls().last_gemm_tc = 0;
         e = lb == ROWS_K ? launch_behind(reduction, cfg, mvm_batch_kernel<ROWS_K>, p, bp, af)
             : lb == K_ROWS ? launch_behind(reduction, cfg, mvm_batch_kernel<K_ROWS>, p, bp, af)
             : lb == F32_ROWS_K ? launch_behind(reduction, cfg, mvm_batch_kernel<F32_ROWS_K>, p, bp, af)

@@ -450,6 +450,7 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
         const char *pb = reinterpret_cast<const char *>(B) + ib * b2;
         char *pc = reinterpret_cast<char *>(prod) + ic * c2;
         EE ret;
+        tls().last_gemm_tc = 0;   // (the GEMM sets it)
         if (p.a.dims[1 - p.kDimA] == 1) {
             ret = b200_matrix_vector_multiply(
                 desc2d(p.qb, p.dfB == DF_TRANSPOSE ? DF_NORMAL : DF_TRANSPOSE, p.b.dims[1], p.b.dims[0]), pb,

@@ -216,7 +216,8 @@ EE bolt_b200_i8_mma_rate(U32 mma_per_sm, F32 *milliseconds, F32 *tops);
 EE bolt_b200_selftest_wait_limit(U32 limit_cycles);
 /* Number of kernels this library has launched in this process (all threads). */
 uint64_t bolt_b200_launch_count(void);
-/* 1 if the u8 x s8 tensor-core (tcgen05) GEMM was used by the last GEMM call of this thread. */
+/* 1 if the last GEMM or matmul call of this thread ran on the tensor cores: every GEMM does (tcgen05, products of few
+ * rows mma.sync).  0 before the first one, and after a matmul whose result has one row or one column (GEMV kernels). */
 int bolt_b200_last_gemm_used_tensor_cores(void);
 
 /* ============================== 2. kernels ================================================ */

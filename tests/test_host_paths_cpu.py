@@ -141,3 +141,35 @@ def test_every_launch_is_counted_once(src, dst, scale):
     assert set(gemm_codes(lib, 8, 64, 64, True) + gemm_codes(lib, 256, 64, 64, False) + gemm_codes(lib, 8, 64, 63, False)) == {B.SUCCESS}
     assert lib.bolt_b200_absmax_scale_f32(C.c_void_p(x.ctypes.data), x.size, s) == B.SUCCESS
     assert lib.bolt_b200_launch_count() - before == lib.fake_launches()
+
+
+KERNELS = {"gemm_skinny_kernel": "rows", "gemm_u8s8_tcgen05_kernel": "tma", "gemm_gather_kernel": "gathered", "mvm_batch_kernel": "row"}
+
+
+def kernel_of(lib):
+    """the kernels of a call, those around the products left out"""
+    return [v for x in fake_gpu.launches(lib) for k, v in KERNELS.items() if k in x]
+
+
+@pytest.mark.parametrize("m,k,n,expect", [
+    (16, 768, 6144, "rows"), (16, 768, 6145, "tma"), (1, 5456, 6144, "rows"), (1, 5472, 6144, "tma"),                 # 32 MiB and 6144 columns
+    (17, 2048, 6144, "rows"), (17, 2064, 6144, "tma"), (32, 16384, 2048, "rows"), (32, 16400, 2048, "tma"), (32, 6144, 2049, "tma"),
+    (33, 768, 1184, "rows"), (33, 768, 1185, "tma"), (64, 768, 1184, "rows"), (65, 768, 1184, "tma"), (64, 28336, 1184, "rows"), (64, 28352, 1184, "tma"),
+    (4096, 768, 3072, "tma"), (16, 760, 768, "gathered"), (300, 515, 1001, "gathered")])
+def test_gemm_dispatch(m, k, n, expect):
+    """both sides of every line of the rules; nothing reads the operands here"""
+    lib = fake_gpu.load()
+    ep = B.GemmEpilogue()
+    ep.out_dt, ep.out_scale, ep.sA, ep.sB = F, 1.0, 1.0, 1.0
+    call = lambda a: lib.bolt_b200_gemm_u8s8_ex(n, m, k, C.c_void_p(a), C.c_void_p(8192), C.c_void_p(8192), C.c_void_p(16384), C.byref(ep))
+    assert call(4096) == B.SUCCESS and kernel_of(lib) == [expect]
+    assert lib.bolt_b200_last_gemm_used_tensor_cores() == 1
+    lib.fake_forget_launches()
+    assert call(4097) == B.SUCCESS and kernel_of(lib) == ["gathered"]      # rows of A off the 16-byte grid
+
+
+def test_matmul_reports_what_ran():
+    lib = fake_gpu.load()
+    for m, n, tc in ((4, 8, 1), (1, 8, 0), (4, 8, 1), (4, 1, 0)):
+        assert matmul_code(lib, (2, m, 16), (2, 16, n), (2, m, n))[0] == B.SUCCESS
+        assert lib.bolt_b200_last_gemm_used_tensor_cores() == tc, (m, n)
