@@ -357,6 +357,7 @@ struct MatmulBatch {
     float c_scale;
 };
 EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st);
+uint32_t gather_block_n(uint64_t tiles_m, uint32_t N, int sms);   // column block of its tiles
 EE launch_pack_rhs(const int8_t *src, bool src_is_nk, uint32_t N, uint32_t K, int8_t *dst,
     uint32_t Kp, uint32_t Np, int32_t *offsetC, cudaStream_t st);
 EE launch_gemv_row(uint32_t N, uint32_t K, const uint8_t *Mx, bool transposed, const int8_t *v, void *y, int out_kind,

@@ -802,8 +802,16 @@ mvm_batch_kernel(const __grid_constant__ GatherParams p, const __grid_constant__
     }
 }
 
+int row_alignment(const void *p, uint64_t ld)
+{
+    const uint64_t a = reinterpret_cast<uintptr_t>(p) | ld;
+    return a % 16 == 0 ? 16 : (a % 8 == 0 ? 8 : 1);
+}
+
+}  // namespace
+
 // Tile width: as few column blocks of at most 128 as cover N, narrower while there are fewer tiles than SMs.
-uint32_t pick_bn(uint64_t tiles_m, uint32_t N, int sms)
+uint32_t gather_block_n(uint64_t tiles_m, uint32_t N, int sms)
 {
     const uint32_t blocks = (N + MAX_BN - 1) / MAX_BN;
     uint32_t bn = (uint32_t)B200_ALIGN((N + blocks - 1) / blocks, 32);
@@ -812,14 +820,6 @@ uint32_t pick_bn(uint64_t tiles_m, uint32_t N, int sms)
     }
     return bn;
 }
-
-int row_alignment(const void *p, uint64_t ld)
-{
-    const uint64_t a = reinterpret_cast<uintptr_t>(p) | ld;
-    return a % 16 == 0 ? 16 : (a % 8 == 0 ? 8 : 1);
-}
-
-}  // namespace
 
 // A u8 [M][K] (or [K][M] when a_transposed), B the packed weight [ALIGN(N,16)][Kp], zero padded.
 EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool a_transposed, const int8_t *B,
@@ -844,7 +844,7 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
     p.N = N;
     p.K = K;
     p.tiles_m = (M + BLOCK_M - 1) / BLOCK_M;
-    p.block_n = pick_bn(p.tiles_m, N, c->sm_count);
+    p.block_n = gather_block_n(p.tiles_m, N, c->sm_count);
     p.tiles_n = (N + p.block_n - 1) / p.block_n;
     p.tmem_cols = p.block_n > 64 ? 128u : p.block_n;
     p.a.p = A;
@@ -1030,7 +1030,7 @@ EE launch_matmul_batch(const MatmulBatch &mb, cudaStream_t st)
                                : launch_behind(reduction, cfg, mvm_batch_kernel<F32_K_ROWS>, p, bp, af);
     } else {
         p.tiles_m = (mb.M + BLOCK_M - 1) / BLOCK_M;
-        p.block_n = pick_bn((uint64_t)p.tiles_m * mb.batches, mb.N, c->sm_count);
+        p.block_n = gather_block_n((uint64_t)p.tiles_m * mb.batches, mb.N, c->sm_count);
         p.tiles_n = (mb.N + p.block_n - 1) / p.block_n;
         p.tmem_cols = p.block_n > 64 ? 128u : p.block_n;
         cfg.dynamicSmemBytes = SMEM_BYTES;

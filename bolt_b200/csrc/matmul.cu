@@ -2,14 +2,15 @@
 // CUDA_B200: both operands may arrive as fp32 and are quantized per call (dynamic scale 127 / absmax, or the
 // scale the tensor carries), and the result is written as fp32 (accumulator / (scaleA * scaleB)) or requantized
 // to u8.  All products of a call run in one launch that quantizes its operands while it loads them
-// (launch_matmul_batch); a single large product, a result of one column and one that lies over its operands take the
-// quantize / pack / multiply kernels one after the other.
+// (launch_matmul_batch); where that is slower (few tiles and a long K, large products), for a result of one column and for
+// one that lies over its operands, the quantize / pack / multiply kernels run one after the other.
 //
 // The x86 convention applies (matmul.cpp:373-398): u8 activations with zero point 128 times s8, except
 // when the result is a vector, where A becomes s8 and B u8.  Leading (batch) dimensions broadcast as in
 // matmul.cpp:489-517.  All work is enqueued on the thread's stream; the scale of a dynamically requantized u8 result
 // comes back to the host, which is what the operator's interface (Tensor::get_scale) requires.
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -180,18 +181,78 @@ U32 global_index(uint64_t ic, const TensorDesc &c, const TensorDesc &x)
     return g;
 }
 
-// One launch for all products, or one product after the other through quantize, pack and the TMA GEMM?  The batched
-// kernel never packs and keeps the host out of it, but it converts an fp32 operand again for every tile row / column
-// of the other one and fills the tensor pipe a quarter as well.  Measured (fp32 in and out, us per call, one launch
-// against one by one): 1 x 512^3 37 / 75, 1 x 1024^3 73 / 83, 1 x 2048^3 209 / 112; 4 x 512^3 42 / 123,
-// 4 x 1024^3 112 / 145, 4 x 2048^3 903 / 272; 384 x (128 x 64 x 128 and 128 x 128 x 64) 47 / 8000 for the pair.
-bool one_launch(const Plan &p)
+// One launch for all products, or one product after the other through quantize, pack and the TMA GEMM (GEMV)?  The batched
+// kernels never pack and keep the host out of it, but they convert an fp32 operand again for every tile row / column of
+// the other one, fill the tensor pipe a quarter as well, and one CTA walks all of a tile's K.  So the two are estimated,
+// in us; the constants are fitted to the figures behind, us per call, one launch against one by one:
+//   fp32 in and out: 128 x 128 with K = 512 22 / 38, 1024 37 / 39, 2048 66 / 43, 16384 466 / 101; 1024 x 1024 with K = 256
+//   18 / 39, 1024 68 / 43; 4 x (128 x 128) with K = 4096 123 / 131, 8192 240 / 189; 12 x (16 x 64) with K = 16384
+//   449 / 648; 4 x 1024^3 86 / 89; 384 x (128 x 64 x 128 and 128 x 128 x 64) 47 / 8000 for the pair
+//   u8 x s8: 128 x 128 with K = 1024 12 / 14, 2048 19 / 14, 65536 427 / 214; 16 x 16384 with K = 4096 39 / 72; 1024^3
+//   14 / 16; 4 x (256 x 256) with K = 16384 115 / 241
+//   K off the 16-byte grid, or A stored [K][M]: fp32 136 x 36 x 25084 719 / 363, 3 x (12 x 7 x 5708) 156 / 274, [K][M]
+//   87 x 9 x 20897 735 / 1047; fp32 x s8, [K][M] 2 x (1860 x 4 x 7664) 381 / 272
+//   a row, matrix stored [N][K]: fp32 768 x 768 14 / 32, 768 x 3072 63 / 38, 1024 x 16384 340 / 70, 4 x (2048 x 2048)
+//   57 / 68; u8 1024 x 1024 12 / 9, 8192 x 8192 68 / 21, 2 x (1024 x 1024) 12 / 13, 96 x (2048 x 64) 25 / 396
+//   a row, matrix stored [K][N]: one launch is faster throughout (1 x 65536 x 64 8 / 10 ... 96 x 64 x 2048 18 / 5318)
+// Products of more than 2^30 multiply-adds always go one by one (1 x 2048^3 209 / 112, 4 x 2048^3 903 / 272).
+struct Product {
+    double M, N, K, batches, elems;   // elems: of the fp32 operands
+    bool f32_a, f32_b, a_cols, b_rows;   // a_cols: A is stored [K][M]; b_rows: B [N][K]
+    bool tma;                            // TMA can fetch the (quantized) A
+};
+bool one_launch_is_faster(const Product &q, int sms)
 {
-    const uint64_t M = p.a.dims[1 - p.kDimA], N = p.b.dims[1 - p.kDimB], K = p.a.dims[p.kDimA];
-    if (M == 1) {
-        return true;    // a row per product: the batched GEMV
+    const double quantize = 12.0 * (q.f32_a + q.f32_b);   // two launches and a wait of the host
+    if (q.M == 1) {
+        if (!q.b_rows) {
+            return true;
+        }
+        // 32 rows per block, eight blocks per SM: a warp's loads one behind the other
+        const double rounds = std::ceil(std::ceil(q.N / 32) * q.batches / (8.0 * sms));
+        const double loads = q.K >= 128 ? 4 * std::ceil(q.K / 128) : std::ceil(q.K / 32);
+        const double batched = 5 + 1.5 * (q.f32_a + q.f32_b) + rounds * loads * (q.f32_b ? 0.65 : 0.235) + 0.8e-6 * q.elems;
+        const double singly = 9 + quantize + 4.3 * (q.batches - 1) + q.batches * q.K * 0.8e-3 + 1.5e-6 * q.elems;
+        return batched <= singly;
     }
-    return N != 1 && M * N <= (1ull << 30) / K;
+    if (q.M * q.N * q.K > (double)(1ull << 30)) {
+        return false;
+    }
+    // K blocks of 128 bytes; the tiles of launch_matmul_batch
+    const double kb = std::ceil(q.K / 128), tiles_m = q.batches * std::ceil(q.M / 128);
+    const double bn = gather_block_n((uint64_t)tiles_m, (uint32_t)q.N, sms), tiles = tiles_m * std::ceil(q.N / bn);
+    const bool f32 = q.f32_a || q.f32_b;   // (binary32 keeps an SM busy; bytes are fetched ahead, and CTAs share the SM)
+    const double rounds = f32 ? std::ceil(tiles / sms) : std::max(1.0, tiles / (2.5 * sms));
+    const double batched = (f32 ? 8 : 5.5) + rounds * kb * (0.83 + (q.a_cols ? 4.0 : 2.4) * q.f32_a + 0.4 * (bn / 32) * q.f32_b) + 0.8e-6 * q.elems;
+    // Singly, B is packed and C is cleared, read and written; a K block costs 0.4 where TMA can fetch A, else its bytes are
+    // gathered, one by one from unaligned columns.
+    const double block = q.tma ? 0.4 : (q.a_cols && (uint64_t)q.M % 4 != 0 ? 6.2 : 1.8);
+    const double singly = std::max(14.0, 8 + block * kb) + quantize + (q.batches - 1) * std::max(10.0, 6 + block * kb) + 1.5e-6 * q.elems +
+        (0.6e-6 * q.K + 2.4e-6 * q.M) * q.N * q.batches;
+    return batched <= singly;
+}
+bool one_launch(const Plan &p, const void *A, int sms, cudaStream_t st)
+{
+    Product q;
+    q.M = p.a.dims[1 - p.kDimA];
+    q.N = p.b.dims[1 - p.kDimB];
+    q.K = p.a.dims[p.kDimA];
+    q.batches = (double)p.loopsC;
+    q.f32_a = p.quantA;
+    q.f32_b = p.quantB;
+    q.elems = (p.quantA ? (double)elems(p.a) : 0) + (p.quantB ? (double)elems(p.b) : 0);
+    q.a_cols = p.dfA == DF_TRANSPOSE;
+    q.b_rows = p.dfB == DF_TRANSPOSE;
+    q.tma = !q.a_cols && p.a.dims[p.kDimA] % 16 == 0 && (p.quantA || reinterpret_cast<uintptr_t>(A) % 16 == 0);
+    if (q.M != 1 && q.N == 1) {
+        return false;   // a result of one column has no batched kernel
+    }
+    if (one_launch_is_faster(q, sms)) {
+        return true;
+    }
+    // The scales of separately quantized operands have to reach the host, which a stream that is being captured cannot wait
+    // for: there the batched kernels take what they can.
+    return (p.quantA || p.quantB) && (q.M == 1 || q.M * q.N * q.K <= (double)(1ull << 30)) && capturing(st);
 }
 
 bool overlap(const void *a, size_t na, const void *b, size_t nb)
@@ -367,7 +428,7 @@ EE matmul_cuda_b200(const TensorDesc *aDesc, int transposeA, const void *A, F32 
     // The batched kernel reads A and B while it writes C.  A result over its own operands (fp32 in, fp32 out) needs the
     // quantized copies of the other way.
     const bool in_place = !p.stageC && (overlap(C, c_bytes, A, (size_t)nA * bytes_of(p.a.dt)) || overlap(C, c_bytes, B, (size_t)nB * bytes_of(p.b.dt)));
-    const bool fused = !in_place && one_launch(p);
+    const bool fused = !in_place && one_launch(p, A, c->sm_count, st);
     // (the tmp bytes count 1 KiB more than what is laid out in it)
     char *t = fused ? reinterpret_cast<char *>(B200_ALIGN(reinterpret_cast<uintptr_t>(tmp), 16)) : reinterpret_cast<char *>(tmp);
     char *slotsA = t, *slotsB = t + (p.quantA ? B200_ALIGN(nA, 256) : 0);

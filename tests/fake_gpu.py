@@ -37,6 +37,7 @@ def load():
     if _lib is None:
         _lib = fresh()
     _lib.fake_refuse_programmatic(0)
+    _lib.fake_capture(0)
     _lib.fake_set_last_error(0)
     _lib.fake_forget_launches()
     return _lib

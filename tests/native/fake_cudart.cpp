@@ -32,7 +32,7 @@ struct Names {
 std::vector<std::string> launched;
 void *max_words = nullptr;   // where the last absmax_kernel was to count
 int refused = 0;
-bool refuse_programmatic = false, refuse_fills = false;
+bool captured = false, refuse_programmatic = false, refuse_fills = false;
 struct Call {
     dim3 grid, block;
     size_t smem;
@@ -102,6 +102,10 @@ void fake_forget_launches(void)
 void *fake_max_words(void)
 {
     return max_words;
+}
+void fake_capture(int on)   // streams are being captured
+{
+    captured = on != 0;
 }
 void fake_refuse_programmatic(int on)
 {
@@ -238,7 +242,7 @@ cudaError_t cudaDeviceSynchronize(void)
 }
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *s)
 {
-    *s = cudaStreamCaptureStatusNone;
+    *s = captured ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t *)

@@ -173,3 +173,46 @@ def test_matmul_reports_what_ran():
     for m, n, tc in ((4, 8, 1), (1, 8, 0), (4, 8, 1), (4, 1, 0)):
         assert matmul_code(lib, (2, m, 16), (2, 16, n), (2, m, n))[0] == B.SUCCESS
         assert lib.bolt_b200_last_gemm_used_tensor_cores() == tc, (m, n)
+
+
+def matmul_route(lib, b, m, n, k, ta, tb, a_dt, b_dt, a_at=1 << 20):
+    """(status, whether the call took the batched kernels)"""
+    a, w, c = B.tensor_nd(a_dt, (b, k, m) if ta else (b, m, k)), B.tensor_nd(b_dt, (b, n, k) if tb else (b, k, n)), B.tensor_nd(F, (b, m, n))
+    nbytes = C.c_uint32()
+    assert lib.matmul_infer_forward_tmp_bytes_cuda_b200(C.byref(a), ta, C.byref(w), tb, C.byref(c), -1.0, C.byref(nbytes)) == B.SUCCESS
+    tmp, out, s = np.empty(nbytes.value, np.uint8), np.empty(b * m * n, np.float32), C.c_float(-1.0)
+    lib.fake_forget_launches()
+    code = lib.matmul_cuda_b200(C.byref(a), ta, C.c_void_p(a_at), 11.0, C.byref(w), tb, C.c_void_p(1 << 40), 7.0, None, None, nbytes.value,
+                                C.c_void_p(tmp.ctypes.data), C.byref(c), C.c_void_p(out.ctypes.data), C.byref(s))
+    return code, any("absmax_pair_kernel" in x or "mvm_batch_kernel" in x or "gemm_gather_kernel" in x and "Lb1EE" in x for x in fake_gpu.launches(lib))
+
+
+@pytest.mark.parametrize("b,m,n,k,tb,f32,batched", [
+    (1, 128, 128, 1024, 1, 1, 1), (1, 128, 128, 2048, 1, 1, 0), (1, 1024, 1024, 256, 1, 1, 1), (1, 1024, 1024, 1024, 1, 1, 0), (1, 4096, 4096, 64, 1, 1, 1),
+    (4, 128, 128, 2048, 1, 1, 1), (4, 128, 128, 8192, 1, 1, 0), (12, 16, 64, 16384, 1, 1, 1), (64, 128, 128, 2048, 1, 1, 1), (24, 128, 64, 128, 0, 1, 1),
+    (1, 128, 128, 1024, 1, 0, 1), (1, 128, 128, 2048, 1, 0, 0), (4, 256, 256, 16384, 1, 0, 1), (1, 16, 16384, 4096, 1, 0, 1), (1, 2048, 2048, 2048, 0, 0, 0),
+    (1, 1, 768, 768, 1, 1, 1), (1, 1, 768, 3072, 1, 1, 0), (1, 1, 768, 3072, 0, 1, 1), (4, 1, 2048, 2048, 1, 1, 1),
+    (1, 1, 1024, 1024, 1, 0, 0), (1, 1, 1024, 1024, 0, 0, 1), (2, 1, 1024, 1024, 1, 0, 1), (96, 1, 2048, 64, 1, 0, 1), (3, 8, 1, 64, 0, 1, 0)])
+def test_matmul_dispatch(b, m, n, k, tb, f32, batched):
+    """both sides of the measured figures beside the rule"""
+    lib = fake_gpu.load()
+    dts = (F, F) if f32 else ((I, U) if 1 in (m, n) else (U, I))
+    assert matmul_route(lib, b, m, n, k, 0, tb, *dts) == (B.SUCCESS, bool(batched))
+    # a captured stream: operands whose scale the host cannot wait for stay with the batched kernels where these exist
+    lib.fake_capture(1)
+    code, took = matmul_route(lib, b, m, n, k, 0, tb, *dts)
+    lib.fake_capture(0)
+    if f32 and n != 1:
+        assert (code, took) == (B.SUCCESS, True)
+    elif not f32:
+        assert (code, took) == (B.SUCCESS, bool(batched))
+    else:
+        assert code == B.UNKNOWN
+
+
+def test_matmul_dispatch_of_operands_that_tma_cannot_fetch():
+    lib = fake_gpu.load()
+    route = lambda *a, **kw: matmul_route(lib, *a, **kw)[1]
+    assert not route(1, 136, 36, 25084, 0, 0, F, F) and route(3, 12, 7, 5708, 0, 1, F, F)        # K off the 16-byte grid
+    assert route(1, 87, 9, 20897, 1, 0, F, F) and not route(2, 1860, 4, 7664, 1, 1, F, I)        # A stored [K][M]
+    assert not route(1, 64, 64, 4096, 0, 1, U, I) and route(1, 64, 64, 4096, 0, 1, U, I, a_at=(1 << 20) + 4)

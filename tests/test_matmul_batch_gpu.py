@@ -74,6 +74,69 @@ def test_result_over_its_operands(m, k, n, over):
     assert to_host(d_c, np.float32, 3 * m * n).tobytes() == np.ascontiguousarray(ref).tobytes()
 
 
+SPECIAL = [np.inf, -np.inf, 3e38, -3e38, np.float32(2147483648.0), np.float32(2147483520.0), -2147483648.0, 254.5, 255.5, -0.5]
+
+
+@pytest.mark.parametrize("m", [1, 5])
+@pytest.mark.parametrize("given", [-1.0, 1.0, 5.0, 1e30])
+def test_quantization_of_extreme_values(m, given):
+    """infinities, products beyond the int32 range and ties through the quantization inside the batched kernels; a given scale
+    above the dynamic one is what takes finite values out of range"""
+    for i, v in enumerate(SPECIAL):
+        a, b = synth.normal(31, (2, m, 40)), synth.normal(32, (2, 40, 24))
+        for x in ((a, b)[i % 2], (a, b)[1 - i % 2]):
+            y = x.copy()
+            y[0, 0, 3] = y[1, -1, 7] = v
+            A, Bm = (y, b) if x is a else (a, y)
+            with np.errstate(all="ignore"):
+                C, _ = matmul_gpu(A, F, given, 0, Bm, F, given, 0, None, F, -1.0)
+                Cp, _ = O.port_matmul(A, F, given, 0, Bm, F, given, 0, None, F, -1.0)
+            assert np.array_equal(C, Cp, equal_nan=True), (v, x is a)
+
+
+@pytest.mark.parametrize("m", [1, 24])
+@pytest.mark.parametrize("given", [-1.0, 5.0])
+def test_nan_goes_the_way_of_the_separate_kernels(m, given):
+    """a NaN is the largest magnitude for every kernel that looks for one, and makes the scale NaN; the result over its own
+    operand takes the quantize and GEMM (GEMV) kernels"""
+    a, b = synth.normal(33, (2, m, 32)), synth.normal(34, (2, 32, 32))
+    a[1, 0, 5] = np.nan
+    ad, bd = B.tensor_nd(F, a.shape), B.tensor_nd(F, b.shape)
+    tmp_bytes = B.matmul_infer_forward_tmp_bytes(ad, 0, bd, 0, ad, -1.0)
+    got = []
+    for apart in (True, False):
+        d_a, d_b = to_dev(a), to_dev(b)
+        d_c = dev_zeros(a.nbytes) if apart else d_a
+        B.matmul(ad, 0, dptr(d_a), given, bd, 0, dptr(d_b), -1.0, None, None, tmp_bytes, dptr(dev_zeros(tmp_bytes)), ad, dptr(d_c), -1.0)
+        got.append(to_host(d_c, np.float32, a.size))
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("m,k,n,batch", [(40, 6001, 33, 1), (128, 9000, 128, 1), (33, 9000, 40, 2), (16, 3000, 24, 7)])
+@pytest.mark.parametrize("a_dt", [F, U])
+@pytest.mark.parametrize("b_dt", [F, I])
+def test_long_k(m, k, n, batch, a_dt, b_dt):
+    """on both sides of the rule that sends a few tiles with a long K through the separate kernels"""
+    sa, sb = (-1.0 if a_dt == F else 11.0), (-1.0 if b_dt == F else 7.0)
+    for ta, tb in itertools.product((0, 1), (0, 1)):
+        a, b = operand(35, (batch, k, m) if ta else (batch, m, k), a_dt), operand(36, (batch, n, k) if tb else (batch, k, n), b_dt)
+        check((a, a_dt, sa, ta, b, b_dt, sb, tb, None, F, -1.0))
+        check((a, a_dt, sa, ta, b, b_dt, sb, tb, synth.normal(37, (n,)), F, -1.0))
+        check((a, a_dt, sa, ta, b, b_dt, sb, tb, None, U, (-1.0, 0.5)[ta]))
+
+
+@pytest.mark.parametrize("k,n,batch", [(4099, 65, 1), (4096, 128, 1), (9001, 96, 2), (2048, 40, 5), (768, 2, 1)])
+@pytest.mark.parametrize("a_dt", [F, I])
+@pytest.mark.parametrize("b_dt", [F, U])
+def test_one_long_row(k, n, batch, a_dt, b_dt):
+    """the same for a result of one row, whose matrix is stored either way"""
+    sa, sb = (-1.0 if a_dt == F else 9.0), (-1.0 if b_dt == F else 13.0)
+    for tb, c_scale in itertools.product((0, 1), (-1.0, 0.5)):
+        a, b = operand(38, (batch, 1, k), a_dt), operand(39, (batch, n, k) if tb else (batch, k, n), b_dt)
+        check((a, a_dt, sa, 0, b, b_dt, sb, tb, None, F if c_scale < 0 else U, c_scale))
+        check((a, a_dt, sa, 0, b, b_dt, sb, tb, None, U, -1.0))
+
+
 def test_single_large_product_goes_one_by_one():
     a, b = synth.normal(9, (1, 1040, 1024)), synth.normal(10, (1, 1024, 1040))
     check((a, F, -1.0, 0, b, F, -1.0, 0, None, F, -1.0))

@@ -15,6 +15,7 @@ from test_gather_gpu import product  # noqa: E402
 from util import dev_zeros, dptr, to_dev, to_host  # noqa: E402
 
 pytestmark = pytest.mark.gpu
+F32 = B.DT_F32
 
 
 @pytest.mark.parametrize("m", [1, 2, 15, 16, 17, 32, 33, 64, 65])
@@ -95,6 +96,66 @@ def test_input_scale_from_an_earlier_call(m):
         B.CHECK_STATUS(lib.bolt_b200_gemm_u8s8_chain(calls, 3))
         B.CHECK_STATUS(lib.bolt_b200_synchronize(), "synchronize")
         assert to_host(d_out, np.float32, m * n).tobytes() == ref
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("n", [24, 33])
+@pytest.mark.parametrize("out", [B.DT_F32, B.DT_U8_Q])
+@pytest.mark.parametrize("scales", ["row", "row_col", "col", "factor", "d_sA"])
+def test_scales(m, n, out, scales):
+    """per-row and per-column scales, ready-made factors, an input scale in device memory: one binary32 product, one division"""
+    k = 272
+    A, W = synth.u8(41, (m, k)), synth.s8(42, (k, n))
+    (_, _, packed, rhs, _), = chain_layers(m, [k, n], 42)
+    row = (np.abs(synth.normal(43, (m,))) + 5).astype(np.float32)
+    col = (np.abs(synth.normal(44, (n,))) + 100).astype(np.float32)
+    num = np.float32(40.0 if out == B.DT_U8_Q else 1.0)
+    ep = B.GemmEpilogue()
+    ep.out_dt, ep.out_scale, ep.sA, ep.sB = out, float(num), 7.5, 90.0
+    sA, sB = np.float32(7.5), np.float32(90.0)
+    d_row, d_col, d_fac, d_sa = to_dev(row), to_dev(col), to_dev((num / col).astype(np.float32)), to_dev(np.array([3.25], np.float32))
+    if "row" in scales:
+        ep.row_scale, sA = d_row.data_ptr(), row[:, None]
+    if "col" in scales:
+        ep.col_scale, sB = d_col.data_ptr(), col[None, :]
+    if scales == "d_sA":
+        ep.d_sA, sA = d_sa.data_ptr(), np.float32(3.25)
+    fac = (num / (sA * sB).astype(np.float32)).astype(np.float32) * np.ones((m, n), np.float32)
+    if scales == "factor":
+        ep.col_factor, fac = d_fac.data_ptr(), (num / col).astype(np.float32)[None, :]
+    d_a, d_c = to_dev(A), dev_zeros(m * n * 4)
+    B.CHECK_STATUS(B.lib().bolt_b200_gemm_u8s8_ex(n, m, k, dptr(d_a), dptr(packed), dptr(packed, rhs), dptr(d_c), C.byref(ep)))
+    v = (O.port_gemm(A, W, O.port_offsetc(W)).astype(np.float32) * fac).astype(np.float32)
+    if out == B.DT_F32:
+        assert to_host(d_c, np.float32, m * n).tobytes() == np.ascontiguousarray(v).tobytes()
+    else:
+        r = np.rint(v).astype(np.int64) + 128
+        assert to_host(d_c, np.uint8, m * n).tobytes() == np.where(r < 0, 255, np.minimum(r, 255)).astype(np.uint8).tobytes()
+
+
+@pytest.mark.parametrize("m", [1, 32])
+def test_chain_with_host_pointers(m):
+    """the first input and the last result in host memory, the layers between them on the device"""
+    lib, dims = B.lib(), [256, 128, 512, 64]
+    layers = chain_layers(m, dims, 800)
+    x = synth.u8(9, (m, dims[0]))
+    bufs = [dev_zeros(m * n * 4) for _, n, _, _, _ in layers]
+    host_out = np.zeros(m * dims[-1], np.float32)
+    got = []
+    for host in (False, True):
+        calls = (B.GemmCall * len(layers))()
+        d_x = to_dev(x)
+        a = x.ctypes.data if host else d_x.data_ptr()
+        for c, (k, n, packed, rhs, col), out in zip(calls, layers, bufs):
+            last = out is bufs[-1]
+            c.N, c.M, c.K, c.A, c.packedB, c.offsetC = n, m, k, a, packed.data_ptr(), packed.data_ptr() + rhs
+            a = c.C = host_out.ctypes.data if host and last else out.data_ptr()
+            c.epilogue.out_dt, c.epilogue.out_scale, c.epilogue.sA, c.epilogue.sB = (F32 if last else B.DT_U8_Q), 0.6, 1.5, 1.0
+            c.epilogue.col_scale = col.data_ptr()
+        B.CHECK_STATUS(lib.bolt_b200_gemm_u8s8_chain(calls, len(calls)))
+        B.CHECK_STATUS(lib.bolt_b200_synchronize(), "synchronize")
+        got.append(host_out.tobytes() if host else to_host(bufs[-1], np.float32, m * dims[-1]).tobytes())
+    assert got[0] == got[1] and np.any(np.frombuffer(got[0], np.float32))
 
 
 def test_chain_errors():
