@@ -195,6 +195,8 @@ U32 global_index(uint64_t ic, const TensorDesc &c, const TensorDesc &x)
 //   a row, matrix stored [N][K]: fp32 768 x 768 14 / 32, 768 x 3072 63 / 38, 1024 x 16384 340 / 70, 4 x (2048 x 2048)
 //   57 / 68; u8 1024 x 1024 12 / 9, 8192 x 8192 68 / 21, 2 x (1024 x 1024) 12 / 13, 96 x (2048 x 64) 25 / 396
 //   a row, matrix stored [K][N]: one launch is faster throughout (1 x 65536 x 64 8 / 10 ... 96 x 64 x 2048 18 / 5318)
+// Over 504 random shapes, types and storage orders it takes the faster way within 10 % in all but seven (at worst 1.8 times:
+// fp32, [K][M] 3 x (1796 x 12 x 12753) 1106 / 609).
 // Products of more than 2^30 multiply-adds always go one by one (1 x 2048^3 209 / 112, 4 x 2048^3 903 / 272).
 struct Product {
     double M, N, K, batches, elems;   // elems: of the fp32 operands
@@ -208,11 +210,14 @@ bool one_launch_is_faster(const Product &q, int sms)
         if (!q.b_rows) {
             return true;
         }
-        // 32 rows per block, eight blocks per SM: a warp's loads one behind the other
+        // 32 rows per block, eight blocks per SM: a warp's loads one behind the other, each a latency (twice that for an fp32
+        // matrix of more than 8 MB; bytes off the 8-byte grid are read one at a time)
         const double rounds = std::ceil(std::ceil(q.N / 32) * q.batches / (8.0 * sms));
-        const double loads = q.K >= 128 ? 4 * std::ceil(q.K / 128) : std::ceil(q.K / 32);
-        const double batched = 5 + 1.5 * (q.f32_a + q.f32_b) + rounds * loads * (q.f32_b ? 0.65 : 0.235) + 0.8e-6 * q.elems;
-        const double singly = 9 + quantize + 4.3 * (q.batches - 1) + q.batches * q.K * 0.8e-3 + 1.5e-6 * q.elems;
+        const double loads = std::ceil(std::min(q.N, 32.0) / 8) * std::ceil(q.K / 128);
+        const double load = q.f32_b ? (q.N * q.K * q.batches > (double)(2 << 20) ? 0.58 : 0.27) : ((uint64_t)q.K % 8 == 0 ? 0.235 : 0.45);
+        const double batched = 5 + 1.5 * (q.f32_a + q.f32_b) + rounds * loads * load + 0.8e-6 * q.elems;
+        const double row = ((uint64_t)q.K % 16 == 0 ? 0.9e-3 : 1.8e-3) * q.K;
+        const double singly = 9 + quantize + 4.3 * (q.batches - 1) + q.batches * row + 1.5e-6 * q.elems;
         return batched <= singly;
     }
     if (q.M * q.N * q.K > (double)(1ull << 30)) {
@@ -223,7 +228,10 @@ bool one_launch_is_faster(const Product &q, int sms)
     const double bn = gather_block_n((uint64_t)tiles_m, (uint32_t)q.N, sms), tiles = tiles_m * std::ceil(q.N / bn);
     const bool f32 = q.f32_a || q.f32_b;   // (binary32 keeps an SM busy; bytes are fetched ahead, and CTAs share the SM)
     const double rounds = f32 ? std::ceil(tiles / sms) : std::max(1.0, tiles / (2.5 * sms));
-    const double batched = (f32 ? 8 : 5.5) + rounds * kb * (0.83 + (q.a_cols ? 4.0 : 2.4) * q.f32_a + 0.4 * (bn / 32) * q.f32_b) + 0.8e-6 * q.elems;
+    // (bytes stored across K in rows off the 4-byte grid are loaded one at a time)
+    const double block_a = q.f32_a ? (q.a_cols ? 4.0 : 2.4) : (q.a_cols && (uint64_t)q.M % 4 != 0 ? 3.0 : 0.0);
+    const double block_b = q.f32_b ? 0.4 * (bn / 32) : (!q.b_rows && (uint64_t)q.N % 4 != 0 ? 3.0 : 0.0);
+    const double batched = (f32 ? 8 : 5.5) + rounds * kb * (0.83 + block_a + block_b) + 0.8e-6 * q.elems;
     // Singly, B is packed and C is cleared, read and written; a K block costs 0.4 where TMA can fetch A, else its bytes are
     // gathered, one by one from unaligned columns.
     const double block = q.tma ? 0.4 : (q.a_cols && (uint64_t)q.M % 4 != 0 ? 6.2 : 1.8);
