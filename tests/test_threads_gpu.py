@@ -11,6 +11,7 @@ import pytest
 sys.path.insert(0, os.path.dirname(__file__))
 import bolt_b200 as B  # noqa: E402
 from bolt_b200 import synth  # noqa: E402
+from test_conv_gpu import conv_gpu  # noqa: E402
 from test_stack_gpu import make_stack  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -34,6 +35,10 @@ class Work:
         self.nb = B.matmul_infer_forward_tmp_bytes(ad, 0, bd, 0, cd, -1.0)
         self.tmp = torch.empty(self.nb, dtype=torch.uint8, device="cuda")
         self.ad, self.bd, self.cd = ad, bd, cd
+        self.conv = (1, 16, 6, 6, 16 + 8 * (t % 4), 3, 3, 1, 1)
+        oc = self.conv[4]
+        self.cx, self.cw = synth.u8(t + 1000, (1, 1, 6, 6, 16)), synth.s8(t + 1100, (oc, 16, 3, 3)) // np.int8(1 + t % 7)
+        self.cb = synth.normal(t + 1200, (oc,))
 
     def run(self):
         p = lambda t: C.c_void_p(t.data_ptr())
@@ -41,8 +46,9 @@ class Work:
         B.quantize(B.tensor1d(B.DT_F32, self.n), p(self.x), B.tensor1d(B.DT_U8_Q, self.n), p(self.q), sq)
         B.quantize(B.tensor1d(B.DT_I32, self.n), p(self.acc), B.tensor1d(B.DT_U8_Q, self.n), p(self.r), sr)
         sm = B.matmul(self.ad, 0, p(self.a), -1.0, self.bd, 0, p(self.b), -1.0, None, None, self.nb, p(self.tmp), self.cd, p(self.c), -1.0)
+        conv, sc, _ = conv_gpu(self.conv, self.cx, self.cw, self.cb, 16, True, True, [31.75, -1.0, 640.0])
         B.CHECK_STATUS(B.lib().bolt_b200_synchronize(), "synchronize")
-        return (sq[0], sr[0], float(sm), self.q.cpu().numpy().tobytes(), self.r.cpu().numpy().tobytes(), self.c.cpu().numpy().tobytes())
+        return (conv.tobytes(), sc[1], sq[0], sr[0], float(sm), self.q.cpu().numpy().tobytes(), self.r.cpu().numpy().tobytes(), self.c.cpu().numpy().tobytes())
 
 
 def test_threads_and_streams_do_not_mix():
