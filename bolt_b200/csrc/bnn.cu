@@ -36,7 +36,7 @@ constexpr int THREADS = WIDEN_THREADS + 32;       // + the warp that issues the 
 constexpr int MAX_BN = 128;                       // output channels of a tile
 constexpr int STAGE_A = 2 * BLOCK_M * BLOCK_K;    // two row blocks: 256 pixels
 constexpr int STAGE = STAGE_A + MAX_BN * BLOCK_K; // 48 KiB; two stages, two CTAs per SM
-constexpr uint32_t MAX_WORDS = 800;               // (tap, word) pairs of a filter
+constexpr uint32_t MAX_WORDS = 800;               // (tap, word) pairs of a filter: its sums, of 25600 bits at most, stay int16
 
 struct B4d {
     DataType dt;

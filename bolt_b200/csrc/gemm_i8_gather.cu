@@ -829,7 +829,7 @@ EE launch_gemm_gather(uint32_t M, uint32_t N, uint32_t K, const uint8_t *A, bool
         return SUCCESS;
     }
     if ((M + 15) / 16 > 65535) {
-        return NOT_SUPPORTED;
+        return NOT_SUPPORTED;   // (a million rows of such operands have never been taken; the kernel itself has no such limit)
     }
     DeviceCtx *c = ctx();
     if (c == nullptr) {

@@ -8,7 +8,7 @@
 // sums meet once in shared memory.
 //
 // 24 layers of 768 x 3072 and 3072 x 768 at 16 tokens, the whole pass: 183 us with a TMA kernel launch and a Python call
-// per layer, 86 us with this (8.8 us are the weights' share of the memory rate; the rest is 24 times a latency).
+// per layer, 95 us with this (9.1 us are the weights' share of the memory rate; the rest is 24 times a latency).
 //
 // In a chain of layers (bolt_b200_gemm_u8s8_chain) the kernel of layer i+1 starts while layer i runs and has its weight
 // fragments, offsets and factors in registers when layer i's result arrives.  That is safe because this kernel lets

@@ -372,12 +372,12 @@ def bnn(peaks, batch=128, iters=5):
     ms = tm.run(lambda: convolution(in_desc, _p(x), ftm_desc, _p(ftm), p, alg, _p(alpha), _p(beta), tb, _p(tmp), out_desc, _p(out)),
                 iters)
     L.bolt_b200_set_pointer_mode(0)
-    words = batch * hw * hw * oc * (k * k * ic // 32)
+    ops = 2.0 * batch * hw * hw * oc * k * k * ic
     bytes_ = x.numel() * 2 + out.numel() * 2 + oc * ic * k * k // 8
-    return {"workload": "bnn_xnor 3x3 C256 28x28 batch %d" % batch, "ms": ms, "Gword_ops_per_s": words / ms / 1e6,
-            "frac_of_popc_issue_nominal": words / ms / 1e6 / (16 * 148 * 1.965), "GBps": bytes_ / ms / 1e6,
+    return {"workload": "bnn_xnor 3x3 C256 28x28 batch %d" % batch, "ms": ms, "tops": ops / ms / 1e9,
+            "frac_of_2x_bf16_burst": ops / ms / 1e9 / (2.0 * peaks["bf16_tflops"]), "GBps": bytes_ / ms / 1e6,
             "frac_of_hbm": bytes_ / ms / 1e6 / peaks["hbm_gbs"],
-            "note": "bound by the popcount issue rate (nominal: 16 per clock per SM x 148 SMs x 1.965 GHz = 4.65 T/s), not by HBM"}
+            "note": "one-bit multiply-adds on the int8 tensor pipe; bound by widening the bits to bytes (issue and shared memory)"}
 
 
 def resnet_conv_u8_once(peaks):
