@@ -23,6 +23,9 @@ ThreadState &tls()
 
 EE cuda_ee(cudaError_t e)
 {
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // reported by this call: the thread's next one does not meet it again
+    }
     switch (e) {
         case cudaSuccess:
             return SUCCESS;

@@ -216,3 +216,19 @@ def test_matmul_dispatch_of_operands_that_tma_cannot_fetch():
     assert not route(1, 136, 36, 25084, 0, 0, F, F) and route(3, 12, 7, 5708, 0, 1, F, F)        # K off the 16-byte grid
     assert route(1, 87, 9, 20897, 1, 0, F, F) and not route(2, 1860, 4, 7664, 1, 1, F, I)        # A stored [K][M]
     assert not route(1, 64, 64, 4096, 0, 1, U, I) and route(1, 64, 64, 4096, 0, 1, U, I, a_at=(1 << 20) + 4)
+
+
+def test_a_reported_error_does_not_stay_in_the_thread():
+    """a launch that is refused fails its own call, and not the next one as well"""
+    lib = fake_gpu.load()
+    for call in (lambda: gemm_codes(lib, 8, 64, 64, False), lambda: gemm_codes(lib, 256, 64, 64, False),
+                 lambda: [matmul_code(lib, (2, 4, 16), (2, 16, 8), (2, 4, 8))[0]]):
+        lib.fake_refuse_programmatic(1)
+        lib.fake_capture(1)                  # (no second try while a stream is captured)
+        assert B.SUCCESS not in call() and lib.fake_last_error() == 0
+        lib.fake_refuse_programmatic(0)
+        lib.fake_capture(0)
+        assert set(call()) == {B.SUCCESS}
+    x, q, s = np.zeros(64, np.uint8), np.zeros(64, np.uint8), (C.c_float * 1)(-1.0)
+    d, o = B.tensor1d(U, 64), B.tensor1d(I, 64)
+    assert lib.quantize_cuda_b200(C.byref(d), C.c_void_p(x.ctypes.data), C.byref(o), C.c_void_p(q.ctypes.data), s, 0) == B.SUCCESS
